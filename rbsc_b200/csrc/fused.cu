@@ -1,0 +1,228 @@
+// fused.cu -- host side of the one-launch refinement (fused_kernels.cuh): when
+// it applies, its working memory, the launch, and the one-shot call of a small
+// host graph.
+#include <algorithm>
+#include <chrono>
+#include <cstring>
+
+#include <cuda_runtime.h>
+
+#include "../../include/rbsc.h"
+#include "common.cuh"
+#include "fused_kernels.cuh"
+#include "internal.h"
+
+using namespace rbsc;
+
+namespace {
+
+// Graphs up to these sizes run on one cluster of 8 blocks, larger ones on the
+// whole chip (us a refinement, cluster / chip: 3,000 nodes and 12,000 arcs
+// 70 / 71, 8,000 and 32,000 76-97 / 72-84, 16,000 and 64,000 115-135 / 80-87).
+constexpr uint32_t kClusterNodes = 8192;
+constexpr uint64_t kClusterArcs = 1u << 15;
+// Beside other contexts' work (a server's executors) only a cluster is safe to
+// launch, and it still beats the launch-per-phase path up to these sizes
+// (16,000 nodes and 128,000 arcs: 92-149 us against 325).
+constexpr uint32_t kSharedNodes = 16384;
+constexpr uint64_t kSharedArcs = 1u << 17;
+constexpr unsigned kClusterBlocks = 8;
+// A host graph of at most this many bytes goes through one pinned staging
+// buffer and one copy.
+constexpr size_t kStageBytes = 256u << 10;
+constexpr uint32_t kStageNodes = 16384;
+
+bool default_knobs(const rbsc_opts& o)
+{
+    return o.relabel == RBSC_RELABEL_HASH && o.use_graph && o.persist_log2 == 0 && o.grid_per_sm == 0 && o.sig_kernel == 0 &&
+           o.persist_bps == 0 && o.persist_sig == 0;
+}
+
+bool one_cluster(const rbsc_ctx* ctx, uint32_t n, uint64_t m)
+{
+    return ctx->shared_gpu || (n <= kClusterNodes && m <= kClusterArcs);
+}
+
+rbsc_status launch(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
+{
+    const bool cluster = one_cluster(ctx, a.n, a.m);
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = kFuThreads;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    if (cluster) {
+        cfg.gridDim = kClusterBlocks;
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = kClusterBlocks;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    } else {
+        // one block per SM (1024 threads of 64 registers)
+        cfg.gridDim = (unsigned)ctx->sm_count;
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        EK(cudaMemsetAsync(a.w, 0, sizeof(FusedWords), s));
+    }
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    ++rbsc::launch_counter();
+    if (cluster) EK(a.wt ? cudaLaunchKernelEx(&cfg, k_refine_fused<true, true>, a) : cudaLaunchKernelEx(&cfg, k_refine_fused<true, false>, a));
+    else EK(a.wt ? cudaLaunchKernelEx(&cfg, k_refine_fused<false, true>, a) : cudaLaunchKernelEx(&cfg, k_refine_fused<false, false>, a));
+    return RBSC_OK;
+}
+
+rbsc_status ensure_pinned(rbsc_ctx* ctx)
+{
+    if (!ctx->h_fused) EKS(host_alloc(ctx, &ctx->h_fused, sizeof(FusedResult)));
+    return RBSC_OK;
+}
+
+void common_args(const rbsc_ctx* ctx, FusedArgs& a)
+{
+    a.res = static_cast<FusedResult*>(ctx->h_fused);  // page-locked, written by the kernel
+    a.verify = ctx->opts.verify ? 1 : 0;
+    a.seed = ctx->opts.seed;
+    a.max_rounds = ctx->opts.max_rounds ? ctx->opts.max_rounds : a.n + 1u;
+    a.hash_bits = ctx->opts.test_hash_bits < 0 ? 64u : (uint32_t)ctx->opts.test_hash_bits;
+}
+
+// Status and statistics of a finished launch.  *handled false: the exact
+// check met a row with more colours than its table holds; the caller refines
+// the graph launch by launch.
+rbsc_status outcome(rbsc_ctx* ctx, rbsc_stats* stats, float ms, bool* handled)
+{
+    const FusedResult& r = *static_cast<const FusedResult*>(ctx->h_fused);
+    *handled = r.status != kFuRowTooWide;
+    switch (r.status) {
+        case kFuBadOffsets:
+            return rbsc_fail(ctx, RBSC_ERR_INVALID, "offsets are not a valid CSR (must start at 0, be non-decreasing and end at M)");
+        case kFuBadHead: return rbsc_fail(ctx, RBSC_ERR_INVALID, "an arc head is >= N");
+        case kFuNotConverged: return rbsc_fail(ctx, RBSC_ERR_NOT_CONVERGED, "no fixpoint after %u passes", r.rounds);
+        case kFuBarrier: return rbsc_fail(ctx, RBSC_ERR_DEVICE, "fused refinement: a grid barrier timed out");
+        default: break;
+    }
+    if (stats && *handled) {
+        stats->rounds = r.rounds;
+        stats->blocks = r.blocks;
+        stats->done = 1;
+        stats->verified = ctx->opts.verify ? 1u : 0u;
+        stats->repairs = r.repairs;
+        stats->initial_blocks = r.initial_blocks;
+        stats->device_ms = ms;
+        stats->init_ms = (double)(r.t[1] - r.t[0]) * 1e-6;
+        stats->loop_ms = (double)(r.t[2] - r.t[1]) * 1e-6;
+        stats->verify_ms = (double)(r.t[3] - r.t[2]) * 1e-6;
+        for (uint32_t i = 0; i < 64 && i <= r.rounds; ++i) stats->round_blocks[i] = r.round_blocks[i];
+    }
+    return RBSC_OK;
+}
+
+}  // namespace
+
+bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m)
+{
+    if (!default_knobs(ctx->opts) || n == 0 || n > (1u << 22) || m >= (1ull << 22)) return false;
+    // a cooperative grid needs the chip to itself; a cluster does not
+    if (ctx->shared_gpu) return n <= kSharedNodes && m <= kSharedArcs;
+    return !ctx->opts.no_persist;
+}
+
+rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled)
+{
+    *handled = false;
+    cudaStream_t s = ctx->stream;
+    const uint64_t lc0 = rbsc::launch_counter();
+    const FusedLayout l = fused_layout(g->n, g->m);
+    if (!g->d_fused) EKS(dev_alloc(ctx, &g->d_fused, l.bytes));
+    if (!d_out) {
+        if (!g->d_out) EKS(dev_alloc(ctx, (void**)&g->d_out, 4 * (size_t)g->n));
+        d_out = g->d_out;
+    }
+    EKS(ensure_pinned(ctx));
+    FusedArgs a{};
+    fused_bind(a, l, static_cast<unsigned char*>(g->d_fused));
+    a.n = g->n;
+    a.m = g->m;
+    a.off = g->d_off;
+    a.off64 = 1;
+    a.idx = g->d_idx;
+    a.wt = g->weighted ? g->d_wt : nullptr;
+    a.init = d_init;
+    a.out = d_out;
+    a.validate = g->prepared || g->trusted ? 0 : 1;
+    common_args(ctx, a);
+    EK(cudaEventRecord(ctx->ev[0], s));
+    EKS(launch(ctx, a, s));
+    EK(cudaEventRecord(ctx->ev[1], s));
+    EK(cudaStreamSynchronize(s));
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+    if (!g->prepared && !g->trusted) cudaEventElapsedTime(&g->up_ms, ctx->ev[2], ctx->ev[3]);
+    EKS(outcome(ctx, stats, ms, handled));
+    if (stats && *handled) stats->kernel_launches = rbsc::launch_counter() - lc0;
+    return RBSC_OK;
+}
+
+// A small host graph, labels back in host memory: the arrays are gathered in a
+// pinned buffer, go to the device in one copy, and the kernel writes the
+// labels and counts into pinned memory.
+rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled)
+{
+    *handled = false;
+    if (c->m > kStageBytes / 4 || c->n > kStageNodes) return RBSC_OK;  // before the sizes below are added up
+    const uint32_t n = c->n;
+    auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    const size_t b_off = (size_t)c->offset_bytes * ((size_t)n + 1), b_idx = 4 * (size_t)c->m, b_wt = c->weights ? 8 * (size_t)c->m : 0,
+                 b_init = init ? 4 * (size_t)n : 0;
+    const size_t in = al(b_off) + al(b_idx) + al(b_wt) + al(b_init);
+    if (!fused_wanted(ctx, n, c->m) || in > kStageBytes) return RBSC_OK;
+    const auto t0 = std::chrono::steady_clock::now();
+    EK(cudaSetDevice(ctx->device));
+    cudaStream_t s = ctx->stream;
+    EKS(ensure_pinned(ctx));
+    if (!ctx->h_stage) EKS(host_alloc(ctx, &ctx->h_stage, kStageBytes + 4 * (size_t)kStageNodes));
+    unsigned char* h = static_cast<unsigned char*>(ctx->h_stage);
+    uint32_t* h_out = reinterpret_cast<uint32_t*>(h + kStageBytes);
+    const size_t o_idx = al(b_off), o_wt = o_idx + al(b_idx), o_init = o_wt + al(b_wt);
+    std::memcpy(h, c->offsets, b_off);
+    if (b_idx) std::memcpy(h + o_idx, c->indices, b_idx);
+    if (b_wt) std::memcpy(h + o_wt, c->weights, b_wt);
+    if (b_init) std::memcpy(h + o_init, init, b_init);
+    const FusedLayout l = fused_layout(n, c->m);
+    Scratch sc(ctx);
+    unsigned char* d = nullptr;
+    EKS(sc.get(&d, l.bytes + in));
+    unsigned char* din = d + l.bytes;
+    FusedArgs a{};
+    fused_bind(a, l, d);
+    a.n = n;
+    a.m = c->m;
+    a.off = din;
+    a.off64 = c->offset_bytes == 8;
+    a.idx = reinterpret_cast<const uint32_t*>(din + o_idx);
+    a.wt = b_wt ? reinterpret_cast<const uint64_t*>(din + o_wt) : nullptr;
+    a.init = b_init ? reinterpret_cast<const uint32_t*>(din + o_init) : nullptr;
+    a.out = h_out;
+    a.validate = 1;
+    common_args(ctx, a);
+    EK(cudaEventRecord(ctx->ev[2], s));
+    EK(cudaMemcpyAsync(din, h, in, cudaMemcpyHostToDevice, s));
+    EK(cudaEventRecord(ctx->ev[0], s));
+    EKS(launch(ctx, a, s));
+    EK(cudaEventRecord(ctx->ev[1], s));
+    EK(cudaStreamSynchronize(s));
+    float ms = 0.f, up = 0.f;
+    cudaEventElapsedTime(&up, ctx->ev[2], ctx->ev[0]);
+    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+    if (stats) std::memset(stats, 0, sizeof *stats);
+    EKS(outcome(ctx, stats, ms, handled));
+    if (!*handled) return RBSC_OK;
+    if (out) std::memcpy(out, h_out, 4 * (size_t)n);
+    if (stats) {
+        stats->kernel_launches = 1;
+        stats->h2d_ms = up;
+        stats->h2d_bytes = b_off + b_idx + b_wt + b_init;
+        stats->d2h_bytes = out ? 4ull * n : 0;
+        stats->time_s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    }
+    return RBSC_OK;
+}

@@ -1,0 +1,1013 @@
+// fused_kernels.cuh -- a whole refinement in one launch, for graphs whose
+// passes are short (below about 2^22 arcs).
+//
+// The launch-per-phase path spends such a graph's time on launches, host
+// synchronisations and phase boundaries, not on work: the 131,072-node lift
+// took 0.42 ms for four passes whose bytes take a few microseconds (0.10 ms
+// here; a 1,000-arc one-shot call 0.44 -> 0.09 ms, R-MAT-18 with 3.9 M arcs
+// 0.36 -> 0.18 ms, 5,000 nodes without allocation 0.18 -> 0.04 ms).  Here one
+// launch checks the graph (on request), classes the initial colours, runs the
+// passes to the fixpoint, checks the fixpoint exactly, repairs it if the check
+// fails and writes the canonical labels.
+//
+// One barrier per pass.  A pass's new colour of a node is the *slot* its key
+// (old colour, signature) takes in the pass's table, which the thread that
+// inserts the key knows at once; no second phase has to look the class up,
+// and no smallest member is kept until the end.  Colours ping-pong between
+// two arrays (a pass reads the old ones while it writes the new ones), and
+// three tables take turns: the pass inserts into one, reads the previous one
+// (was a second node in my class? no: the node is alone for good and leaves
+// the passes as kSingleton | node) and zeroes the third for the next pass.
+// Any injective renaming of the colours gives the same partition, so blocks,
+// rounds and the final labels are those of the launch-per-phase path.
+//
+// A table entry is one 64-bit word: a 63-bit fingerprint of the key and the
+// joined bit (exact keys in the initial and repair passes).  Keys that share a
+// fingerprint would merge two classes; the exact check finds that.
+//
+// Rows: nodes are dealt to warps 32 at a time, interleaved over the SMs.  The
+// warp lays the arcs of its unfinished rows end to end and takes 32 of them
+// per step, one per lane (the heads of neighbouring rows lie side by side in
+// memory, so a step's loads coalesce, and no lane waits for a longer row);
+// a running prefix sum is read off at the row starts, and a row's sum is the
+// difference of two of them.  Rows of more than kFuChunk arcs, and
+// rows of more than kFuGroupRow arcs in a group of more than kFuGroupArcs (the
+// low node ids of an R-MAT graph are all hubs), are cut into chunks that all
+// warps share (the warp that completes a row's last chunk inserts it).
+// R-MAT-14 (228,000 arcs), first pass with only rows above 512 arcs shared:
+// 90 us, one warp holding most of the arcs.
+//
+// CLUSTER: the grid is one cluster (blocks are resident together by
+// construction, hardware barrier); otherwise a cooperative launch with a
+// counter barrier whose waits are bounded.
+#pragma once
+#include <algorithm>
+#include <cstdint>
+#include <cuda_runtime.h>
+#include "common.cuh"
+#include "refine_kernels.cuh"
+#include "verify_kernels.cuh"
+
+namespace rbsc {
+
+constexpr int kFuThreads = 1024;
+constexpr uint32_t kFuChunk = 256;
+constexpr uint32_t kFuGroupArcs = 1024;  // a warp's 32 rows together: beyond this its rows of more than
+constexpr uint32_t kFuGroupRow = 64;     // kFuGroupRow arcs are shared out too
+constexpr uint32_t kFuCache = 1024;         // per block: slots of classes it met that have two members
+// Shared memory is kept small on purpose: what it leaves is L1, whose lines
+// hold the gathers in flight (with 200 KB of check tables a pass of the
+// 131,072-node lift took 16.5 us, with 48 KB 13 us).
+constexpr uint32_t kFuCheckSlots = 2048;    // per block: colours of one long row (exact check)
+constexpr uint32_t kFuWarpSlots = kFuCheckSlots / (kFuThreads / 32);
+constexpr uint32_t kFuWarpRow = kFuWarpSlots - 8;  // rows up to this length are tried by one warp
+constexpr uint32_t kFuWideSlots = 32768;    // per block, in global memory: any row of a graph of at most 16384 nodes
+
+// outcome of a launch (FusedResult.status)
+// kFuRowTooWide: the launcher takes the launch-per-phase path
+constexpr int kFuOk = 0, kFuBadOffsets = 1, kFuBadHead = 2, kFuNotConverged = 3, kFuRowTooWide = 4, kFuBarrier = 5;
+
+// Counters of one launch, zero at its start (zeroed by the launcher, or by
+// block 0 of a cluster).
+struct FusedWords {
+    unsigned long long bar[2];  // barrier words (fu_barrier)
+    uint32_t pad[28];
+    uint32_t bad;          // 1 = offsets, 2 = a head
+    uint32_t overflow;     // a long row had more colours than the check's table
+    uint32_t nlong, nchunk;
+    uint32_t nlist[2];     // long rows of the running check (by repair parity)
+};
+
+struct FusedResult {
+    uint32_t rounds, blocks, initial_blocks, repairs;
+    int32_t status;
+    uint32_t pad;
+    uint64_t t[4];         // globaltimer: start, initial colours done, fixpoint, end
+    uint32_t round_blocks[kRoundLog];
+};
+
+struct FusedArgs {
+    uint32_t n;
+    uint64_t m;
+    const void* off;
+    const uint32_t* idx;
+    const uint64_t* wt;
+    const uint32_t* init;
+    uint32_t* out;
+    uint32_t* col[2];
+    unsigned long long* tab[3];
+    uint32_t log2tab;
+    uint32_t* minm;        // per slot of the final table: smallest member
+    uint32_t* list;        // nodes whose check needs a shared table
+    uint8_t* fail;
+    unsigned char* wide;   // kFuWideSlots counters per block for rows with more colours than the
+                           // shared table holds; null: such a row ends the launch (kFuRowTooWide)
+    uint32_t* lrow;        // long rows: node, first chunk, running sum, chunks done
+    uint32_t* lfirst;
+    unsigned long long* lsum;
+    uint32_t* ldone;
+    uint32_t* lchunk;      // chunk -> long row
+    uint32_t long_cap, chunk_cap;
+    FusedWords* w;
+    FusedResult* res;              // or:
+    rbsc_noalloc_result* na_res;
+    uint64_t seed;
+    uint32_t max_rounds;
+    uint32_t hash_bits;
+    uint8_t off64, validate, verify;
+};
+
+__device__ __forceinline__ uint64_t fu_off(const FusedArgs& a, uint32_t u)
+{
+    return a.off64 ? __ldg(reinterpret_cast<const unsigned long long*>(a.off) + u)
+                   : (uint64_t)__ldg(reinterpret_cast<const uint32_t*>(a.off) + u);
+}
+
+// Whether a row of d arcs in a group of `group` arcs goes in chunks.
+__device__ __forceinline__ bool fu_shared_row(uint32_t d, uint32_t group)
+{
+    return d > kFuChunk || (group > kFuGroupArcs && d > kFuGroupRow);
+}
+
+__device__ __forceinline__ uint64_t fu_timer()
+{
+    uint64_t t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// The per-arc term on the whole colour word (a bijection of it, salted).
+__device__ __forceinline__ uint64_t fu_term(uint32_t c, uint64_t salt)
+{
+    uint64_t y = (uint64_t)(c ^ (uint32_t)salt) * 0x9e3779b97f4a7c15ull;
+    y ^= y >> 32;
+    y *= 0xd6e8feb86659fd93ull;
+    y ^= y >> 32;
+    return y + (salt >> 32);
+}
+
+__device__ __forceinline__ uint64_t fu_warp_sum(uint64_t v, int width)
+{
+    for (int d = width >> 1; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+    return v;
+}
+
+struct FuCache {
+    unsigned long long key[kFuCache];
+    uint32_t slot[kFuCache];
+};
+
+__device__ __forceinline__ void fu_cache_clear(FuCache& c)
+{
+    for (uint32_t i = threadIdx.x; i < kFuCache; i += kFuThreads) {
+        c.key[i] = 0ull;
+        c.slot[i] = 0xffffffffu;
+    }
+}
+
+// Slot of fingerprint fp (bit 0 clear, not 0) for one node, or for several
+// (multi); claimed: this call opened the class.  A class already met by the block with two members answers from
+// shared memory: the few big classes of an early pass would otherwise be one
+// L2 address for the whole grid.  A cache word is written once per pass, by
+// the thread whose compare-and-swap took it.
+__device__ __forceinline__ uint32_t fu_insert(unsigned long long* __restrict__ tab, uint32_t log2tab, uint64_t fp, bool multi, FuCache& cache,
+                                              bool& claimed)
+{
+    const uint64_t h = fp * kGolden;
+    const uint32_t ci = (uint32_t)(h >> 20) & (kFuCache - 1u);
+    const uint64_t ck = *(volatile unsigned long long*)&cache.key[ci];
+    claimed = false;
+    if (ck == fp) {
+        const uint32_t s = *(volatile uint32_t*)&cache.slot[ci];
+        if (s != 0xffffffffu) return s;
+    }
+    const uint32_t mask = (1u << log2tab) - 1u;
+    uint32_t s = (uint32_t)(h >> (64 - log2tab));
+    // at most half of the entries are taken, so an empty one ends the probe;
+    // the bound only keeps a broken table from looping
+    for (uint32_t probe = 0; probe <= mask; ++probe, s = (s + 1u) & mask) {
+        unsigned long long e = __ldcg(tab + s);
+        if (e == 0ull) {
+            e = atomicCAS(tab + s, 0ull, (unsigned long long)fp | (multi ? 1ull : 0ull));
+            if (e == 0ull) {
+                claimed = true;
+                return s;
+            }
+        }
+        if ((e & ~1ull) == fp) {
+            if (!(e & 1ull)) atomicOr(tab + s, 1ull);
+            if (ck == 0ull && atomicCAS(&cache.key[ci], 0ull, (unsigned long long)fp) == 0ull)
+                *(volatile uint32_t*)&cache.slot[ci] = s;
+            return s;
+        }
+    }
+    return 0u;
+}
+
+// The lanes with `need` insert their keys; `few`: the classes are few beside
+// the nodes, so lanes with equal keys send one of them (32 compare-and-swaps
+// of a warp on one address would be served one after another).
+__device__ __forceinline__ uint32_t fu_insert_warp(bool need, bool few, unsigned long long* __restrict__ tab, uint32_t log2tab,
+                                                   uint64_t fp, FuCache& cache, uint32_t& made)
+{
+    const unsigned m = __ballot_sync(0xffffffffu, need);
+    uint32_t s = 0;
+    if (need) {
+        bool claimed = false;
+        if (few) {
+            const unsigned peers = __match_any_sync(m, (unsigned long long)fp);
+            const int leader = __ffs(peers) - 1;
+            if ((int)(threadIdx.x & 31) == leader) s = fu_insert(tab, log2tab, fp, (peers & (peers - 1u)) != 0u, cache, claimed);
+            s = __shfl_sync(peers, s, leader);
+        } else {
+            s = fu_insert(tab, log2tab, fp, false, cache, claimed);
+        }
+        made += claimed ? 1u : 0u;
+    }
+    return s;
+}
+
+// Barrier over the whole grid that also adds up `val` over the blocks (thread
+// 0's values): *total = the sum.  A word counts arrivals in its low half and
+// the values in its high half, both over all barriers so far, so one atomic
+// and one polled load do both.  Two words take turns: a block that is already
+// at the next barrier adds to the other one, so what this barrier reads is the
+// same for every block.  False: a wait ran out.
+struct FuSync {
+    uint32_t epoch = 0;           // barriers so far
+    uint32_t seen0 = 0, seen1 = 0;  // the words' high halves after their last barriers
+};
+
+template <bool CLUSTER>
+__device__ __forceinline__ bool fu_barrier(FusedWords* w, FuSync& y, uint32_t val, uint32_t* total, uint32_t* s_word)
+{
+    const uint32_t par = y.epoch & 1u;
+    const unsigned target = ((y.epoch >> 1) + 1u) * gridDim.x;  // arrivals at this word
+    ++y.epoch;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long* const word = &w->bar[par];
+        const unsigned long long add = ((unsigned long long)val << 32) | 1ull;
+        __threadfence();
+        unsigned long long v = atomicAdd(word, add) + add;
+        if (!CLUSTER) {
+            uint32_t it = 0;
+            while ((uint32_t)v < target) {
+                if (++it > (1u << 22)) {  // about two seconds
+                    s_word[1] = 1u;
+                    break;
+                }
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
+            }
+            s_word[0] = (uint32_t)(v >> 32);
+        }
+        __threadfence();
+    }
+    if (CLUSTER) {
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (threadIdx.x == 0) s_word[0] = (uint32_t)(__ldcg(&w->bar[par]) >> 32);
+    }
+    __syncthreads();
+    const uint32_t all = *(volatile uint32_t*)&s_word[0];
+    if (total) *total = all - (par ? y.seen1 : y.seen0);
+    if (par) y.seen1 = all;
+    else y.seen0 = all;
+    return CLUSTER || *(volatile uint32_t*)&s_word[1] == 0u;
+}
+
+// Group g (of 32 / G) of a warp takes the g-th set bit of `m` as its source
+// lane (-1: none); the bits taken are cleared.
+template <int G>
+__device__ __forceinline__ int fu_take(unsigned& m, int lane)
+{
+    int src = -1;
+#pragma unroll
+    for (int q = 0; q < 32 / G; ++q) {
+        const int b = m ? __ffs(m) - 1 : -1;
+        if (m) m &= m - 1u;
+        if (lane / G == q) src = b;
+    }
+    return src;
+}
+
+// Exact comparison of two rows of at most G arcs by groups of G lanes: lane gl
+// of a group holds arc gl of both rows (colour 0xffffffff and weight 0 past a
+// row's end).  Unit weights: both rows sorted in registers.  Weighted: every
+// lane adds up its colour's weight over both rows; a difference that is not 0
+// (mod 2^64) is one.
+template <bool WEIGHTED, int G>
+__device__ __forceinline__ bool fu_lane_differs(uint32_t a, uint32_t b, uint64_t wa, uint64_t wb)
+{
+    if (!WEIGHTED) return group_sort<G>(a) != group_sort<G>(b);
+    uint64_t da = 0, db = 0;
+#pragma unroll
+    for (int j = 0; j < G; ++j) {
+        const uint32_t ca = __shfl_sync(0xffffffffu, a, j, G), cb = __shfl_sync(0xffffffffu, b, j, G);
+        const uint64_t va = __shfl_sync(0xffffffffu, wa, j, G), vb = __shfl_sync(0xffffffffu, wb, j, G);
+        if (ca == a) da += va;
+        if (cb == a) da -= vb;
+        if (ca == b) db += va;
+        if (cb == b) db -= vb;
+    }
+    return (a != 0xffffffffu && da != 0) || (b != 0xffffffffu && db != 0);
+}
+
+// The rows (bu, du) and (br, dr) of the lanes in `m`, G lanes each; sets the
+// owner lane's `bad`.
+template <bool WEIGHTED, int G>
+__device__ __forceinline__ void fu_check_rows(unsigned m, int lane, const uint32_t* __restrict__ idx, const uint64_t* __restrict__ wt,
+                                              const uint32_t* __restrict__ col, uint64_t bu, uint32_t du, uint64_t br, uint32_t dr,
+                                              bool& bad)
+{
+    const int gl = lane & (G - 1);
+    while (m) {
+        const unsigned m0 = m;
+        const int src = fu_take<G>(m, lane);
+        const int s = src < 0 ? 0 : src;
+        const uint64_t xbu = __shfl_sync(0xffffffffu, bu, s), xbr = __shfl_sync(0xffffffffu, br, s);
+        const uint32_t xdu = __shfl_sync(0xffffffffu, du, s), xdr = __shfl_sync(0xffffffffu, dr, s);
+        uint32_t a = 0xffffffffu, b = 0xffffffffu;
+        uint64_t wa = 0, wb = 0;
+        if (src >= 0) {
+            if ((uint32_t)gl < xdu) {
+                a = __ldcg(col + __ldg(idx + xbu + gl));
+                if (WEIGHTED) wa = __ldg(reinterpret_cast<const unsigned long long*>(wt) + xbu + gl);
+            }
+            if ((uint32_t)gl < xdr) {
+                b = __ldcg(col + __ldg(idx + xbr + gl));
+                if (WEIGHTED) wb = __ldg(reinterpret_cast<const unsigned long long*>(wt) + xbr + gl);
+            }
+        }
+        const unsigned diff = __ballot_sync(0xffffffffu, fu_lane_differs<WEIGHTED, G>(a, b, wa, wb));
+        // which of this step's groups is the lane's own row in?
+        unsigned left = m0;
+#pragma unroll
+        for (int q = 0; q < 32 / G; ++q) {
+            if (!left) break;
+            const int b0 = __ffs(left) - 1;
+            left &= left - 1u;
+            const unsigned gm = G == 32 ? 0xffffffffu : (((1u << (G & 31)) - 1u) << (q * G));
+            if (lane == b0 && (diff & gm)) bad = true;
+        }
+    }
+}
+
+// Ascending bitonic sort of 32 * K values, K per lane (value i of the
+// sequence: register i / 32 of lane i % 32).
+template <int K> __device__ __forceinline__ void fu_sort(uint32_t (&v)[K])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 2; k <= 32 * K; k <<= 1)
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= 32) {
+#pragma unroll
+                for (int q = 0; q < K; ++q)
+                    if (!(q & (j / 32))) {
+                        const bool up = ((q * 32) & k) == 0;
+                        const uint32_t x = v[q], y = v[q | (j / 32)];
+                        v[q] = up ? min(x, y) : max(x, y);
+                        v[q | (j / 32)] = up ? max(x, y) : min(x, y);
+                    }
+            } else {
+#pragma unroll
+                for (int q = 0; q < K; ++q) {
+                    const uint32_t o = __shfl_xor_sync(0xffffffffu, v[q], j);
+                    const bool up = ((q * 32 + lane) & k) == 0;
+                    v[q] = ((lane & j) == 0) == up ? min(v[q], o) : max(v[q], o);
+                }
+            }
+        }
+}
+
+// The rows of the lanes in `m` (unit weights, equal lengths of at most 32 * K
+// arcs), one after another by the whole warp.
+template <int K>
+__device__ __forceinline__ void fu_check_long(unsigned m, int lane, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ col,
+                                              uint64_t bu, uint64_t br, uint32_t d, bool& bad)
+{
+    while (m) {
+        const int s = __ffs(m) - 1;
+        m &= m - 1u;
+        const uint64_t xbu = __shfl_sync(0xffffffffu, bu, s), xbr = __shfl_sync(0xffffffffu, br, s);
+        const uint32_t xd = __shfl_sync(0xffffffffu, d, s);
+        uint32_t a[K], b[K];
+#pragma unroll
+        for (int q = 0; q < K; ++q) {
+            const uint32_t i = 32u * q + lane;
+            a[q] = i < xd ? __ldcg(col + __ldg(idx + xbu + i)) : 0xffffffffu;
+            b[q] = i < xd ? __ldcg(col + __ldg(idx + xbr + i)) : 0xffffffffu;
+        }
+        fu_sort<K>(a);
+        fu_sort<K>(b);
+        bool diff = false;
+#pragma unroll
+        for (int q = 0; q < K; ++q) diff |= a[q] != b[q];
+        if (__any_sync(0xffffffffu, diff) && lane == s) bad = true;
+    }
+}
+
+// Adds sign * weight to colour c in an open-addressed table; false when full.
+__device__ __forceinline__ bool fu_count(uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t c, uint64_t w)
+{
+    uint32_t h = (c * 0x9e3779b1u) >> 7 & mask;
+    for (uint32_t p = 0; p <= mask; ++p, h = (h + 1u) & mask) {
+        const uint32_t k = atomicCAS(&key[h], 0xffffffffu, c);
+        if (k == 0xffffffffu || k == c) {
+            atomicAdd(&val[h], (unsigned long long)w);
+            return true;
+        }
+    }
+    return false;
+}
+
+template <bool CLUSTER, bool WEIGHTED>
+static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __grid_constant__ FusedArgs a)
+{
+    __shared__ FuCache s_cache;
+    __shared__ unsigned long long s_val[kFuCheckSlots];
+    __shared__ uint32_t s_key[kFuCheckSlots];
+    __shared__ uint32_t s_sum, s_flag, s_word[2];
+    __shared__ uint32_t s_delta[kFuThreads];  // per warp: its rows' (first arc - position) by rank
+    const uint32_t n = a.n;
+    const int lane = threadIdx.x & 31;
+    // warps dealt over the blocks: neighbouring node groups on different SMs
+    const uint32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const uint32_t nw = gridDim.x * (kFuThreads / 32);
+    const uint32_t gt = blockIdx.x * kFuThreads + threadIdx.x;
+    const uint32_t nt = gridDim.x * kFuThreads;
+    const uint32_t* __restrict__ idx = a.idx;
+    const uint64_t* __restrict__ wt = a.wt;
+    FusedWords* const w = a.w;
+    FuSync sync;
+    const bool first = gt == 0;
+    uint64_t t0 = 0, t1 = 0, t2 = 0;
+    if (first) t0 = fu_timer();
+    if (threadIdx.x == 0) {
+        s_sum = 0u;
+        s_word[0] = s_word[1] = 0u;
+    }
+    fu_cache_clear(s_cache);
+    if (CLUSTER) {
+        if (first) {
+            w->bar[0] = w->bar[1] = 0ull;
+            w->bad = w->overflow = 0u;
+            w->nlong = w->nchunk = 0u;
+            w->nlist[0] = w->nlist[1] = 0u;
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    }
+
+    auto finish = [&](int status, uint32_t rounds, uint32_t blocks, uint32_t initial, uint32_t repairs) {
+        if (!first) return;
+        if (a.res) {
+            a.res->rounds = rounds;
+            a.res->blocks = blocks;
+            a.res->initial_blocks = initial;
+            a.res->repairs = repairs;
+            a.res->status = status;
+            a.res->t[0] = t0;
+            a.res->t[1] = t1;
+            a.res->t[2] = t2;
+            a.res->t[3] = fu_timer();
+        }
+        if (a.na_res) {
+            a.na_res->blocks = blocks;
+            a.na_res->rounds = rounds;
+            a.na_res->repairs = repairs;
+            a.na_res->status = status == kFuOk                                        ? RBSC_OK
+                               : status == kFuBadOffsets || status == kFuBadHead ? RBSC_ERR_INVALID
+                               : status == kFuNotConverged                            ? RBSC_ERR_NOT_CONVERGED
+                                                                                      : RBSC_ERR_DEVICE;
+        }
+    };
+
+    if (n == 0) {
+        finish(kFuOk, 0u, 0u, 0u, 0u);
+        return;
+    }
+
+    // clear the tables, check the graph, list the long rows
+    const uint32_t tabn = 1u << a.log2tab;
+    auto clear_tab = [&](unsigned long long* t) {
+        ulonglong2* q = reinterpret_cast<ulonglong2*>(t);
+        for (uint32_t i = gt; i < tabn / 2; i += nt) q[i] = make_ulonglong2(0ull, 0ull);
+    };
+    auto clear_min = [&]() {
+        uint4* q = reinterpret_cast<uint4*>(a.minm);
+        for (uint32_t i = gt; i < tabn / 4; i += nt) q[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    };
+    clear_tab(a.tab[0]);
+    clear_tab(a.tab[1]);
+    clear_min();
+    uint32_t bad_in = 0;
+    for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
+        const uint32_t u = base + lane;
+        uint64_t b = 0, e = 0;
+        bool bad = false;
+        if (u < n) {
+            b = fu_off(a, u);
+            e = fu_off(a, u + 1);
+            bad = a.validate && (b > e || e > a.m || (u == 0 && b != 0) || (u == n - 1 && e != a.m));
+            if (!a.init) a.col[0][u] = 0u;
+        }
+        // (with a bad row anywhere nothing below is used)
+        const uint32_t d = bad ? 0u : (uint32_t)(e - b);
+        if (fu_shared_row(d, __reduce_add_sync(0xffffffffu, d))) {
+            const uint32_t nc = (d + kFuChunk - 1) / kFuChunk;
+            const uint32_t j = atomicAdd(&w->nlong, 1u), f = atomicAdd(&w->nchunk, nc);
+            if (j < a.long_cap) {
+                a.lrow[j] = u;
+                a.lfirst[j] = f;
+                a.lsum[j] = 0ull;
+                a.ldone[j] = 0u;
+                for (uint32_t i = 0; i < nc && f + i < a.chunk_cap; ++i) a.lchunk[f + i] = j;
+            }
+        }
+        bad_in |= bad ? 1u : 0u;
+    }
+    if (a.validate)
+        for (uint64_t k = gt; k < a.m; k += nt)
+            if (__ldg(idx + k) >= n) bad_in |= 2u;
+    if (bad_in) atomicOr(&w->bad, bad_in);
+    if (!fu_barrier<CLUSTER>(w, sync, 0u, nullptr, s_word)) {
+        finish(kFuBarrier, 0u, 0u, 0u, 0u);
+        return;
+    }
+    {
+        const uint32_t bad = __ldcg(&w->bad);
+        if (bad) {  // nothing is written, nothing read through the graph
+            finish((bad & 1u) ? kFuBadOffsets : kFuBadHead, 0u, 0u, 0u, 0u);
+            return;
+        }
+    }
+    const uint32_t nchunk = min(__ldcg(&w->nchunk), a.chunk_cap);
+
+    uint32_t p = 0;  // current colours: col[p & 1], classes: tab[p % 3]
+    uint32_t made = 0;
+    auto block_total = [&](uint32_t v) -> uint32_t {
+        v = __reduce_add_sync(0xffffffffu, v);
+        if (lane == 0 && v) atomicAdd(&s_sum, v);
+        __syncthreads();
+        return *(volatile uint32_t*)&s_sum;
+    };
+    uint32_t prev = 1;
+    bool has_classes = a.init != nullptr;
+    if (a.init) {
+        for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
+            const uint32_t u = base + lane;
+            const bool valid = u < n;
+            const uint64_t fp = valid ? ((uint64_t)__ldg(a.init + u) + 1ull) << 1 : 0ull;
+            const uint32_t s = fu_insert_warp(valid, true, a.tab[0], a.log2tab, fp, s_cache, made);
+            if (valid) a.col[0][u] = s;
+        }
+        const uint32_t tot = block_total(made);
+        if (!fu_barrier<CLUSTER>(w, sync, tot, &prev, s_word)) {
+            finish(kFuBarrier, 0u, 0u, 0u, 0u);
+            return;
+        }
+    }
+    const uint32_t initial = prev;
+    if (first) {
+        t1 = fu_timer();
+        if (a.res) a.res->round_blocks[0] = prev;
+    }
+
+    // one pass from col[p & 1] to the other array; REPAIR: the key is (colour,
+    // failed) instead of (colour, signature).  Returns false on a timeout.
+    uint32_t round = 0, repairs = 0, count = 0;
+    auto pass = [&](bool repair) -> bool {
+        const uint32_t* __restrict__ co = a.col[p & 1u];
+        uint32_t* __restrict__ cn = a.col[(p & 1u) ^ 1u];
+        const unsigned long long* __restrict__ tp = a.tab[p % 3u];
+        unsigned long long* tc = a.tab[(p + 1u) % 3u];
+        fu_cache_clear(s_cache);
+        if (threadIdx.x == 0) s_sum = 0u;
+        __syncthreads();
+        clear_tab(a.tab[(p + 2u) % 3u]);
+        if (repair) clear_min();
+        const uint64_t salt = pass_salt1(a.seed, round);
+        const bool uniform = !has_classes && !WEIGHTED;  // one class: a row's sum is its length times one term
+        const bool few = (uint64_t)prev * 1024ull < n;
+        const uint64_t t_one = fu_term(0u, salt);
+        const uint64_t hmask = a.hash_bits == 0 ? ~0ull : a.hash_bits >= 64 ? 0ull : (1ull << a.hash_bits) - 1ull;
+        made = 0;
+        auto fingerprint = [&](uint32_t c, uint64_t s1) -> uint64_t {
+            const uint64_t f = fmix64((s1 & hmask) ^ (((uint64_t)c + 1ull) * kGolden ^ a.seed)) & ~1ull;
+            return f ? f : 2ull;
+        };
+        for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
+            const uint32_t u = base + lane;
+            const bool valid = u < n;
+            uint32_t c = valid ? __ldcg(co + u) : kSingleton;
+            bool act = !(c & kSingleton);
+            unsigned long long e = 1ull;
+            uint64_t b = 0;
+            uint32_t d = 0;
+            if (valid && !repair) {
+                b = fu_off(a, u);
+                d = (uint32_t)(fu_off(a, u + 1) - b);
+            }
+            if (act) {
+                if (has_classes) e = __ldcg(tp + c);
+                else e = n > 1u ? 1ull : 0ull;
+                if (!(e & 1ull)) {  // nobody joined: alone for good
+                    act = false;
+                    c = kSingleton | u;
+                }
+            }
+            if (valid && !act) {
+                cn[u] = c;
+                ++made;
+            }
+            uint64_t fp = 0;
+            if (repair) {
+                if (act) fp = ((((uint64_t)c << 1) | (a.fail[u] ? 1ull : 0ull)) + 1ull) << 1;
+            } else {
+                uint64_t s1 = 0;
+                if (uniform) {
+                    s1 = t_one * d;
+                } else {
+                    if (fu_shared_row(d, __reduce_add_sync(0xffffffffu, d))) act = false;  // in chunks, below
+                    const unsigned rows = __ballot_sync(0xffffffffu, act && d > 0);
+                    const uint32_t dd = act ? d : 0u;
+                    uint32_t end = dd;  // inclusive prefix: where the row ends in the warp's sequence
+#pragma unroll
+                    for (int o = 1; o < 32; o <<= 1) {
+                        const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+                        if (lane >= o) end += x;
+                    }
+                    const uint32_t total = __shfl_sync(0xffffffffu, end, 31), start = end - dd;
+                    uint32_t* const delta = s_delta + (threadIdx.x & ~31u);
+                    if (dd) delta[__popc(rows & ((1u << lane) - 1u))] = (uint32_t)b - start;
+                    __syncwarp();
+                    uint64_t run = 0, at_start = 0;
+                    uint32_t before = 0;  // rows that start before the step
+                    constexpr int U = 4;  // steps whose loads are in flight together
+                    for (uint32_t j0 = 0; j0 < total; j0 += 32u * U) {
+                        uint32_t cc[U], pos[U];
+                        uint64_t x[U];
+#pragma unroll
+                        for (int q = 0; q < U; ++q) {
+                            const uint32_t j = j0 + 32u * q;
+                            // bit i: a row starts at position j + i
+                            const unsigned heads = __reduce_or_sync(0xffffffffu, dd && start - j < 32u ? 1u << (start - j) : 0u);
+                            const uint32_t rank = before + __popc(heads & (0xffffffffu >> (31 - lane)));
+                            before += __popc(heads);
+                            pos[q] = j + lane < total ? delta[rank - 1u] + j + lane : 0xffffffffu;
+                        }
+#pragma unroll
+                        for (int q = 0; q < U; ++q) cc[q] = pos[q] != 0xffffffffu ? __ldg(idx + pos[q]) : 0u;
+                        if (WEIGHTED) {
+#pragma unroll
+                            for (int q = 0; q < U; ++q)
+                                x[q] = pos[q] != 0xffffffffu ? __ldg(reinterpret_cast<const unsigned long long*>(wt) + pos[q]) : 0ull;
+                        }
+#pragma unroll
+                        for (int q = 0; q < U; ++q) cc[q] = pos[q] != 0xffffffffu ? __ldcg(co + cc[q]) : 0u;
+#pragma unroll
+                        for (int q = 0; q < U; ++q) {
+                            uint64_t t = pos[q] != 0xffffffffu ? fu_term(cc[q], salt) : 0ull;
+                            if (WEIGHTED) t *= x[q];
+                            uint64_t in = t;
+#pragma unroll
+                            for (int o = 1; o < 32; o <<= 1) {
+                                const uint64_t y = __shfl_up_sync(0xffffffffu, in, o);
+                                if (lane >= o) in += y;
+                            }
+                            const uint64_t ex = run + in - t;
+                            const uint32_t rel = start - (j0 + 32u * q);
+                            const uint64_t v = __shfl_sync(0xffffffffu, ex, rel & 31u);
+                            if (dd && rel < 32u) at_start = v;
+                            run += __shfl_sync(0xffffffffu, in, 31);
+                        }
+                    }
+                    // a row ends where the next one starts
+                    const unsigned above = lane == 31 ? 0u : rows & (0xffffffffu << (lane + 1));
+                    const uint64_t next = __shfl_sync(0xffffffffu, at_start, above ? __ffs(above) - 1 : 0);
+                    if (dd) s1 = (above ? next : run) - at_start;
+                    __syncwarp();
+                }
+                if (act) fp = fingerprint(c, s1);
+            }
+            const uint32_t s = fu_insert_warp(act, few, tc, a.log2tab, fp, s_cache, made);
+            if (act) cn[u] = s;
+        }
+        if (!repair && !uniform)
+            for (uint32_t ch = nw - 1u - gw; ch < nchunk; ch += nw) {
+                const uint32_t j = a.lchunk[ch], u = a.lrow[j], f = a.lfirst[j];
+                const uint32_t c = __ldcg(co + u);
+                if ((c & kSingleton) || (has_classes && !(__ldcg(tp + c) & 1ull)) || n == 1u) continue;
+                const uint64_t b = fu_off(a, u), e = fu_off(a, u + 1);
+                const uint64_t s = b + (uint64_t)(ch - f) * kFuChunk, t = min(e, s + kFuChunk);
+                uint64_t sum = 0;
+#pragma unroll 8
+                for (uint64_t i = s + lane; i < t; i += 32) {
+                    const uint64_t x = fu_term(__ldcg(co + __ldg(idx + i)), salt);
+                    sum += WEIGHTED ? x * __ldg(reinterpret_cast<const unsigned long long*>(wt) + i) : x;
+                }
+                sum = fu_warp_sum(sum, 32);
+                if (lane == 0) {
+                    const uint32_t nc = (uint32_t)((e - b + kFuChunk - 1) / kFuChunk);
+                    bool last = nc == 1u;
+                    if (!last) {
+                        atomicAdd(&a.lsum[j], (unsigned long long)sum);
+                        __threadfence();
+                        last = atomicAdd(&a.ldone[j], 1u) + 1u == nc;
+                        if (last) {
+                            __threadfence();
+                            sum = atomicExch(&a.lsum[j], 0ull);
+                            a.ldone[j] = 0u;
+                        }
+                    }
+                    if (last) {
+                        bool claimed;
+                        cn[u] = fu_insert(tc, a.log2tab, fingerprint(c, sum), false, s_cache, claimed);
+                        made += claimed ? 1u : 0u;
+                    }
+                }
+            }
+        const uint32_t tot = block_total(made);
+        if (!fu_barrier<CLUSTER>(w, sync, tot, &count, s_word)) return false;
+        ++p;
+        has_classes = true;
+        return true;
+    };
+
+    int status = kFuOk;
+    for (;;) {
+        // hashed passes to the fixpoint
+        for (;;) {
+            if (!pass(false)) {
+                finish(kFuBarrier, round, prev, initial, repairs);
+                return;
+            }
+            ++round;
+            const bool done = count == prev;
+            prev = count;
+            if (first && a.res && round < (uint32_t)kRoundLog) a.res->round_blocks[round] = count;
+            if (done) break;
+            if (round >= a.max_rounds) {
+                status = kFuNotConverged;
+                break;
+            }
+        }
+        if (first) t2 = fu_timer();
+        // the smallest member of every class
+        const uint32_t* __restrict__ col = a.col[p & 1u];
+        const uint32_t par = repairs & 1u;
+        if (first) w->nlist[par ^ 1u] = 0u;
+        for (uint32_t u = gt; u < n; u += nt) {
+            const uint32_t c = __ldcg(col + u);
+            if (!(c & kSingleton) && __ldcg(a.minm + c) > u) atomicMin(a.minm + c, u);
+        }
+        if (!fu_barrier<CLUSTER>(w, sync, 0u, nullptr, s_word)) {
+            finish(kFuBarrier, round, prev, initial, repairs);
+            return;
+        }
+        // labels, and the exact check of every node against that member
+        const bool check = a.verify && status == kFuOk;
+        uint32_t nbad = 0;
+        for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
+            const uint32_t u = base + lane;
+            const bool valid = u < n;
+            const uint32_t c = valid ? __ldcg(col + u) : kSingleton;
+            const uint32_t r = (c & kSingleton) ? u : __ldcg(a.minm + c);
+            if (valid) a.out[u] = r;
+            if (!check) continue;
+            const bool chk = valid && r != u;
+            uint64_t bu = 0, br = 0;
+            uint32_t du = 0, dr = 0, iu = 0, ir = 0;
+            if (chk) {
+                bu = fu_off(a, u);
+                br = fu_off(a, r);
+                du = (uint32_t)(fu_off(a, u + 1) - bu);
+                dr = (uint32_t)(fu_off(a, r + 1) - br);
+                if (a.init) {
+                    iu = __ldg(a.init + u);
+                    ir = __ldg(a.init + r);
+                }
+            }
+            bool bad = chk && (iu != ir || (!WEIGHTED && du != dr));
+            const uint32_t mx = chk && !bad ? max(du, dr) : 0u;
+            fu_check_rows<WEIGHTED, 8>(__ballot_sync(0xffffffffu, mx > 0 && mx <= 8), lane, idx, wt, col, bu, du, br, dr, bad);
+            fu_check_rows<WEIGHTED, 16>(__ballot_sync(0xffffffffu, mx > 8 && mx <= 16), lane, idx, wt, col, bu, du, br, dr, bad);
+            fu_check_rows<WEIGHTED, 32>(__ballot_sync(0xffffffffu, mx > 16 && mx <= 32), lane, idx, wt, col, bu, du, br, dr, bad);
+            uint32_t reg = 32;  // longest row compared in registers
+            if (!WEIGHTED) {
+                fu_check_long<2>(__ballot_sync(0xffffffffu, mx > 32 && mx <= 64), lane, idx, col, bu, br, du, bad);
+                fu_check_long<4>(__ballot_sync(0xffffffffu, mx > 64 && mx <= 128), lane, idx, col, bu, br, du, bad);
+                reg = 128;
+            }
+            const unsigned ml = __ballot_sync(0xffffffffu, mx > reg);
+            if (ml) {
+                uint32_t at = 0;
+                if (lane == 0) at = atomicAdd(&w->nlist[par], (uint32_t)__popc(ml));
+                at = __shfl_sync(0xffffffffu, at, 0);
+                if (mx > reg) a.list[at + __popc(ml & ((1u << lane) - 1u))] = u;
+            }
+            if (valid && !(c & kSingleton)) a.fail[u] = bad ? 1 : 0;
+            nbad += bad ? 1u : 0u;
+        }
+        if (!check) {
+            finish(status, round, prev, initial, repairs);
+            return;
+        }
+        if (threadIdx.x == 0) s_sum = 0u;
+        __syncthreads();
+        uint32_t tot = block_total(nbad), nfail = 0, more = 0;
+        if (!fu_barrier<CLUSTER>(w, sync, tot, &nfail, s_word)) {
+            finish(kFuBarrier, round, prev, initial, repairs);
+            return;
+        }
+        const uint32_t nlist = __ldcg(&w->nlist[par]);
+        if (nlist) {
+            // longer rows: colours counted in a table, + for the member's row
+            // and - for the node's; all must end at 0.  A warp tries the short
+            // ones (weighted) in its part of the block's table and leaves them
+            // to the block when they do not fit.
+            nbad = 0;
+            auto add_row = [&](uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t x, bool minus, uint32_t at,
+                               uint32_t step) -> bool {
+                bool ok = true;
+                const uint64_t b = fu_off(a, x), e = fu_off(a, x + 1);
+                for (uint64_t i = b + at; i < e; i += step) {
+                    const uint64_t v = WEIGHTED ? __ldg(reinterpret_cast<const unsigned long long*>(wt) + i) : 1ull;
+                    ok &= fu_count(key, val, mask, __ldcg(col + __ldg(idx + i)), minus ? 0ull - v : v);
+                }
+                return ok;
+            };
+            auto longest = [&](uint32_t u, uint32_t r) {
+                return max((uint32_t)(fu_off(a, u + 1) - fu_off(a, u)), (uint32_t)(fu_off(a, r + 1) - fu_off(a, r)));
+            };
+            if (WEIGHTED) {
+                const uint32_t wi = threadIdx.x >> 5;
+                uint32_t* key = s_key + wi * kFuWarpSlots;
+                unsigned long long* val = s_val + wi * kFuWarpSlots;
+                for (uint32_t i = gw; i < nlist; i += nw) {
+                    const uint32_t u = a.list[i], r = __ldcg(a.minm + __ldcg(col + u));
+                    if (longest(u, r) > kFuWarpRow) continue;
+                    for (uint32_t k = lane; k < kFuWarpSlots; k += 32) {
+                        key[k] = 0xffffffffu;
+                        val[k] = 0ull;
+                    }
+                    __syncwarp();
+                    bool ok = add_row(key, val, kFuWarpSlots - 1u, r, false, lane, 32);
+                    ok &= add_row(key, val, kFuWarpSlots - 1u, u, true, lane, 32);
+                    __syncwarp();
+                    bool diff = false;
+                    for (uint32_t k = lane; k < kFuWarpSlots; k += 32) diff |= val[k] != 0ull;
+                    ok = __all_sync(0xffffffffu, ok);
+                    diff = __any_sync(0xffffffffu, diff);
+                    if (lane == 0) {
+                        if (!ok) a.fail[u] = 2;  // undecided
+                        else if (diff) {
+                            a.fail[u] = 1;
+                            ++nbad;
+                        }
+                    }
+                    __syncwarp();
+                }
+                // the undecided marks are read by other blocks
+                if (!fu_barrier<CLUSTER>(w, sync, 0u, nullptr, s_word)) {
+                    finish(kFuBarrier, round, prev, initial, repairs);
+                    return;
+                }
+            }
+            for (uint32_t i = blockIdx.x; i < nlist; i += gridDim.x) {
+                const uint32_t u = a.list[i], r = __ldcg(a.minm + __ldcg(col + u));
+                if (WEIGHTED && longest(u, r) <= kFuWarpRow && __ldcg(a.fail + u) != 2) continue;
+                uint32_t* key = s_key;
+                unsigned long long* val = s_val;
+                uint32_t slots = kFuCheckSlots;
+                for (;;) {
+                    for (uint32_t k = threadIdx.x; k < slots; k += kFuThreads) {
+                        key[k] = 0xffffffffu;
+                        val[k] = 0ull;
+                    }
+                    if (threadIdx.x == 0) s_flag = 0u;
+                    __syncthreads();
+                    bool ok = add_row(key, val, slots - 1u, r, false, threadIdx.x, kFuThreads);
+                    ok &= add_row(key, val, slots - 1u, u, true, threadIdx.x, kFuThreads);
+                    if (!ok) atomicOr(&s_flag, 2u);
+                    __syncthreads();
+                    bool diff = false;
+                    for (uint32_t k = threadIdx.x; k < slots; k += kFuThreads) diff |= val[k] != 0ull;
+                    if (diff) atomicOr(&s_flag, 1u);
+                    __syncthreads();
+                    const uint32_t f = *(volatile uint32_t*)&s_flag;
+                    __syncthreads();
+                    if ((f & 2u) && key == s_key && a.wide) {
+                        // more colours than the shared table holds: once more in global memory
+                        val = reinterpret_cast<unsigned long long*>(a.wide + (size_t)blockIdx.x * kFuWideSlots * 12);
+                        key = reinterpret_cast<uint32_t*>(val + kFuWideSlots);
+                        slots = kFuWideSlots;
+                        continue;
+                    }
+                    if (threadIdx.x == 0) {
+                        if (f & 2u) atomicOr(&w->overflow, 1u);
+                        a.fail[u] = (f & 1u) ? 1 : 0;
+                        nbad += f & 1u;
+                    }
+                    break;
+                }
+            }
+            if (threadIdx.x == 0) s_sum = 0u;
+            __syncthreads();
+            tot = block_total(nbad);
+            if (!fu_barrier<CLUSTER>(w, sync, tot, &more, s_word)) {
+                finish(kFuBarrier, round, prev, initial, repairs);
+                return;
+            }
+            if (__ldcg(&w->overflow)) {
+                finish(kFuRowTooWide, round, prev, initial, repairs);
+                return;
+            }
+        }
+        if (nfail + more == 0u) {
+            finish(kFuOk, round, prev, initial, repairs);
+            return;
+        }
+        // split the failed nodes off and refine on
+        ++repairs;
+        if (!pass(true)) {
+            finish(kFuBarrier, round, prev, initial, repairs);
+            return;
+        }
+        prev = count;
+        if (round >= a.max_rounds) {
+            // no pass left: the labels of the partition as it stands, unchecked
+            status = kFuNotConverged;
+            const uint32_t* __restrict__ cc = a.col[p & 1u];
+            for (uint32_t u = gt; u < n; u += nt) {
+                const uint32_t c = __ldcg(cc + u);
+                if (!(c & kSingleton) && __ldcg(a.minm + c) > u) atomicMin(a.minm + c, u);
+            }
+            if (!fu_barrier<CLUSTER>(w, sync, 0u, nullptr, s_word)) {
+                finish(kFuBarrier, round, prev, initial, repairs);
+                return;
+            }
+            for (uint32_t u = gt; u < n; u += nt) {
+                const uint32_t c = __ldcg(cc + u);
+                a.out[u] = (c & kSingleton) ? u : __ldcg(a.minm + c);
+            }
+            finish(status, round, prev, initial, repairs);
+            return;
+        }
+    }
+}
+
+// Working memory of a fused refinement: offsets of its arrays in one block.
+struct FusedLayout {
+    size_t col[2], tab[3], minm, list, fail, lrow, lfirst, lsum, ldone, lchunk, words, bytes;
+    uint32_t log2tab, long_cap, chunk_cap;
+};
+
+inline FusedLayout fused_layout(uint32_t n, uint64_t m)
+{
+    FusedLayout l{};
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t r = at;
+        at += (bytes + 255) & ~(size_t)255;
+        return r;
+    };
+    l.log2tab = 10;
+    while ((1ull << l.log2tab) < 2ull * n) ++l.log2tab;
+    l.long_cap = (uint32_t)std::min<uint64_t>(n, m / (kFuGroupRow + 1)) + 1u;  // rows that go in chunks
+    l.chunk_cap = (uint32_t)(m / kFuChunk) + l.long_cap;                         // at most one partial chunk each
+    l.words = take(sizeof(FusedWords));
+    for (int i = 0; i < 2; ++i) l.col[i] = take(4ull * n);
+    for (int i = 0; i < 3; ++i) l.tab[i] = take(8ull << l.log2tab);
+    l.minm = take(4ull << l.log2tab);
+    l.list = take(4ull * n);
+    l.fail = take(n);
+    l.lrow = take(4ull * l.long_cap);
+    l.lfirst = take(4ull * l.long_cap);
+    l.lsum = take(8ull * l.long_cap);
+    l.ldone = take(4ull * l.long_cap);
+    l.lchunk = take(4ull * l.chunk_cap);
+    l.bytes = at;
+    return l;
+}
+
+inline void fused_bind(FusedArgs& a, const FusedLayout& l, unsigned char* base)
+{
+    a.w = reinterpret_cast<FusedWords*>(base + l.words);
+    for (int i = 0; i < 2; ++i) a.col[i] = reinterpret_cast<uint32_t*>(base + l.col[i]);
+    for (int i = 0; i < 3; ++i) a.tab[i] = reinterpret_cast<unsigned long long*>(base + l.tab[i]);
+    a.log2tab = l.log2tab;
+    a.minm = reinterpret_cast<uint32_t*>(base + l.minm);
+    a.list = reinterpret_cast<uint32_t*>(base + l.list);
+    a.fail = base + l.fail;
+    a.lrow = reinterpret_cast<uint32_t*>(base + l.lrow);
+    a.lfirst = reinterpret_cast<uint32_t*>(base + l.lfirst);
+    a.lsum = reinterpret_cast<unsigned long long*>(base + l.lsum);
+    a.ldone = reinterpret_cast<uint32_t*>(base + l.ldone);
+    a.lchunk = reinterpret_cast<uint32_t*>(base + l.lchunk);
+    a.long_cap = l.long_cap;
+    a.chunk_cap = l.chunk_cap;
+}
+
+}  // namespace rbsc

@@ -41,6 +41,13 @@ struct rbsc_ctx {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int sm_count = 148;
+    // other contexts' work runs beside this one's (a server's executors): no
+    // cooperative launches
+    bool shared_gpu = false;
+    // the one-launch refinement (fused.cu): its page-locked result and the
+    // staging buffer of small one-shot calls
+    void* h_fused = nullptr;
+    void* h_stage = nullptr;
     std::string err;
 };
 
@@ -61,6 +68,12 @@ struct rbsc_graph {
     uint32_t nsplit = 0;
     uint32_t* d_split = nullptr;
     uint8_t* d_head8 = nullptr;  // row-head bitmap, one bit per arc
+    bool prepared = false;       // checked and tiled (graph_prepare); a graph the one-launch
+                                 // refinement takes is checked there and needs no tiling
+    float up_ms = 0.f;           // its host-to-device copies, timed by fused_refine
+    bool trusted = false;        // built by the library from a checked graph
+
+    void* d_fused = nullptr;     // working memory of the one-launch refinement
 
     // refinement state (allocated on first refine, reused)
     bool bufs = false;
@@ -180,6 +193,9 @@ rbsc_status host_alloc(rbsc_ctx* ctx, void** p, size_t bytes);
 void host_free(rbsc_ctx* ctx, void*& p);
 rbsc_status ensure_temp(rbsc_ctx* ctx, rbsc_graph* g, size_t bytes);
 rbsc_status graph_prepare(rbsc_ctx* ctx, rbsc_graph* g);
+// Copies a host CSR to the device without checking or tiling it, for a graph
+// that fused_wanted takes (refine_resident prepares it if it has to).
+rbsc_status graph_upload_unprepared(rbsc_ctx* ctx, const rbsc_csr* host_graph, rbsc_graph** out, double* h2d_ms, uint64_t* h2d_bytes);
 rbsc_status graph_alloc_csr(rbsc_ctx* ctx, rbsc_graph* g, bool weighted);
 rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats,
                             rbsc_kernel_times* kt);
@@ -223,6 +239,13 @@ struct Scratch {
         rbsc_status s_ = (call);       \
         if (s_ != RBSC_OK) return s_;  \
     } while (0)
+
+// The one-launch refinement of small graphs (fused.cu).  fused_wanted: the
+// context's options and the sizes allow it.  *handled false on RBSC_OK: it
+// does not apply after all, and the caller takes the launch-per-phase path.
+bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m);
+rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled);
+rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled);
 
 // sort-based relabel (sortrelabel.cu)
 rbsc_status ensure_sort_relabel_bufs(rbsc_ctx* ctx, rbsc_graph* g);

@@ -241,6 +241,8 @@ extern "C" void rbsc_ctx_destroy(rbsc_ctx* ctx)
         cudaStreamDestroy(ctx->side);
     }
     cudaStreamDestroy(ctx->stream);
+    host_free(ctx, ctx->h_fused);
+    host_free(ctx, ctx->h_stage);
     pool_release(ctx->dpool);
     pool_release(ctx->hpool);
     delete ctx;
@@ -323,6 +325,7 @@ static void graph_release_refine(rbsc_graph* g)
     dev_free(g->ctx, (void*&)g->d_vals[1]);
     dev_free(g->ctx, (void*&)g->d_small);
     dev_free(g->ctx, g->d_tmp);
+    dev_free(g->ctx, g->d_fused);
     g->tmp_bytes = 0;
     g->key_cap = 0;
     host_free(g->ctx, (void*&)g->h_st);
@@ -490,6 +493,7 @@ rbsc_status graph_prepare(rbsc_ctx* ctx, rbsc_graph* g)
         g->nsplit = 0;
         CKS(dev_alloc(ctx, (void**)&g->d_split, sizeof(uint32_t)));
     }
+    g->prepared = true;
     return RBSC_OK;
 }
 
@@ -523,8 +527,11 @@ rbsc_status graph_alloc_csr(rbsc_ctx* ctx, rbsc_graph* g, bool weighted)
 // defer_heads: the heads are not copied here; they arrive in chunks during
 // the first pass that reads them (stream_signature's upload mode), which
 // overlaps their copy with the initial colours, the setup and that pass.
+// unprepared: neither checked nor tiled here, and the copies are not waited
+// for: the one-launch refinement that follows checks the graph itself.
 static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device, rbsc_graph** out, double* h2d_ms,
-                              uint64_t* h2d_bytes, bool defer_heads = false, const uint32_t* h_init = nullptr)
+                              uint64_t* h2d_bytes, bool defer_heads = false, const uint32_t* h_init = nullptr,
+                              bool unprepared = false)
 {
     *out = nullptr;
     CKS(check_csr_args(ctx, c));
@@ -542,11 +549,11 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
     cudaStream_t s = ctx->stream;
     const cudaMemcpyKind kind = from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     auto t0 = std::chrono::steady_clock::now();
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = unprepared ? cudaEventRecord(ctx->ev[2], s) : cudaSuccess;
     const size_t offb = (size_t)c->offset_bytes * ((size_t)c->n + 1);
     uint64_t bytes = offb + sizeof(uint32_t) * c->m + (c->weights ? sizeof(uint64_t) * c->m : 0);
     if (c->offset_bytes == 8) {
-        e = cudaMemcpyAsync(g->d_off, c->offsets, offb, kind, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(g->d_off, c->offsets, offb, kind, s);
     } else {
         // stage the 32-bit offsets in the (not yet used) index buffer tail? use a scratch buffer
         void* tmp = nullptr;
@@ -561,7 +568,7 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
             k_widen_offsets<uint32_t><<<grid_for((uint64_t)c->n + 1, 256), 256, 0, s>>>((uint64_t)c->n + 1, (const uint32_t*)tmp, g->d_off);
             e = cudaGetLastError();
         }
-        cudaStreamSynchronize(s);
+        if (!unprepared) cudaStreamSynchronize(s);
         dev_free(ctx, tmp);
     }
     defer_heads = defer_heads && !from_device && !c->weights && c->m > 0;
@@ -606,14 +613,19 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
         e = cudaMemcpyAsync(g->d_idx, c->indices, sizeof(uint32_t) * c->m, kind, s);
     }
     if (e == cudaSuccess && c->weights && c->m) e = cudaMemcpyAsync(g->d_wt, c->weights, sizeof(uint64_t) * c->m, kind, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess && !unprepared) e = cudaStreamSynchronize(s);
     auto t1 = std::chrono::steady_clock::now();
-    if (h2d_ms) *h2d_ms = std::chrono::duration<double, std::milli>(t1 - t0).count();
+    if (h2d_ms) *h2d_ms = unprepared ? 0.0 : std::chrono::duration<double, std::milli>(t1 - t0).count();
     if (h2d_bytes) *h2d_bytes = from_device ? 0 : bytes;
     if (e != cudaSuccess) {
         rbsc_cuda_fail(ctx, e, "graph copy", __LINE__);
         rbsc_graph_free(g);
         return e == cudaErrorMemoryAllocation ? RBSC_ERR_OOM : RBSC_ERR_CUDA;
+    }
+    if (unprepared) {
+        CK(cudaEventRecord(ctx->ev[3], s));  // fused_refine reads the copies' time
+        *out = g;
+        return RBSC_OK;
     }
     st = graph_prepare(ctx, g);
     if (st != RBSC_OK) {
@@ -622,6 +634,11 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
     }
     *out = g;
     return RBSC_OK;
+}
+
+rbsc_status graph_upload_unprepared(rbsc_ctx* ctx, const rbsc_csr* host_graph, rbsc_graph** out, double* h2d_ms, uint64_t* h2d_bytes)
+{
+    return graph_load(ctx, host_graph, false, out, h2d_ms, h2d_bytes, false, nullptr, true);
 }
 
 extern "C" rbsc_status rbsc_graph_upload(rbsc_ctx* ctx, const rbsc_csr* host_graph, rbsc_graph** out)
@@ -745,7 +762,7 @@ static rbsc_status ensure_refine_bufs(rbsc_ctx* ctx, rbsc_graph* g)
     CKS(dev_alloc(ctx, (void**)&g->d_sig, sizeof(Sig) * n));
     CKS(dev_alloc(ctx, (void**)&g->d_slot, 4 * n));
     CKS(dev_alloc(ctx, (void**)&g->d_joined, 4 * n));
-    CKS(dev_alloc(ctx, (void**)&g->d_out, 4 * n));
+    if (!g->d_out) CKS(dev_alloc(ctx, (void**)&g->d_out, 4 * n));
     CKS(dev_alloc(ctx, (void**)&g->d_rank, 2 * n));
     CKS(dev_alloc(ctx, (void**)&g->d_small, 256));
     g->log2tab = std::max<uint32_t>(10, log2_ceil(2ull * n));
@@ -1674,6 +1691,12 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         if (stats) stats->done = stats->verified = 1;
         return RBSC_OK;
     }
+    if (!kt && !g->host_arcs && fused_wanted(ctx, n, g->m)) {
+        bool handled = false;
+        CKS(fused_refine(ctx, g, d_init, d_out, stats, &handled));
+        if (handled) return RBSC_OK;
+    }
+    if (!g->prepared) CKS(graph_prepare(ctx, g));
     CKS(ensure_refine_bufs(ctx, g));
     g->first_sig_ms = 0.f;
     g->first_sig_arcs = 0;
@@ -1881,7 +1904,7 @@ extern "C" rbsc_status rbsc_graph_refine(rbsc_ctx* ctx, rbsc_graph* g, const uin
     if (!ctx || !g) return rbsc_fail(ctx, RBSC_ERR_INVALID, "null argument");
     CK(cudaSetDevice(ctx->device));
     auto t0 = std::chrono::steady_clock::now();
-    CKS(ensure_refine_bufs(ctx, g));
+    if (!g->d_out) CKS(dev_alloc(ctx, (void**)&g->d_out, 4 * (size_t)std::max<uint32_t>(g->n, 1)));
     double h2d = 0, d2h = 0;
     const uint32_t* d_init = nullptr;
     if (init_colors && g->n && init_colors == g->h_init_loaded) {
@@ -1920,11 +1943,16 @@ extern "C" rbsc_status rbsc_refine(rbsc_ctx* ctx, const rbsc_csr* host_graph, co
     rbsc_graph* g = nullptr;
     double up_ms = 0;
     uint64_t up_bytes = 0;
+    CKS(check_csr_args(ctx, host_graph));
+    bool handled = false;
+    CKS(fused_oneshot(ctx, host_graph, init_colors, out_labels, stats, &handled));
+    if (handled) return RBSC_OK;
     // large unweighted graphs: the heads' copy overlaps the refinement
-    const bool defer = host_graph && !host_graph->weights && host_graph->m >= (1ull << 22);
-    CKS(graph_load(ctx, host_graph, false, &g, &up_ms, &up_bytes, defer, init_colors));
+    const bool defer = !host_graph->weights && host_graph->m >= (1ull << 22);
+    CKS(graph_load(ctx, host_graph, false, &g, &up_ms, &up_bytes, defer, init_colors, fused_wanted(ctx, host_graph->n, host_graph->m)));
     g->oneshot = true;
     rbsc_status st = rbsc_graph_refine(ctx, g, init_colors, out_labels, stats);
+    up_ms += g->up_ms;
     rbsc_graph_free(g);
     if (st == RBSC_OK && stats) {
         stats->h2d_ms += up_ms;

@@ -464,6 +464,7 @@ extern "C" rbsc_status rbsc_serve_create(const rbsc_serve_opts* opts, rbsc_serve
                 delete srv;
                 return s;
             }
+            sl->ctx->shared_gpu = true;
             // unused cached blocks of a slot count against nobody's budget, but
             // giving them back costs a cudaFree, which waits for every slot's
             // work on the device: a slot keeps up to its share of the budget
