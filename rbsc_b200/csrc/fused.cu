@@ -10,6 +10,8 @@
 #include "../../include/rbsc.h"
 #include "common.cuh"
 #include "fused_kernels.cuh"
+#include "deep_kernels.cuh"
+#include "scan.cuh"
 #include "internal.h"
 
 using namespace rbsc;
@@ -85,6 +87,117 @@ void common_args(const rbsc_ctx* ctx, FusedArgs& a)
     a.hash_bits = ctx->opts.test_hash_bits < 0 ? 64u : (uint32_t)ctx->opts.test_hash_bits;
 }
 
+// When to look for a deep refinement: once the passes so far have cost about
+// as much as the change to the work list does (us; a pass takes about 6 + 1
+// per 100,000 arcs, the change 150 + 1 per 20,000).
+uint32_t deep_round(uint64_t m)
+{
+    const double pass = 6.0 + (double)m / 100e3, change = 150.0 + (double)m / 20e3;
+    return (uint32_t)std::max(6.0, change / pass);
+}
+
+// The passes after a launch that ended with kFuDeep, on a work list: the
+// classes of its last two passes are in a.col.  Leaves the launch that
+// confirms (or goes on) in `a`.
+rbsc_status deep_tail(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
+{
+    FusedResult& r = *static_cast<FusedResult*>(ctx->h_fused);
+    const uint32_t n = a.n, passes = r.rounds - a.round0;
+    uint32_t* col = a.col[passes & 1u];
+    const uint32_t* old = a.col[(passes & 1u) ^ 1u];
+    const size_t slots = (size_t)1 << a.log2tab, ids = slots + n / 2 + 2;
+    Scratch sc(ctx);
+    // zeroed together: class sizes, in-degrees, T stamps, largest parts, counters
+    const size_t z_size = 0, z_deg = z_size + 4 * ids, z_flag = z_deg + 4 * (size_t)n, z_ctr = z_flag + 4 * (size_t)n,
+                 z_best = (z_ctr + sizeof(IncCounters) + 255) & ~(size_t)255, z_bytes = z_best + 8 * slots;
+    unsigned char* z = nullptr;
+    unsigned long long *sig = nullptr, *S = nullptr;
+    uint32_t *cursor = nullptr, *tsrc = nullptr, *colm = nullptr, *tlist = nullptr;
+    uint64_t* twt = nullptr;
+    unsigned char* tmp = nullptr;
+    EKS(sc.get(&z, z_bytes));
+    EKS(sc.get(&S, ids));
+    EKS(sc.get(&sig, n));
+    EKS(sc.get(&cursor, n));
+    EKS(sc.get(&colm, n));
+    EKS(sc.get(&tlist, kIncCap));
+    EKS(sc.get(&tsrc, a.m));
+    if (a.wt) EKS(sc.get(&twt, a.m));
+    EKS(sc.get(&tmp, scan_temp_bytes<uint32_t>((uint64_t)n + 1) + 1024));
+    uint32_t* size = reinterpret_cast<uint32_t*>(z + z_size);
+    uint32_t* deg = reinterpret_cast<uint32_t*>(z + z_deg);
+    IncCounters* ctr = reinterpret_cast<IncCounters*>(z + z_ctr);
+    unsigned long long* best = reinterpret_cast<unsigned long long*>(z + z_best);
+    EK(cudaMemsetAsync(z, 0, z_bytes, s));
+    EK(cudaMemsetAsync(S, 0xff, 8 * ids, s));
+    const unsigned grid = (unsigned)ctx->sm_count * 8;
+    const uint64_t salt = pass_salt1(a.seed, 0x40000000u + r.rounds);
+    rbsc::launch_counter() += 5;
+    k_inc_degrees<<<grid, 256, 0, s>>>(a, col, size, deg);
+    EK((exclusive_scan<uint32_t, uint32_t>(deg, cursor, n, (uint32_t*)nullptr, tmp, s)));
+    if (a.wt) k_inc_transpose<true><<<grid, 256, 0, s>>>(a, col, old, size, cursor, tsrc, twt, best);
+    else k_inc_transpose<false><<<grid, 256, 0, s>>>(a, col, old, size, cursor, tsrc, twt, best);
+    k_inc_mark<<<grid, 256, 0, s>>>(n, col, old, best, colm);
+    if (a.wt) k_inc_sums<true><<<grid, 256, 0, s>>>(a, colm, size, salt, sig, S, tlist, ctr);
+    else k_inc_sums<false><<<grid, 256, 0, s>>>(a, colm, size, salt, sig, S, tlist, ctr);
+    IncArgs t{};
+    t.col = col;
+    t.sig = sig;
+    t.S = S;
+    t.size = size;
+    t.tend = cursor;
+    t.tsrc = tsrc;
+    t.twt = twt;
+    t.tflag = reinterpret_cast<uint32_t*>(z + z_flag);
+    t.tlist = tlist;
+    t.ctr = ctr;
+    t.res = &r;
+    t.salt = salt;
+    t.first_id = (uint32_t)slots;
+    t.round = r.rounds;
+    t.blocks = r.blocks;
+    t.max_rounds = a.max_rounds;
+    const void* k = a.wt ? (const void*)k_inc_passes<true> : (const void*)k_inc_passes<false>;
+    EK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(IncSmem)));
+    if (a.wt) k_inc_passes<true><<<1, 1024, sizeof(IncSmem), s>>>(t);
+    else k_inc_passes<false><<<1, 1024, sizeof(IncSmem), s>>>(t);
+    EK(cudaGetLastError());
+    IncCounters h{};
+    EK(cudaMemcpyAsync(&h, ctr, sizeof h, cudaMemcpyDeviceToHost, s));
+    EK(cudaStreamSynchronize(s));
+    if (h.over) return rbsc_fail(ctx, RBSC_ERR_NOT_CONVERGED, "no fixpoint after %u passes", h.rounds);
+    a.start = col;
+    a.validate = 0;
+    // the pass that found nothing to change is run again in full, to confirm it
+    a.round0 = h.done ? h.rounds - 1u : h.rounds;
+    a.deep_round = h.done ? 0u : 2u * h.rounds;
+    return RBSC_OK;
+}
+
+// The launch, and where it stops early the work-list passes and a launch that
+// confirms them; waits for the stream.  ev[0] and ev[1] enclose it.
+rbsc_status run(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
+{
+    FusedResult& r = *static_cast<FusedResult*>(ctx->h_fused);
+    a.deep_round = deep_round(a.m);
+    EK(cudaEventRecord(ctx->ev[0], s));
+    EKS(launch(ctx, a, s));
+    EK(cudaEventRecord(ctx->ev[1], s));
+    EK(cudaStreamSynchronize(s));
+    const uint32_t initial = r.initial_blocks;
+    const uint64_t t0 = r.t[0], t1 = r.t[1];
+    while (r.status == kFuDeep) {
+        EKS(deep_tail(ctx, a, s));
+        EKS(launch(ctx, a, s));
+        EK(cudaEventRecord(ctx->ev[1], s));
+        EK(cudaStreamSynchronize(s));
+        r.initial_blocks = initial;
+        r.t[0] = t0;
+        r.t[1] = t1;
+    }
+    return RBSC_OK;
+}
+
 // Status and statistics of a finished launch.  *handled false: the exact
 // check met a row with more colours than its table holds; the caller refines
 // the graph launch by launch.
@@ -150,10 +263,7 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
     a.out = d_out;
     a.validate = g->prepared || g->trusted ? 0 : 1;
     common_args(ctx, a);
-    EK(cudaEventRecord(ctx->ev[0], s));
-    EKS(launch(ctx, a, s));
-    EK(cudaEventRecord(ctx->ev[1], s));
-    EK(cudaStreamSynchronize(s));
+    EKS(run(ctx, a, s));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (!g->prepared && !g->trusted) cudaEventElapsedTime(&g->up_ms, ctx->ev[2], ctx->ev[3]);
@@ -168,6 +278,7 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
 rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled)
 {
     *handled = false;
+    const uint64_t lc0 = rbsc::launch_counter();
     if (c->m > kStageBytes / 4 || c->n > kStageNodes) return RBSC_OK;  // before the sizes below are added up
     const uint32_t n = c->n;
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -206,19 +317,17 @@ rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init
     common_args(ctx, a);
     EK(cudaEventRecord(ctx->ev[2], s));
     EK(cudaMemcpyAsync(din, h, in, cudaMemcpyHostToDevice, s));
-    EK(cudaEventRecord(ctx->ev[0], s));
-    EKS(launch(ctx, a, s));
-    EK(cudaEventRecord(ctx->ev[1], s));
-    EK(cudaStreamSynchronize(s));
+    EK(cudaEventRecord(ctx->ev[3], s));
+    EKS(run(ctx, a, s));
     float ms = 0.f, up = 0.f;
-    cudaEventElapsedTime(&up, ctx->ev[2], ctx->ev[0]);
+    cudaEventElapsedTime(&up, ctx->ev[2], ctx->ev[3]);
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (stats) std::memset(stats, 0, sizeof *stats);
     EKS(outcome(ctx, stats, ms, handled));
     if (!*handled) return RBSC_OK;
     if (out) std::memcpy(out, h_out, 4 * (size_t)n);
     if (stats) {
-        stats->kernel_launches = 1;
+        stats->kernel_launches = rbsc::launch_counter() - lc0;
         stats->h2d_ms = up;
         stats->h2d_bytes = b_off + b_idx + b_wt + b_init;
         stats->d2h_bytes = out ? 4ull * n : 0;

@@ -65,7 +65,8 @@ constexpr uint32_t kFuWideSlots = 32768;    // per block, in global memory: any 
 
 // outcome of a launch (FusedResult.status)
 // kFuRowTooWide: the launcher takes the launch-per-phase path
-constexpr int kFuOk = 0, kFuBadOffsets = 1, kFuBadHead = 2, kFuNotConverged = 3, kFuRowTooWide = 4, kFuBarrier = 5;
+constexpr int kFuOk = 0, kFuBadOffsets = 1, kFuBadHead = 2, kFuNotConverged = 3, kFuRowTooWide = 4, kFuBarrier = 5,
+              kFuDeep = 6;  // stopped after deep_round passes or more: the last ones changed little (deep_kernels.cuh)
 
 // Counters of one launch, zero at its start (zeroed by the launcher, or by
 // block 0 of a cluster).
@@ -93,6 +94,7 @@ struct FusedArgs {
     const uint32_t* idx;
     const uint64_t* wt;
     const uint32_t* init;
+    const uint32_t* start; // classes to start from instead of init's (a continued refinement), or null
     uint32_t* out;
     uint32_t* col[2];
     unsigned long long* tab[3];
@@ -114,8 +116,12 @@ struct FusedArgs {
     uint64_t seed;
     uint32_t max_rounds;
     uint32_t hash_bits;
+    uint32_t round0;       // passes already run
+    uint32_t deep_round;   // from this pass on stop (kFuDeep) when a pass made few new classes; 0: never
     uint8_t off64, validate, verify;
 };
+
+constexpr uint32_t kFuDeepNew = 256;  // "few": at most this many
 
 __device__ __forceinline__ uint64_t fu_off(const FusedArgs& a, uint32_t u)
 {
@@ -501,6 +507,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
     clear_tab(a.tab[0]);
     clear_tab(a.tab[1]);
     clear_min();
+    const uint32_t* __restrict__ const ini = a.start ? a.start : a.init;
     uint32_t bad_in = 0;
     for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
         const uint32_t u = base + lane;
@@ -510,7 +517,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
             b = fu_off(a, u);
             e = fu_off(a, u + 1);
             bad = a.validate && (b > e || e > a.m || (u == 0 && b != 0) || (u == n - 1 && e != a.m));
-            if (!a.init) a.col[0][u] = 0u;
+            if (!ini) a.col[0][u] = 0u;
         }
         // (with a bad row anywhere nothing below is used)
         const uint32_t d = bad ? 0u : (uint32_t)(e - b);
@@ -553,12 +560,12 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         return *(volatile uint32_t*)&s_sum;
     };
     uint32_t prev = 1;
-    bool has_classes = a.init != nullptr;
-    if (a.init) {
+    bool has_classes = ini != nullptr;
+    if (ini) {
         for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
             const uint32_t u = base + lane;
             const bool valid = u < n;
-            const uint64_t fp = valid ? ((uint64_t)__ldg(a.init + u) + 1ull) << 1 : 0ull;
+            const uint64_t fp = valid ? ((uint64_t)__ldcg(ini + u) + 1ull) << 1 : 0ull;
             const uint32_t s = fu_insert_warp(valid, true, a.tab[0], a.log2tab, fp, s_cache, made);
             if (valid) a.col[0][u] = s;
         }
@@ -571,12 +578,12 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
     const uint32_t initial = prev;
     if (first) {
         t1 = fu_timer();
-        if (a.res) a.res->round_blocks[0] = prev;
+        if (a.res && !a.start) a.res->round_blocks[0] = prev;
     }
 
     // one pass from col[p & 1] to the other array; REPAIR: the key is (colour,
     // failed) instead of (colour, signature).  Returns false on a timeout.
-    uint32_t round = 0, repairs = 0, count = 0;
+    uint32_t round = a.round0, repairs = 0, count = 0;
     auto pass = [&](bool repair) -> bool {
         const uint32_t* __restrict__ co = a.col[p & 1u];
         uint32_t* __restrict__ cn = a.col[(p & 1u) ^ 1u];
@@ -745,12 +752,18 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
             }
             ++round;
             const bool done = count == prev;
+            const bool little = count - prev <= kFuDeepNew;
             prev = count;
             if (first && a.res && round < (uint32_t)kRoundLog) a.res->round_blocks[round] = count;
             if (done) break;
             if (round >= a.max_rounds) {
                 status = kFuNotConverged;
                 break;
+            }
+            if (a.deep_round && round >= a.deep_round && little && repairs == 0u) {
+                if (first) t2 = fu_timer();
+                finish(kFuDeep, round, prev, initial, repairs);
+                return;
             }
         }
         if (first) t2 = fu_timer();

@@ -183,3 +183,58 @@ def test_device_pointers_and_small_offsets():
         assert r.blocks == ex.blocks and np.array_equal(d_out.cpu().numpy().view(np.uint32), ex.labels)
         g.free()
         _same(ctx.refine(off.astype(np.uint32), idx, None, init), ex)
+
+
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("chain", [40, 64, 65, 700])
+@pytest.mark.parametrize("nodes", [3, 300])
+def test_many_rounds(nodes, chain, weighted):
+    """Enough passes for the work-list tail: a chain beside a lift whose blocks
+    keep several nodes (chains hang off every copy, so whole blocks move)."""
+    lift = 6
+    off, idx = G.random_lift(nodes, 2 * nodes, lift, seed=chain)
+    n = len(off) - 1
+    s, d = G.arcs_of(off, idx)
+    k = np.arange(chain - 1)
+    src, dst = [s, np.arange(lift)], [d, np.full(lift, n)]  # the copies of base node 0 point at the chain
+    for c in range(3):  # three equal chains: their nodes share blocks
+        src.append(n + c * chain + k)
+        dst.append(n + c * chain + k + 1)
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    perm = np.random.default_rng(chain).permutation(n + 3 * chain)
+    off2, idx2, wt2 = G.csr_from_arcs(n + 3 * chain, perm[src], perm[dst], np.full(len(src), 3) if weighted else None)
+    ex = oracle.refine_exact(off2, idx2, wt2)
+    assert ex.rounds >= chain // 2
+    with R.Context(0) as ctx:
+        for _ in range(2):
+            _same(ctx.refine(off2, idx2, wt2), ex)
+        g = ctx.upload(off2, idx2, wt2)
+        _same(g.refine(), ex)
+        g.free()
+        ctx.set_opts(max_rounds=ex.rounds - 1)
+        with pytest.raises(R.RbscError, match="no fixpoint"):
+            ctx.refine(off2, idx2, wt2)
+        ctx.set_opts(max_rounds=ex.rounds)
+        _same(ctx.refine(off2, idx2, wt2), ex)
+
+
+def test_many_rounds_with_wide_passes():
+    """Passes that change more sums than the work list holds go back to full
+    passes: 1,500 chains of 60 nodes, each node pointed at by two more."""
+    c, k = 1500, 60
+    base = np.arange(c * k).reshape(c, k)
+    src = np.concatenate([base[:, :-1].ravel(), c * k + base.ravel(), 2 * c * k + base.ravel()])
+    dst = np.concatenate([base[:, 1:].ravel(), base.ravel(), base.ravel()])
+    init = np.zeros(3 * c * k, np.uint32)
+    off, idx, _ = G.csr_from_arcs(3 * c * k, src, dst)
+    ex = oracle.refine_exact(off, idx, None, init)
+    assert ex.rounds >= 55
+    with R.Context(0) as ctx:
+        _same(ctx.refine(off, idx, None, init), ex)
+
+
+@pytest.mark.parametrize("n", [1, 2, 40, 1025, 6000])
+def test_paths_and_cycles(n):
+    for off, idx in ((G.path(n), G.cycle(n)) if n > 1 else (G.cycle(n),)):
+        with R.Context(0) as ctx:
+            _same(ctx.refine(off, idx), oracle.refine_exact(off, idx))
