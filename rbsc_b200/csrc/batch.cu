@@ -233,8 +233,8 @@ extern "C" rbsc_status rbsc_batch_refine(rbsc_ctx* ctx, const rbsc_csr* graphs, 
     if (!ctx) return rbsc_fail(nullptr, RBSC_ERR_INVALID, "null context");
     auto t0 = std::chrono::steady_clock::now();
     rbsc_graph* g = nullptr;
-    rbsc_status st = graphs && fused_wanted(ctx, graphs->n, graphs->m) ? graph_upload_unprepared(ctx, graphs, &g, nullptr, nullptr)
-                                                                      : rbsc_graph_upload(ctx, graphs, &g);
+    const bool one = graphs && fused_wanted(ctx, graphs->n, graphs->m, graphs->weights != nullptr, false);
+    rbsc_status st = one ? graph_upload_unprepared(ctx, graphs, &g, nullptr, nullptr) : rbsc_graph_upload(ctx, graphs, &g);
     if (st != RBSC_OK) return st;
     g->oneshot = true;
     st = rbsc_graph_batch_refine(ctx, g, graph_nodes, num_graphs, init_colors, out, stats);

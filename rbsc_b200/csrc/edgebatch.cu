@@ -272,7 +272,7 @@ rbsc_status refine_batch(rbsc_ctx* ctx, const Runs& rs, uint32_t n, uint32_t k0,
     ++rbsc::launch_counter();
     k_eb_mark_sources<<<grid_of(k1 - k0), 256, 0, s>>>(k0, k1, rs.rsrc, col);
     EK(cudaGetLastError());
-    if (fused_wanted(ctx, g->n, g->m)) g->trusted = true;  // built here: nothing to check, no tiling
+    if (fused_wanted(ctx, g->n, g->m, g->weighted, false)) g->trusted = true;  // built here: nothing to check, no tiling
     else EKS(graph_prepare(ctx, g));
     rbsc_stats st;
     EKS(refine_resident(ctx, g, col, lab, &st, nullptr));

@@ -231,9 +231,19 @@ rbsc_status outcome(rbsc_ctx* ctx, rbsc_stats* stats, float ms, bool* handled)
 
 }  // namespace
 
-bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m)
+// Below 2^22 arcs one launch always wins.  Above, the tile fold of the
+// launch-per-phase path catches up, first where it has more to offer (rival:
+// hot heads, or heads whose copy overlaps the first pass).  us a refinement,
+// one launch / launch per phase, uniform start: R-MAT-20 with 16 M arcs 487 /
+// 626, R-MAT-21 with 32 M 918 / 810; weighted (whose rows the launch-per-phase
+// check sorts) R-MAT-20 511 / 938 and R-MAT-21 947 / 1220 from degree colours,
+// R-MAT-22 with 65 M 1933 / 1852.
+constexpr uint64_t kSmallArcs = 1ull << 22, kLargeArcs = 3ull << 23, kLargeWeighted = 1ull << 25;
+
+bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m, bool weighted, bool rival)
 {
-    if (!default_knobs(ctx->opts) || n == 0 || n > (1u << 22) || m >= (1ull << 22)) return false;
+    if (!default_knobs(ctx->opts) || n == 0 || n > kIncMaxNodes) return false;
+    if (m >= kSmallArcs && (rival || m >= (weighted ? kLargeWeighted : kLargeArcs))) return false;
     // a cooperative grid needs the chip to itself; a cluster does not
     if (ctx->shared_gpu) return n <= kSharedNodes && m <= kSharedArcs;
     return !ctx->opts.no_persist;
@@ -285,7 +295,7 @@ rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init
     const size_t b_off = (size_t)c->offset_bytes * ((size_t)n + 1), b_idx = 4 * (size_t)c->m, b_wt = c->weights ? 8 * (size_t)c->m : 0,
                  b_init = init ? 4 * (size_t)n : 0;
     const size_t in = al(b_off) + al(b_idx) + al(b_wt) + al(b_init);
-    if (!fused_wanted(ctx, n, c->m) || in > kStageBytes) return RBSC_OK;
+    if (!fused_wanted(ctx, n, c->m, c->weights != nullptr, false) || in > kStageBytes) return RBSC_OK;
     const auto t0 = std::chrono::steady_clock::now();
     EK(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;

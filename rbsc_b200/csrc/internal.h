@@ -240,10 +240,11 @@ struct Scratch {
         if (s_ != RBSC_OK) return s_;  \
     } while (0)
 
-// The one-launch refinement of small graphs (fused.cu).  fused_wanted: the
-// context's options and the sizes allow it.  *handled false on RBSC_OK: it
+// The one-launch refinement (fused.cu).  fused_wanted: the context's options
+// and the sizes allow it; rival: a large graph would get hot heads or an
+// overlapped upload on the launch-per-phase path.  *handled false on RBSC_OK: it
 // does not apply after all, and the caller takes the launch-per-phase path.
-bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m);
+bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m, bool weighted, bool rival);
 rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled);
 rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled);
 

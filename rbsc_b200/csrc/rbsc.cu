@@ -1133,10 +1133,7 @@ static rbsc_status launch_pass(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s, cud
         ++rbsc::launch_counter();
         if (first == kPassUniform) {
             const unsigned ugrid = persistent_grid(ctx, g->K, kNodeThreads);
-            if (g->weighted)
-                k_signature_uniform<true><<<ugrid, kNodeThreads, 0, s>>>(g->d_as, g->d_st, g->d_off, g->d_wt, c0, g->d_sig);
-            else
-                k_signature_uniform<false><<<ugrid, kNodeThreads, 0, s>>>(g->d_as, g->d_st, g->d_off, g->d_wt, c0, g->d_sig);
+            k_signature_uniform<<<ugrid, kNodeThreads, 0, s>>>(g->d_as, g->d_st, g->d_off, c0, g->d_sig);
         } else if (staged_signature(ctx, g)) {
             const TileRange all{0u, 0u, nullptr, nullptr, 0ull};
             if (first == kPassRank8)
@@ -1691,7 +1688,7 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         if (stats) stats->done = stats->verified = 1;
         return RBSC_OK;
     }
-    if (!kt && !g->host_arcs && fused_wanted(ctx, n, g->m)) {
+    if (!kt && !g->host_arcs && !g->stream_upload && fused_wanted(ctx, n, g->m, g->weighted, d_init && !g->oneshot)) {
         bool handled = false;
         CKS(fused_refine(ctx, g, d_init, d_out, stats, &handled));
         if (handled) return RBSC_OK;
@@ -1773,7 +1770,10 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
     int first = kPassFull;
     uint32_t c0 = 0;
     if (g->m > 0 && ctx->opts.relabel != RBSC_RELABEL_SORT) {
-        if (initial_blocks == 1) {
+        if (initial_blocks == 1 && g->weighted) {
+            // the rows' weights have to be added up: the tile fold shares a
+            // hub's out (a thread per row took 3.7 ms on R-MAT-20's 16 M arcs)
+        } else if (initial_blocks == 1) {
             first = kPassUniform;
             c0 = 0;  // the one class is labelled by node 0
         } else if (initial_blocks <= 65536) {
@@ -1949,7 +1949,8 @@ extern "C" rbsc_status rbsc_refine(rbsc_ctx* ctx, const rbsc_csr* host_graph, co
     if (handled) return RBSC_OK;
     // large unweighted graphs: the heads' copy overlaps the refinement
     const bool defer = !host_graph->weights && host_graph->m >= (1ull << 22);
-    CKS(graph_load(ctx, host_graph, false, &g, &up_ms, &up_bytes, defer, init_colors, fused_wanted(ctx, host_graph->n, host_graph->m)));
+    CKS(graph_load(ctx, host_graph, false, &g, &up_ms, &up_bytes, defer, init_colors,
+                   fused_wanted(ctx, host_graph->n, host_graph->m, host_graph->weights != nullptr, defer)));
     g->oneshot = true;
     rbsc_status st = rbsc_graph_refine(ctx, g, init_colors, out_labels, stats);
     up_ms += g->up_ms;

@@ -730,14 +730,12 @@ static __global__ void __launch_bounds__(kTileThreads) k_signature_chunk(const A
     signature_body<WEIGHTED, ColT, true, true>(as, st, col, sig, rng);
 }
 
-// First pass when every node starts in one block (the reference's default):
-// every arc's term is the same, so a row's signature is its length (or its
-// total weight) times that term, and no arc needs to be read.
-template <bool WEIGHTED>
+// First pass when every node starts in one block (the reference's default)
+// and every arc weighs 1: every arc's term is the same, so a row's signature
+// is its length times that term, and no arc needs to be read.
 static __global__ void __launch_bounds__(kNodeThreads) k_signature_uniform(const ActiveSet* __restrict__ as,
                                                                            const RoundState* __restrict__ st,
-                                                                           const uint64_t* __restrict__ off,
-                                                                           const uint64_t* __restrict__ wt, uint32_t c0,
+                                                                           const uint64_t* __restrict__ off, uint32_t c0,
                                                                            Sig* __restrict__ sig)
 {
     const uint32_t K = as->K;
@@ -747,18 +745,8 @@ static __global__ void __launch_bounds__(kNodeThreads) k_signature_uniform(const
     arc_terms(c0, pass_salt1(st->seed, st->round), t1, t2);
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < K; k += gridDim.x * blockDim.x) {
         const uint32_t u = rows[k];
-        const uint64_t b = off[u], e = off[u + 1];
-        uint64_t w = e - b;
-        uint32_t w2 = (uint32_t)w;
-        if (WEIGHTED) {
-            w = 0;
-            w2 = 0;
-            for (uint64_t j = b; j < e; ++j) {
-                w += wt[j];
-                w2 += (uint32_t)wt[j];
-            }
-        }
-        sig_store(&sig[u], w * t1, w2 * t2);
+        const uint64_t w = off[u + 1] - off[u];
+        sig_store(&sig[u], w * t1, (uint32_t)w * t2);
     }
 }
 

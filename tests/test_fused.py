@@ -238,3 +238,22 @@ def test_paths_and_cycles(n):
     for off, idx in ((G.path(n), G.cycle(n)) if n > 1 else (G.cycle(n),)):
         with R.Context(0) as ctx:
             _same(ctx.refine(off, idx), oracle.refine_exact(off, idx))
+
+
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("m", [(1 << 22) + 7, 3 << 23])
+def test_large_resident_graphs(m, weighted):
+    """From 2^22 arcs on one launch takes a resident graph with no initial
+    colours (to 24 M arcs, weighted to 32 M), with the other path's result."""
+    off, idx = R.gen_er_host(600000, m / 600000, seed=m & 63)
+    wt = np.random.default_rng(1).integers(0, 4, size=len(idx)).astype(np.uint64) if weighted else None
+    with R.Context(0) as ctx, R.Context(0, persistent=False) as per_phase:
+        for init in (None, R.degree_bucket_colors(off)):
+            g = ctx.upload(off, idx, wt)
+            a = g.refine(init)
+            g.free()
+            b = per_phase.refine(off, idx, wt, init)
+            assert (a.blocks, a.rounds, a.round_blocks) == (b.blocks, b.rounds, b.round_blocks)
+            assert np.array_equal(a.labels, b.labels) and a.verified == b.verified == 1
+            if init is None:
+                assert (a.kernel_launches <= 2) == (len(idx) < (1 << 25 if weighted else 3 << 23))
