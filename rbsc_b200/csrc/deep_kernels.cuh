@@ -58,7 +58,7 @@ static __global__ void k_inc_degrees(FusedArgs a, const uint32_t* __restrict__ c
         const uint32_t c = col[u];
         if (c & kSingleton) continue;
         if (gl == 0) atomicAdd(&size[c], 1u);
-        const uint64_t e = fu_off(a, u + 1);
+        const uint64_t e = fu_end(a, u);
         for (uint64_t i = fu_off(a, u) + gl; i < e; i += 8) {
             const uint32_t v = a.idx[i];
             if (!(col[v] & kSingleton)) atomicAdd(&indeg[v], 1u);
@@ -81,7 +81,7 @@ static __global__ void k_inc_transpose(FusedArgs a, const uint32_t* __restrict__
             const unsigned long long v = ((unsigned long long)size[c] << 32) | c;
             if (__ldcg(&best[old[u]]) < v) atomicMax(&best[old[u]], v);
         }
-        const uint64_t e = fu_off(a, u + 1);
+        const uint64_t e = fu_end(a, u);
         for (uint64_t i = fu_off(a, u) + gl; i < e; i += 8) {
             const uint32_t v = a.idx[i];
             if (col[v] & kSingleton) continue;
@@ -116,7 +116,7 @@ static __global__ void k_inc_sums(FusedArgs a, const uint32_t* __restrict__ colm
         uint64_t s = 0;
         uint32_t touched = 0;
         if (act) {
-            const uint64_t e = fu_off(a, u + 1);
+            const uint64_t e = fu_end(a, u);
             for (uint64_t i = fu_off(a, u) + gl; i < e; i += 8) {
                 const uint32_t w = colm[a.idx[i]];
                 touched |= w & kIncMark;

@@ -79,6 +79,18 @@ __global__ void k_eb_local_deg(uint32_t k0, uint32_t k1, const uint32_t* __restr
         deg[rsrc[k]] = roff[k + 1] - roff[k];
 }
 
+// rows of runs [k0, k1) where they lie in the arc list, from arc a0 on (nodes
+// without a run: an empty row, cleared before)
+__global__ void k_eb_local_rows(uint32_t k0, uint32_t k1, uint64_t a0, const uint32_t* __restrict__ rsrc,
+                                const uint64_t* __restrict__ roff, uint32_t* __restrict__ begin, uint32_t* __restrict__ end)
+{
+    for (uint64_t k = k0 + blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < k1; k += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t u = rsrc[k];
+        begin[u] = (uint32_t)(roff[k] - a0);
+        end[u] = (uint32_t)(roff[k + 1] - a0);
+    }
+}
+
 __global__ void k_eb_local_fill(uint32_t k0, uint32_t k1, const uint32_t* __restrict__ rsrc, const uint64_t* __restrict__ roff,
                                 const uint32_t* __restrict__ dst, const uint64_t* __restrict__ wt,
                                 const uint64_t* __restrict__ loff, uint32_t* __restrict__ lidx, uint64_t* __restrict__ lwt)
@@ -151,7 +163,7 @@ __global__ void k_eb_first_run(uint32_t R, const uint32_t* __restrict__ rsrc, co
                                uint32_t* __restrict__ first)
 {
     for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < R; k += (uint64_t)gridDim.x * blockDim.x)
-        atomicMin(&first[w[rsrc[k]]], (uint32_t)k);
+        if (*(volatile uint32_t*)&first[w[rsrc[k]]] > (uint32_t)k) atomicMin(&first[w[rsrc[k]]], (uint32_t)k);
 }
 
 __global__ void k_eb_keep(uint32_t R, const uint32_t* __restrict__ rsrc, const uint32_t* __restrict__ w,
@@ -165,22 +177,52 @@ __global__ void k_eb_keep(uint32_t R, const uint32_t* __restrict__ rsrc, const u
     }
 }
 
-// keys (kept run rank << 32 | head class), values weights; one warp per run
-__global__ void k_eb_keys(uint32_t R, const uint64_t* __restrict__ roff, const uint32_t* __restrict__ dst,
-                          const uint64_t* __restrict__ wt, const uint32_t* __restrict__ w, const uint32_t* __restrict__ keep,
-                          const uint32_t* __restrict__ krank, const uint64_t* __restrict__ kpos,
-                          unsigned long long* __restrict__ keys, unsigned long long* __restrict__ vals)
+// keys (kept run rank << cb | head class), values weights; a block per tile of
+// arcs, whose runs' starts it looks up once (a warp per run: 0.62 ms on
+// R-MAT-20's 16 M arcs, most lanes idle on short runs; eight lanes per run 2.0
+// ms, waiting for the hubs)
+constexpr uint32_t kEbTile = 2048;
+
+__global__ void __launch_bounds__(256) k_eb_keys(uint32_t R, uint64_t E, uint32_t cb, const uint64_t* __restrict__ roff,
+                                                 const uint32_t* __restrict__ dst, const uint64_t* __restrict__ wt,
+                                                 const uint32_t* __restrict__ w, const uint32_t* __restrict__ keep,
+                                                 const uint32_t* __restrict__ krank, const uint64_t* __restrict__ kpos,
+                                                 unsigned long long* __restrict__ keys, unsigned long long* __restrict__ vals)
 {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t k = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; k < R; k += warps) {
-        if (!keep[k]) continue;
-        const uint64_t a = roff[k], len = roff[k + 1] - a, o = kpos[k];
-        const unsigned long long hi = (unsigned long long)krank[k] << 32;
-        for (uint64_t j = lane; j < len; j += 32) {
-            keys[o + j] = hi | w[dst[a + j]];
-            vals[o + j] = wt ? wt[a + j] : 1ull;
+    __shared__ uint32_t s_start[kEbTile];  // tile position of each run's first arc in the tile
+    __shared__ uint32_t s_run[2];
+    for (uint64_t t0 = (uint64_t)blockIdx.x * kEbTile; t0 < E; t0 += (uint64_t)gridDim.x * kEbTile) {
+        const uint64_t t1 = min(E, t0 + kEbTile);
+        if (threadIdx.x < 2) {
+            // the runs of the tile's first and last arc (no run is empty)
+            const uint64_t e = threadIdx.x ? t1 - 1 : t0;
+            uint32_t lo = 0, hi = R - 1;
+            while (lo < hi) {
+                const uint32_t mid = lo + ((hi - lo + 1) >> 1);
+                if (roff[mid] <= e) lo = mid;
+                else hi = mid - 1;
+            }
+            s_run[threadIdx.x] = lo;
         }
+        __syncthreads();
+        const uint32_t k0 = s_run[0], cnt = s_run[1] - k0 + 1u;
+        for (uint32_t i = threadIdx.x; i < cnt; i += 256) s_start[i] = (uint32_t)(max(roff[k0 + i], t0) - t0);
+        __syncthreads();
+        for (uint64_t e = t0 + threadIdx.x; e < t1; e += 256) {
+            const uint32_t x = (uint32_t)(e - t0);
+            uint32_t lo = 0, hi = cnt - 1;
+            while (lo < hi) {
+                const uint32_t mid = lo + ((hi - lo + 1) >> 1);
+                if (s_start[mid] <= x) lo = mid;
+                else hi = mid - 1;
+            }
+            const uint32_t k = k0 + lo;
+            if (!keep[k]) continue;
+            const uint64_t o = kpos[k] + (e - roff[k]);
+            keys[o] = ((unsigned long long)krank[k] << cb) | w[dst[e]];
+            vals[o] = wt ? wt[e] : 1ull;
+        }
+        __syncthreads();
     }
 }
 
@@ -191,7 +233,7 @@ __global__ void k_eb_heads(uint64_t n, const unsigned long long* __restrict__ ke
 }
 
 // one merged arc per segment of equal keys; a new run where the run rank changes
-__global__ void k_eb_merge(uint64_t n, const unsigned long long* __restrict__ keys, const unsigned long long* __restrict__ vals,
+__global__ void k_eb_merge(uint64_t n, uint32_t cb, const unsigned long long* __restrict__ keys, const unsigned long long* __restrict__ vals,
                            const uint32_t* __restrict__ head, const uint64_t* __restrict__ hpos, uint32_t* __restrict__ ndst,
                            uint64_t* __restrict__ nwt, uint64_t* __restrict__ nroff)
 {
@@ -201,9 +243,9 @@ __global__ void k_eb_merge(uint64_t n, const unsigned long long* __restrict__ ke
         unsigned long long s = vals[i];
         for (uint64_t j = i + 1; j < n && keys[j] == k; ++j) s += vals[j];
         const uint64_t p = hpos[i];
-        ndst[p] = (uint32_t)k;
+        ndst[p] = (uint32_t)(k & ((1ull << cb) - 1ull));
         nwt[p] = s;
-        if (i == 0 || (keys[i - 1] >> 32) != (k >> 32)) nroff[k >> 32] = p;
+        if (i == 0 || (keys[i - 1] >> cb) != (k >> cb)) nroff[k >> cb] = p;
     }
 }
 
@@ -218,7 +260,7 @@ __global__ void k_eb_new_src(uint32_t R, const uint32_t* __restrict__ rsrc, cons
 __global__ void k_eb_min_node(uint32_t n, const uint32_t* __restrict__ cls, uint32_t* __restrict__ first)
 {
     for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x)
-        atomicMin(&first[cls[u]], (uint32_t)u);
+        if (*(volatile uint32_t*)&first[cls[u]] > (uint32_t)u) atomicMin(&first[cls[u]], (uint32_t)u);  // few nodes lower it
 }
 
 __global__ void k_eb_labels(uint32_t n, const uint32_t* __restrict__ cls, const uint32_t* __restrict__ first,
@@ -240,14 +282,34 @@ struct Runs {
 
 // The local graph of runs [k0, k1) over n nodes, refined exactly from the
 // batch's initial colours; canonical labels into lab.
-rbsc_status refine_batch(rbsc_ctx* ctx, const Runs& rs, uint32_t n, uint32_t k0, uint32_t k1, const uint8_t* has, bool first_batch,
-                         uint32_t* col, uint32_t* lab, uint32_t* rounds)
+rbsc_status refine_batch(rbsc_ctx* ctx, const Runs& rs, uint32_t n, uint32_t k0, uint32_t k1, uint64_t a0, uint64_t a1,
+                         const uint8_t* has, bool first_batch, uint32_t* col, uint32_t* lab, uint32_t* rounds)
 {
     cudaStream_t s = ctx->stream;
-    uint64_t a0 = 0, a1 = 0;
-    EK(cudaMemcpyAsync(&a0, rs.roff + k0, 8, cudaMemcpyDeviceToHost, s));
-    EK(cudaMemcpyAsync(&a1, rs.roff + k1, 8, cudaMemcpyDeviceToHost, s));
-    EK(cudaStreamSynchronize(s));
+    ++rbsc::launch_counter();
+    k_eb_local_init<<<grid_of(n), 256, 0, s>>>(n, has, first_batch ? 1 : 0, col);
+    ++rbsc::launch_counter();
+    k_eb_mark_sources<<<grid_of(k1 - k0), 256, 0, s>>>(k0, k1, rs.rsrc, col);
+    EK(cudaGetLastError());
+    if (fused_wanted(ctx, n, a1 - a0, rs.wt != nullptr, false)) {
+        // refined where the runs lie: no local copy of the arcs (0.26 ms per
+        // batch of R-MAT-20 in quarters), no check and no tiling
+        Scratch sc(ctx);
+        uint32_t* rows = nullptr;
+        EKS(sc.get(&rows, 2 * (size_t)n));
+        EK(cudaMemsetAsync(rows, 0, 8 * (size_t)n, s));
+        ++rbsc::launch_counter();
+        k_eb_local_rows<<<grid_of(k1 - k0), 256, 0, s>>>(k0, k1, a0, rs.rsrc, rs.roff, rows, rows + n);
+        EK(cudaGetLastError());
+        const FusedRows fr{n, a1 - a0, rows, rows + n, rs.dst + a0, rs.wt ? rs.wt + a0 : nullptr};
+        rbsc_stats st;
+        bool handled = false;
+        EKS(fused_refine_rows(ctx, fr, col, lab, &st, &handled));
+        if (handled) {
+            *rounds += st.rounds;
+            return RBSC_OK;
+        }
+    }
     rbsc_graph* g = new (std::nothrow) rbsc_graph();
     if (!g) return rbsc_fail(ctx, RBSC_ERR_OOM, "out of host memory");
     struct Free { rbsc_graph* g; ~Free() { rbsc_graph_free(g); } } guard{g};
@@ -267,13 +329,8 @@ rbsc_status refine_batch(rbsc_ctx* ctx, const Runs& rs, uint32_t n, uint32_t k0,
     ++rbsc::launch_counter();
     k_eb_local_fill<<<grid_of((uint64_t)(k1 - k0) * 32), 256, 0, s>>>(k0, k1, rs.rsrc, rs.roff, rs.dst, rs.wt, g->d_off, g->d_idx,
                                                                     g->d_wt);
-    ++rbsc::launch_counter();
-    k_eb_local_init<<<grid_of(n), 256, 0, s>>>(n, has, first_batch ? 1 : 0, col);
-    ++rbsc::launch_counter();
-    k_eb_mark_sources<<<grid_of(k1 - k0), 256, 0, s>>>(k0, k1, rs.rsrc, col);
     EK(cudaGetLastError());
-    if (fused_wanted(ctx, g->n, g->m, g->weighted, false)) g->trusted = true;  // built here: nothing to check, no tiling
-    else EKS(graph_prepare(ctx, g));
+    EKS(graph_prepare(ctx, g));
     rbsc_stats st;
     EKS(refine_resident(ctx, g, col, lab, &st, nullptr));
     *rounds += st.rounds;
@@ -372,7 +429,7 @@ extern "C" rbsc_status rbsc_refine_edge_batches(rbsc_ctx* ctx, const rbsc_csr* h
             if (k0 >= cur.R || roff_h[k0] >= be) continue;
             const uint32_t k1 = (uint32_t)(std::upper_bound(roff_h.begin() + k0, roff_h.end(), be) - roff_h.begin()) - 1;
             if (k1 <= k0) continue;
-            EKS(refine_batch(ctx, cur, node_n, k0, k1, has, b == 0, col, lab, &rounds));
+            EKS(refine_batch(ctx, cur, node_n, k0, k1, roff_h[k0], roff_h[k1], has, b == 0, col, lab, &rounds));
             ++refinements;
             // fresh ids for the batch's classes, in the order of their smallest node
             ++rbsc::launch_counter();
@@ -434,13 +491,14 @@ extern "C" rbsc_status rbsc_refine_edge_batches(rbsc_ctx* ctx, const rbsc_csr* h
         EKS(q.get(&vals, E2));
         EKS(q.get(&vals2, E2));
         ++rbsc::launch_counter();
-        k_eb_keys<<<grid_of((uint64_t)cur.R * 32), 256, 0, s>>>(cur.R, cur.roff, cur.dst, cur.wt, w, keep, krank, klen, keys, vals);
+        const uint32_t cb = std::max(1u, 32u - (uint32_t)__builtin_clz(std::max(1u, new_node_n - 1u)));  // class bits of a key
+        k_eb_keys<<<grid_of(cur.E, kEbTile), 256, 0, s>>>(cur.R, cur.E, cb, cur.roff, cur.dst, cur.wt, w, keep, krank, klen, keys, vals);
         EK(cudaGetLastError());
         int rbits = 0;
         while (rbits < 32 && (1ull << rbits) < (uint64_t)R2) ++rbits;
         EKS(need_tmp(std::max(radix_temp_bytes(E2), scan_temp_bytes<uint64_t>(E2 + 1)) + 1024));
         bool alt = false;
-        EK(radix_sort<unsigned long long>(keys, keys2, vals, vals2, E2, 0, 32 + rbits, tmp, s, &alt));
+        EK(radix_sort<unsigned long long>(keys, keys2, vals, vals2, E2, 0, (int)cb + rbits, tmp, s, &alt));
         if (alt) {
             std::swap(keys, keys2);
             std::swap(vals, vals2);
@@ -463,7 +521,7 @@ extern "C" rbsc_status rbsc_refine_edge_batches(rbsc_ctx* ctx, const rbsc_csr* h
         EKS(sc.get(&nr.dst, E3));
         EKS(sc.get(&nr.wt, E3));
         ++rbsc::launch_counter();
-        k_eb_merge<<<grid_of(E2), 256, 0, s>>>(E2, keys, vals, head, hpos, nr.dst, nr.wt, nr.roff);
+        k_eb_merge<<<grid_of(E2), 256, 0, s>>>(E2, cb, keys, vals, head, hpos, nr.dst, nr.wt, nr.roff);
         ++rbsc::launch_counter();
         k_eb_new_src<<<grid_of(cur.R), 256, 0, s>>>(cur.R, cur.rsrc, w, keep, krank, nr.rsrc);
         EK(cudaGetLastError());

@@ -265,21 +265,47 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
     fused_bind(a, l, static_cast<unsigned char*>(g->d_fused));
     a.n = g->n;
     a.m = g->m;
-    a.off = g->d_off;
-    a.off64 = 1;
+    fused_csr(a, g->d_off, true);
     a.idx = g->d_idx;
     a.wt = g->weighted ? g->d_wt : nullptr;
     a.init = d_init;
     a.out = d_out;
-    a.validate = g->prepared || g->trusted ? 0 : 1;
+    a.validate = g->prepared ? 0 : 1;
     common_args(ctx, a);
     EKS(run(ctx, a, s));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
-    if (!g->prepared && !g->trusted) cudaEventElapsedTime(&g->up_ms, ctx->ev[2], ctx->ev[3]);
+    if (!g->prepared) cudaEventElapsedTime(&g->up_ms, ctx->ev[2], ctx->ev[3]);
     EKS(outcome(ctx, stats, ms, handled));
     if (stats && *handled) stats->kernel_launches = rbsc::launch_counter() - lc0;
     return RBSC_OK;
+}
+
+rbsc_status fused_refine_rows(rbsc_ctx* ctx, const FusedRows& r, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled)
+{
+    *handled = false;
+    cudaStream_t s = ctx->stream;
+    const FusedLayout l = fused_layout(r.n, r.m);
+    Scratch sc(ctx);
+    unsigned char* d = nullptr;
+    EKS(sc.get(&d, l.bytes));
+    EKS(ensure_pinned(ctx));
+    FusedArgs a{};
+    fused_bind(a, l, d);
+    a.n = r.n;
+    a.m = r.m;
+    a.off = r.begin;
+    a.off_end = r.end;
+    a.idx = r.idx;
+    a.wt = r.wt;
+    a.init = d_init;
+    a.out = d_out;
+    common_args(ctx, a);
+    EKS(run(ctx, a, s));
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+    if (stats) std::memset(stats, 0, sizeof *stats);
+    return outcome(ctx, stats, ms, handled);
 }
 
 // A small host graph, labels back in host memory: the arrays are gathered in a
@@ -317,8 +343,7 @@ rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init
     fused_bind(a, l, d);
     a.n = n;
     a.m = c->m;
-    a.off = din;
-    a.off64 = c->offset_bytes == 8;
+    fused_csr(a, din, c->offset_bytes == 8);
     a.idx = reinterpret_cast<const uint32_t*>(din + o_idx);
     a.wt = b_wt ? reinterpret_cast<const uint64_t*>(din + o_wt) : nullptr;
     a.init = b_init ? reinterpret_cast<const uint32_t*>(din + o_init) : nullptr;

@@ -90,7 +90,8 @@ struct FusedResult {
 struct FusedArgs {
     uint32_t n;
     uint64_t m;
-    const void* off;
+    const void* off;       // where each row starts; rows may lie anywhere in idx
+    const void* off_end;   // where it ends (CSR offsets: off + 1 entry)
     const uint32_t* idx;
     const uint64_t* wt;
     const uint32_t* init;
@@ -123,11 +124,12 @@ struct FusedArgs {
 
 constexpr uint32_t kFuDeepNew = 256;  // "few": at most this many
 
-__device__ __forceinline__ uint64_t fu_off(const FusedArgs& a, uint32_t u)
+__device__ __forceinline__ uint64_t fu_ld(const void* p, bool wide, uint32_t u)
 {
-    return a.off64 ? __ldg(reinterpret_cast<const unsigned long long*>(a.off) + u)
-                   : (uint64_t)__ldg(reinterpret_cast<const uint32_t*>(a.off) + u);
+    return wide ? __ldg(reinterpret_cast<const unsigned long long*>(p) + u) : (uint64_t)__ldg(reinterpret_cast<const uint32_t*>(p) + u);
 }
+__device__ __forceinline__ uint64_t fu_off(const FusedArgs& a, uint32_t u) { return fu_ld(a.off, a.off64, u); }
+__device__ __forceinline__ uint64_t fu_end(const FusedArgs& a, uint32_t u) { return fu_ld(a.off_end, a.off64, u); }
 
 // Whether a row of d arcs in a group of `group` arcs goes in chunks.
 __device__ __forceinline__ bool fu_shared_row(uint32_t d, uint32_t group)
@@ -515,7 +517,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         bool bad = false;
         if (u < n) {
             b = fu_off(a, u);
-            e = fu_off(a, u + 1);
+            e = fu_end(a, u);
             bad = a.validate && (b > e || e > a.m || (u == 0 && b != 0) || (u == n - 1 && e != a.m));
             if (!ini) a.col[0][u] = 0u;
         }
@@ -614,7 +616,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
             uint32_t d = 0;
             if (valid && !repair) {
                 b = fu_off(a, u);
-                d = (uint32_t)(fu_off(a, u + 1) - b);
+                d = (uint32_t)(fu_end(a, u) - b);
             }
             if (act) {
                 if (has_classes) e = __ldcg(tp + c);
@@ -706,7 +708,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
                 const uint32_t j = a.lchunk[ch], u = a.lrow[j], f = a.lfirst[j];
                 const uint32_t c = __ldcg(co + u);
                 if ((c & kSingleton) || (has_classes && !(__ldcg(tp + c) & 1ull)) || n == 1u) continue;
-                const uint64_t b = fu_off(a, u), e = fu_off(a, u + 1);
+                const uint64_t b = fu_off(a, u), e = fu_end(a, u);
                 const uint64_t s = b + (uint64_t)(ch - f) * kFuChunk, t = min(e, s + kFuChunk);
                 uint64_t sum = 0;
 #pragma unroll 8
@@ -795,8 +797,8 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
             if (chk) {
                 bu = fu_off(a, u);
                 br = fu_off(a, r);
-                du = (uint32_t)(fu_off(a, u + 1) - bu);
-                dr = (uint32_t)(fu_off(a, r + 1) - br);
+                du = (uint32_t)(fu_end(a, u) - bu);
+                dr = (uint32_t)(fu_end(a, r) - br);
                 if (a.init) {
                     iu = __ldg(a.init + u);
                     ir = __ldg(a.init + r);
@@ -844,7 +846,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
             auto add_row = [&](uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t x, bool minus, uint32_t at,
                                uint32_t step) -> bool {
                 bool ok = true;
-                const uint64_t b = fu_off(a, x), e = fu_off(a, x + 1);
+                const uint64_t b = fu_off(a, x), e = fu_end(a, x);
                 for (uint64_t i = b + at; i < e; i += step) {
                     const uint64_t v = WEIGHTED ? __ldg(reinterpret_cast<const unsigned long long*>(wt) + i) : 1ull;
                     ok &= fu_count(key, val, mask, __ldcg(col + __ldg(idx + i)), minus ? 0ull - v : v);
@@ -852,7 +854,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
                 return ok;
             };
             auto longest = [&](uint32_t u, uint32_t r) {
-                return max((uint32_t)(fu_off(a, u + 1) - fu_off(a, u)), (uint32_t)(fu_off(a, r + 1) - fu_off(a, r)));
+                return max((uint32_t)(fu_end(a, u) - fu_off(a, u)), (uint32_t)(fu_end(a, r) - fu_off(a, r)));
             };
             if (WEIGHTED) {
                 const uint32_t wi = threadIdx.x >> 5;
@@ -1003,6 +1005,14 @@ inline FusedLayout fused_layout(uint32_t n, uint64_t m)
     l.lchunk = take(4ull * l.chunk_cap);
     l.bytes = at;
     return l;
+}
+
+// The rows of a CSR with offsets of 4 or 8 bytes.
+inline void fused_csr(FusedArgs& a, const void* off, bool off64)
+{
+    a.off = off;
+    a.off_end = static_cast<const char*>(off) + (off64 ? 8 : 4);
+    a.off64 = off64 ? 1 : 0;
 }
 
 inline void fused_bind(FusedArgs& a, const FusedLayout& l, unsigned char* base)

@@ -71,7 +71,6 @@ struct rbsc_graph {
     bool prepared = false;       // checked and tiled (graph_prepare); a graph the one-launch
                                  // refinement takes is checked there and needs no tiling
     float up_ms = 0.f;           // its host-to-device copies, timed by fused_refine
-    bool trusted = false;        // built by the library from a checked graph
 
     void* d_fused = nullptr;     // working memory of the one-launch refinement
 
@@ -246,6 +245,17 @@ struct Scratch {
 // does not apply after all, and the caller takes the launch-per-phase path.
 bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m, bool weighted, bool rival);
 rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled);
+// The same on rows that lie anywhere in the arc arrays (device memory, checked
+// by the caller): row u = arcs [begin[u], end[u]), m arcs in all.
+struct FusedRows {
+    uint32_t n;
+    uint64_t m;
+    const uint32_t* begin;
+    const uint32_t* end;
+    const uint32_t* idx;
+    const uint64_t* wt;
+};
+rbsc_status fused_refine_rows(rbsc_ctx* ctx, const FusedRows& r, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled);
 rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled);
 
 // sort-based relabel (sortrelabel.cu)

@@ -95,8 +95,7 @@ extern "C" rbsc_status rbsc_refine_noalloc(const rbsc_csr* g, const uint32_t* d_
     a.wide = scratch + kNaWork;
     a.n = g->n;
     a.m = g->m;
-    a.off = g->offsets;
-    a.off64 = g->offset_bytes == 8;
+    fused_csr(a, g->offsets, g->offset_bytes == 8);
     a.idx = g->indices;
     a.wt = g->weights;
     a.init = d_init_colors;

@@ -113,3 +113,25 @@ def test_cli_edge_batch_size_matches_reference():
                          check=True).stdout.decode()
     lines = out.strip().splitlines()
     assert (int(lines[1]), int(lines[2])) == (case["done_aggressive"], case["nodes_aggressive"])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("weighted", [False, True], ids=["unit", "weighted"])
+@pytest.mark.parametrize("n,m,batch", [(900, 2047, 1000), (900, 2048, 1024), (700, 4097, 1500), (5000, 30011, 9001)])
+def test_gpu_quotient_tiles(n, m, batch, weighted):
+    """The quotient's keys by tiles of 2,048 arcs: whole and partial tiles, runs
+    that cross them (node 0's is longer than a tile), and batches refined
+    where their runs lie against batches with an arc set of their own."""
+    rng = np.random.default_rng(m)
+    hub = m // 2 if m > 2048 else 40
+    src = np.concatenate([np.zeros(hub, np.int64), rng.integers(0, n, m - hub)])
+    dst = rng.integers(0, n // 4, m)
+    wt = rng.integers(1, 4, m).astype(np.uint64) if weighted else None
+    off, idx, wt = G.csr_from_arcs(n, src, dst, wt)
+    b = max(batch, hub + 1)
+    ex = oracle.refine_edge_batches(off, idx, wt, batch=b)
+    for persistent in (True, False):
+        with R.Context(0, persistent=persistent) as ctx:
+            r, info = ctx.refine_edge_batches(off, idx, wt, edge_batch_size=b)
+        assert (r.done, r.blocks, info["iterations"]) == (ex.done, ex.blocks, ex.iterations)
+        assert np.array_equal(r.labels, ex.labels)
