@@ -195,12 +195,12 @@ extern "C" rbsc_status rbsc_graph_batch_refine(rbsc_ctx* ctx, rbsc_graph* g, con
     k_batch_blocks<<<grid_of(G), 256, 0, s>>>(G, hoff, blocks);
     BK(cudaGetLastError());
     BK(cudaEventRecord(e1, s));
-    if (out->local) BK(cudaMemcpyAsync(out->local, local, 4 * (size_t)n, cudaMemcpyDeviceToHost, s));
+    if (out->local) BKS(copy_out(ctx, out->local, local, 4 * (size_t)n, s));
     if (out->blocks) BK(cudaMemcpyAsync(out->blocks, blocks, 4 * (size_t)G, cudaMemcpyDeviceToHost, s));
     if (out->fingerprint) BK(cudaMemcpyAsync(out->fingerprint, fp, 8 * (size_t)G, cudaMemcpyDeviceToHost, s));
     if (out->hist_offsets) BK(cudaMemcpyAsync(out->hist_offsets, hoff, 8 * ((size_t)G + 1), cudaMemcpyDeviceToHost, s));
-    if (out->hist_colors) BK(cudaMemcpyAsync(out->hist_colors, ecolor, 4 * (size_t)H, cudaMemcpyDeviceToHost, s));
-    if (out->hist_counts) BK(cudaMemcpyAsync(out->hist_counts, ecount, 4 * (size_t)H, cudaMemcpyDeviceToHost, s));
+    if (out->hist_colors) BKS(copy_out(ctx, out->hist_colors, ecolor, 4 * (size_t)H, s));
+    if (out->hist_counts) BKS(copy_out(ctx, out->hist_counts, ecount, 4 * (size_t)H, s));
     BK(cudaStreamSynchronize(s));
     cudaEventElapsedTime(&batch_ms, e0, e1);
     if (stats) {

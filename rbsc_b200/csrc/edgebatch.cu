@@ -552,7 +552,7 @@ extern "C" rbsc_status rbsc_refine_edge_batches(rbsc_ctx* ctx, const rbsc_csr* h
         ++rbsc::launch_counter();
         k_eb_labels<<<grid_of(N), 256, 0, s>>>(N, cls, firstn, lab);
         EK(cudaGetLastError());
-        EK(cudaMemcpyAsync(out_labels, lab, 4 * (size_t)N, cudaMemcpyDeviceToHost, s));
+        EKS(copy_out(ctx, out_labels, lab, 4 * (size_t)N, s));
     }
     EK(cudaStreamSynchronize(s));
     if (stats) {

@@ -26,6 +26,8 @@ struct MemPool {
     size_t cap = (size_t)48 << 30;             // most bytes of unused blocks kept
 };
 
+struct HostCopier;
+
 struct rbsc_ctx {
     int device = 0;
     MemPool dpool;
@@ -48,6 +50,7 @@ struct rbsc_ctx {
     // staging buffer of small one-shot calls
     void* h_fused = nullptr;
     void* h_stage = nullptr;
+    HostCopier* copier = nullptr;  // pinned slots of large pageable copies (hostcopy.cu)
     std::string err;
 };
 
@@ -198,6 +201,12 @@ rbsc_status graph_upload_unprepared(rbsc_ctx* ctx, const rbsc_csr* host_graph, r
 rbsc_status graph_alloc_csr(rbsc_ctx* ctx, rbsc_graph* g, bool weighted);
 rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats,
                             rbsc_kernel_times* kt);
+
+// Copies between the device and host memory, queued on s like
+// cudaMemcpyAsync; large pageable ones by several threads (hostcopy.cu).
+rbsc_status copy_in(rbsc_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s);
+rbsc_status copy_out(rbsc_ctx* ctx, void* dst, const void* src, size_t bytes, cudaStream_t s);
+void copier_release(rbsc_ctx* ctx);
 
 // Device scratch of one call: every block is released when it goes out of
 // scope (the modules that build their own working set per call).

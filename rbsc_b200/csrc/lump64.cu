@@ -373,7 +373,7 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
     uint32_t* d_init = nullptr;
     if (init_colors) {
         EKS(sc.get(&d_init, N));
-        EK(cudaMemcpyAsync(d_init, init_colors, 4ull * N, cudaMemcpyHostToDevice, s));
+        EKS(copy_in(ctx, d_init, init_colors, 4ull * N, s));
     }
     uint32_t stamp = 1;
     L64Counters hc{};
@@ -500,7 +500,7 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
         if (rounds >= max_rounds) return rbsc_fail(ctx, RBSC_ERR_NOT_CONVERGED, "no fixpoint after %u passes", rounds);
     }
     EK(cudaEventRecord(e1, s));
-    EK(cudaMemcpyAsync(out_labels, col, 4ull * N, cudaMemcpyDeviceToHost, s));
+    EKS(copy_out(ctx, out_labels, col, 4ull * N, s));
     EK(cudaStreamSynchronize(s));
     float dev_ms = 0.f;
     cudaEventElapsedTime(&dev_ms, e0, e1);

@@ -241,6 +241,7 @@ extern "C" void rbsc_ctx_destroy(rbsc_ctx* ctx)
         cudaStreamDestroy(ctx->side);
     }
     cudaStreamDestroy(ctx->stream);
+    copier_release(ctx);
     host_free(ctx, ctx->h_fused);
     host_free(ctx, ctx->h_stage);
     pool_release(ctx->dpool);
@@ -547,13 +548,17 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
         return st;
     }
     cudaStream_t s = ctx->stream;
-    const cudaMemcpyKind kind = from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+    // a copy of an input array; the first failure ends the load below
+    auto bring = [&](void* dst, const void* src, size_t b) -> cudaError_t {
+        if (from_device) return cudaMemcpyAsync(dst, src, b, cudaMemcpyDeviceToDevice, s);
+        return copy_in(ctx, dst, src, b, s) == RBSC_OK ? cudaSuccess : cudaErrorUnknown;
+    };
     auto t0 = std::chrono::steady_clock::now();
     cudaError_t e = unprepared ? cudaEventRecord(ctx->ev[2], s) : cudaSuccess;
     const size_t offb = (size_t)c->offset_bytes * ((size_t)c->n + 1);
     uint64_t bytes = offb + sizeof(uint32_t) * c->m + (c->weights ? sizeof(uint64_t) * c->m : 0);
     if (c->offset_bytes == 8) {
-        if (e == cudaSuccess) e = cudaMemcpyAsync(g->d_off, c->offsets, offb, kind, s);
+        if (e == cudaSuccess) e = bring(g->d_off, c->offsets, offb);
     } else {
         // stage the 32-bit offsets in the (not yet used) index buffer tail? use a scratch buffer
         void* tmp = nullptr;
@@ -562,7 +567,7 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
             rbsc_graph_free(g);
             return st;
         }
-        e = cudaMemcpyAsync(tmp, c->offsets, offb, kind, s);
+        e = bring(tmp, c->offsets, offb);
         if (e == cudaSuccess) {
             ++rbsc::launch_counter();
             k_widen_offsets<uint32_t><<<grid_for((uint64_t)c->n + 1, 256), 256, 0, s>>>((uint64_t)c->n + 1, (const uint32_t*)tmp, g->d_off);
@@ -581,7 +586,7 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
             rbsc_graph_free(g);
             return st;
         }
-        e = cudaMemcpyAsync(g->d_init, h_init, 4 * (size_t)c->n, cudaMemcpyHostToDevice, s);
+        e = bring(g->d_init, h_init, 4 * (size_t)c->n);
         if (e == cudaSuccess) g->h_init_loaded = h_init;
     }
     if (defer_heads) {
@@ -610,9 +615,9 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
             g->upload_issued = e == cudaSuccess;
         }
     } else if (e == cudaSuccess && c->m) {
-        e = cudaMemcpyAsync(g->d_idx, c->indices, sizeof(uint32_t) * c->m, kind, s);
+        e = bring(g->d_idx, c->indices, sizeof(uint32_t) * c->m);
     }
-    if (e == cudaSuccess && c->weights && c->m) e = cudaMemcpyAsync(g->d_wt, c->weights, sizeof(uint64_t) * c->m, kind, s);
+    if (e == cudaSuccess && c->weights && c->m) e = bring(g->d_wt, c->weights, sizeof(uint64_t) * c->m);
     if (e == cudaSuccess && !unprepared) e = cudaStreamSynchronize(s);
     auto t1 = std::chrono::steady_clock::now();
     if (h2d_ms) *h2d_ms = unprepared ? 0.0 : std::chrono::duration<double, std::milli>(t1 - t0).count();
@@ -1042,7 +1047,7 @@ static rbsc_status stream_signature(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s
             CK(cudaStreamWaitEvent(s, g->ev_chunk[c], 0));
         } else {
             if (upload) {
-                CK(cudaMemcpyAsync(g->d_idx + a0, g->h_upload + a0, 4 * (a1 - a0), cudaMemcpyHostToDevice, g->copy_stream));
+                CKS(copy_in(ctx, g->d_idx + a0, g->h_upload + a0, 4 * (a1 - a0), g->copy_stream));
             } else {
                 CK(cudaStreamWaitEvent(g->copy_stream, g->ev_used[slot], 0));
                 CK(cudaMemcpyAsync(g->d_chunk[slot], g->d_idx + a0, 4 * (a1 - a0), cudaMemcpyHostToDevice, g->copy_stream));
@@ -1091,7 +1096,7 @@ static rbsc_status finish_upload(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s)
             while (last > 0 && !g->ev_chunk[last]) --last;
             CK(cudaStreamWaitEvent(s, g->ev_chunk[last], 0));
         } else {
-            CK(cudaMemcpyAsync(g->d_idx, g->h_upload, 4 * g->m, cudaMemcpyHostToDevice, s));
+            CKS(copy_in(ctx, g->d_idx, g->h_upload, 4 * g->m, s));
         }
         ++rbsc::launch_counter();
         k_validate_heads<<<persistent_grid(ctx, ceil_div<uint64_t>(g->m, 256), 1), 256, 0, s>>>(0, g->m, g->n, g->d_idx, g->d_st);
@@ -1913,7 +1918,7 @@ extern "C" rbsc_status rbsc_graph_refine(rbsc_ctx* ctx, rbsc_graph* g, const uin
     } else if (init_colors && g->n) {
         if (!g->d_init) CKS(dev_alloc(ctx, (void**)&g->d_init, 4 * (size_t)g->n));
         auto a = std::chrono::steady_clock::now();
-        CK(cudaMemcpyAsync(g->d_init, init_colors, 4 * (size_t)g->n, cudaMemcpyHostToDevice, ctx->stream));
+        CKS(copy_in(ctx, g->d_init, init_colors, 4 * (size_t)g->n, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         h2d = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - a).count();
         d_init = g->d_init;
@@ -1921,7 +1926,7 @@ extern "C" rbsc_status rbsc_graph_refine(rbsc_ctx* ctx, rbsc_graph* g, const uin
     CKS(refine_resident(ctx, g, d_init, nullptr, stats, nullptr));
     if (out_labels && g->n) {
         auto a = std::chrono::steady_clock::now();
-        CK(cudaMemcpyAsync(out_labels, g->d_out, 4 * (size_t)g->n, cudaMemcpyDeviceToHost, ctx->stream));
+        CKS(copy_out(ctx, out_labels, g->d_out, 4 * (size_t)g->n, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
         d2h = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - a).count();
     }
