@@ -30,6 +30,9 @@
 //      stamped 16-byte relabel table of the integer path, new label = smallest
 //      member;
 //   6. the host reads the class count: unchanged = fixpoint.
+// Nodes alone in their class take no further part as rows (their blocks still
+// do as successors): their arcs are dropped before the next pass's sort
+// (R-MAT-20, 16 M arcs, five passes: 8.4 -> 3.5 ms of device time).
 // Exact check at the fixpoint (the groups of the last pass are those of the
 // final partition, whose canonical labels the pass left unchanged): the
 // nonzero groups are compacted and re-sorted by row (stable, row bits only),
@@ -176,40 +179,61 @@ __global__ void k_l64_sums(L64Counters* __restrict__ c, uint64_t m, uint32_t lb,
     }
 }
 
-// One warp per long group: the lanes load 32 keys and weights at a time (the
-// next 32 while lane 0 adds the current ones, handed over by shuffles in lane
-// order), so the sum is the same arc-order double sum as k_l64_sums', at the
-// pace of the dependent adds rather than of one load per weight.
+// One warp per long group: the lanes bring the next 128 weights to shared
+// memory while lane 0 adds the current ones, so the arc-order sum runs at the
+// pace of its dependent adds alone (the loads from shared memory do not depend
+// on them).  R-MAT-20's first pass, whose longest row has 40,000 arcs, with the
+// weights handed over by shuffles: 1.3 ms; here 0.9.
+constexpr uint32_t kLongStep = 128;
+
 __global__ void __launch_bounds__(kT) k_l64_long_sums(const L64Counters* __restrict__ c, uint64_t m, uint32_t lb,
                                                       const unsigned long long* __restrict__ keys,
                                                       const unsigned long long* __restrict__ vals, uint64_t salt1,
                                                       uint32_t salt2, int hash_bits, Sig* __restrict__ sig,
                                                       uint32_t* __restrict__ bits, const uint32_t* __restrict__ long_list)
 {
+    constexpr int P = kLongStep / 32;
+    __shared__ double s_w[kT / 32][kLongStep];
     const uint32_t L = c->long_groups;
     const uint32_t lane = threadIdx.x & 31;
+    double* sw = s_w[threadIdx.x >> 5];
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     for (uint64_t t = blockIdx.x * (uint64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); t < L; t += warps) {
         const uint64_t b = long_list[t];
         const unsigned long long k = keys[b];
         double s = 0.0;
-        bool in = b + lane < m && keys[b + lane] == k;
-        double x = in ? __longlong_as_double((long long)vals[b + lane]) : 0.0;
-        for (uint64_t a0 = b;; a0 += 32) {
-            // the group is contiguous: its lanes of this chunk are a prefix
-            const uint32_t cnt = (uint32_t)__popc(__ballot_sync(0xffffffffu, in));
-            const uint64_t a1 = a0 + 32;
-            const bool nin = cnt == 32u && a1 + lane < m && keys[a1 + lane] == k;
-            const double nx = nin ? __longlong_as_double((long long)vals[a1 + lane]) : 0.0;
-            for (uint32_t j = 0; j < cnt; ++j) {
-                const double v = __shfl_sync(0xffffffffu, x, j);
-                if (lane == 0) s += v;
+        double x[P];
+        uint32_t cnt = 0;  // of the step in x: the group is contiguous, so its positions are a prefix
+        auto fetch = [&](uint64_t a) {
+            cnt = 0;
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                const uint64_t i = a + 32u * q + lane;
+                const bool in = i < m && keys[i] == k;
+                x[q] = in ? __longlong_as_double((long long)vals[i]) : 0.0;
+                cnt += (uint32_t)__popc(__ballot_sync(0xffffffffu, in));
             }
-            if (cnt < 32u) break;
-            in = nin;
-            x = nx;
+        };
+        fetch(b);
+        for (uint64_t a = b;; a += kLongStep) {
+            const uint32_t now = cnt;
+            __syncwarp();
+#pragma unroll
+            for (int q = 0; q < P; ++q) sw[32 * q + lane] = x[q];
+            __syncwarp();
+            if (now == kLongStep) fetch(a + kLongStep);
+            if (lane == 0) {
+                uint32_t i = 0;
+                for (; i + 8 <= now; i += 8) {
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) s += sw[i + q];
+                }
+                for (; i < now; ++i) s += sw[i];
+            }
+            if (now < kLongStep) break;
         }
         if (lane == 0) group_done(b, s, k, lb, salt1, salt2, hash_bits, sig, bits);
+        __syncwarp();
     }
 }
 
@@ -218,11 +242,13 @@ __global__ void __launch_bounds__(kT) k_l64_long_sums(const L64Counters* __restr
 template <int MODE>
 __global__ void k_l64_insert(uint32_t n, const uint32_t* __restrict__ col, const Sig* __restrict__ sig,
                              const uint32_t* __restrict__ aux, uint64_t seed, uint32_t stamp, Entry* __restrict__ tab,
-                             uint32_t log2size, uint32_t* __restrict__ slot, L64Counters* __restrict__ c)
+                             uint32_t log2size, uint32_t* __restrict__ slot, const uint8_t* __restrict__ alone,
+                             L64Counters* __restrict__ c)
 {
     for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); base < n; base += (uint64_t)gridDim.x * blockDim.x) {
-        const bool need = base + (threadIdx.x & 31) < n;
         const uint32_t u = (uint32_t)(base + (threadIdx.x & 31));
+        const bool in = base + (threadIdx.x & 31) < n;
+        const bool need = in && !alone[u];
         uint64_t k1 = 0;
         uint32_t k2 = stamp;
         if (need) {
@@ -236,19 +262,55 @@ __global__ void k_l64_insert(uint32_t n, const uint32_t* __restrict__ col, const
                 k1 = (uint64_t)col[u] | ((uint64_t)(aux[u] != 0u) << 32);
             }
         }
-        bool nb = false;
+        bool nb = in && !need;  // alone: a block of its own
         insert_warp(need, u, u, false, k1, k2, stamp, tab, log2size, slot, &c->error, nb);
         count_blocks(nb, &c->classes);
     }
 }
 
+// New labels; alone[u] = 1 when nobody else is in u's class.  A class of one
+// never splits again: its node leaves the inserts, its row the sorts.
 __global__ void k_l64_relabel(uint32_t n, const Entry* __restrict__ tab, const uint32_t* __restrict__ slot,
-                              uint32_t* __restrict__ col)
+                              uint32_t* __restrict__ col, uint8_t* __restrict__ alone)
 {
     for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t* v = reinterpret_cast<const uint32_t*>(tab + slot[u]) + 3;
-        col[u] = __ldg(v) & kLabelMask;
+        if (alone[u]) continue;
+        const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(tab + slot[u]) + 3);
+        col[u] = v & kLabelMask;
+        if (!(v & kJoined)) alone[u] = 1;
     }
+}
+
+// The arcs of the rows still in play: row lengths (0 for a node that is alone;
+// every node's row of the current set: [start[u], start[u + 1])), then, after
+// a scan, the arcs moved to their new places, in order.
+__global__ void k_l64_live_lengths(uint32_t n, const uint32_t* __restrict__ start, const uint8_t* __restrict__ alone,
+                                   uint32_t* __restrict__ len)
+{
+    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u < n; u += (uint64_t)gridDim.x * blockDim.x)
+        len[u] = alone[u] ? 0u : start[u + 1] - start[u];
+}
+
+__global__ void k_l64_live_arcs(uint64_t m, const uint32_t* __restrict__ src, const uint32_t* __restrict__ idx,
+                                const unsigned long long* __restrict__ w, const uint32_t* __restrict__ start,
+                                const uint32_t* __restrict__ nstart, const uint8_t* __restrict__ alone, uint32_t* __restrict__ nsrc,
+                                uint32_t* __restrict__ nidx, unsigned long long* __restrict__ nw)
+{
+    for (uint64_t a = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; a < m; a += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t u = src[a];
+        if (alone[u]) continue;
+        const uint32_t p = nstart[u] + ((uint32_t)a - start[u]);
+        nsrc[p] = u;
+        nidx[p] = idx[a];
+        nw[p] = w[a];
+    }
+}
+
+// 32-bit row starts (fewer than 2^32 arcs)
+__global__ void k_l64_starts(uint32_t n, const uint64_t* __restrict__ off, uint32_t* __restrict__ start)
+{
+    for (uint64_t u = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; u <= n; u += (uint64_t)gridDim.x * blockDim.x)
+        start[u] = (uint32_t)off[u];
 }
 
 // nzflag[i] = position i starts a group with a nonzero rounded sum
@@ -340,6 +402,9 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
     unsigned long long *keys = nullptr, *keys_alt = nullptr, *vals = nullptr, *vals_alt = nullptr;
     Sig* sig = nullptr;
     Entry* tab = nullptr;
+    uint8_t* alone = nullptr;
+    uint32_t *start[2] = {nullptr, nullptr}, *lsrc[2] = {nullptr, nullptr}, *lidx[2] = {nullptr, nullptr};
+    unsigned long long* lw[2] = {nullptr, nullptr};
     L64Counters* dc = nullptr;
     void* tmp = nullptr;
     EKS(sc.get(&col, N));
@@ -350,6 +415,9 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
     EKS(sc.get(&sig, N));
     EKS(sc.get(&tab, (size_t)1 << log2tab));
     EKS(sc.get(&dc, 1));
+    EKS(sc.get(&alone, N));
+    EKS(sc.get(&start[0], (size_t)N + 1));
+    EKS(sc.get(&start[1], (size_t)N + 1));
     EKS(sc.get(&src, M));
     EKS(sc.get(&keys, M));
     EKS(sc.get(&keys_alt, M));
@@ -363,10 +431,13 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
     EKS(sc.get((char**)&tmp, std::max(radix_temp_bytes(M), scan_temp_bytes<uint32_t>(big)) + 1024));
     EK(cudaMemsetAsync(dc, 0, sizeof(L64Counters), s));
     EK(cudaMemsetAsync(tab, 0, sizeof(Entry) << log2tab, s));
+    EK(cudaMemsetAsync(alone, 0, N, s));
     ++rbsc::launch_counter();
     k_l64_check_weights<<<grid_of(M), kT, 0, s>>>(M, w, dc);
     ++rbsc::launch_counter();
     k_l64_rows<<<grid_of(32ull * N), kT, 0, s>>>(N, g->d_off, src);
+    ++rbsc::launch_counter();
+    k_l64_starts<<<grid_of((uint64_t)N + 1), kT, 0, s>>>(N, g->d_off, start[0]);
     EK(cudaGetLastError());
 
     // the initial colours' classes in the table (stamp 1), canonical labels
@@ -390,13 +461,13 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
         EK(cudaMemsetAsync(&dc->classes, 0, 4, s));
         ++rbsc::launch_counter();
         if (mode == 0)
-            k_l64_insert<0><<<grid_of(N), kT, 0, s>>>(N, col, sig, aux, ctx->opts.seed, stamp, tab, log2tab, slot, dc);
+            k_l64_insert<0><<<grid_of(N), kT, 0, s>>>(N, col, sig, aux, ctx->opts.seed, stamp, tab, log2tab, slot, alone, dc);
         else if (mode == 1)
-            k_l64_insert<1><<<grid_of(N), kT, 0, s>>>(N, col, sig, aux, ctx->opts.seed, stamp, tab, log2tab, slot, dc);
+            k_l64_insert<1><<<grid_of(N), kT, 0, s>>>(N, col, sig, aux, ctx->opts.seed, stamp, tab, log2tab, slot, alone, dc);
         else
-            k_l64_insert<2><<<grid_of(N), kT, 0, s>>>(N, col, sig, aux, ctx->opts.seed, stamp, tab, log2tab, slot, dc);
+            k_l64_insert<2><<<grid_of(N), kT, 0, s>>>(N, col, sig, aux, ctx->opts.seed, stamp, tab, log2tab, slot, alone, dc);
         ++rbsc::launch_counter();
-        k_l64_relabel<<<grid_of(N), kT, 0, s>>>(N, tab, slot, col);
+        k_l64_relabel<<<grid_of(N), kT, 0, s>>>(N, tab, slot, col, alone);
         EK(cudaGetLastError());
         // next stamp; the table is cleared when it wraps
         stamp = stamp % 255u + 1u;
@@ -416,7 +487,41 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
     const int hash_bits = ctx->opts.test_hash_bits;
     const unsigned long long* w64 = reinterpret_cast<const unsigned long long*>(g->d_wt);
     const unsigned long_grid = (unsigned)ctx->sm_count * 8;
+    // the arcs in play: all of them at first; once a pass leaves less than 3/4
+    // of them, the others are dropped (a copy in order, two buffers in turn)
+    uint64_t live = M;
+    const uint32_t *asrc = src, *aidx = g->d_idx;
+    const unsigned long long* aw = w64;
+    int sb = 0, ab = 0;  // start[sb]: the row starts of the arcs in play; l*[ab]: where the next copy goes
+    const uint64_t M0 = M;
     for (;;) {
+        if (rounds > 0 && M0) {
+            ++rbsc::launch_counter();
+            k_l64_live_lengths<<<grid_of(N), kT, 0, s>>>(N, start[sb], alone, start[sb ^ 1]);
+            EK((exclusive_scan<uint32_t, uint32_t>(start[sb ^ 1], start[sb ^ 1], N, start[sb ^ 1] + N, tmp, s)));
+            uint32_t left = 0;
+            EK(cudaMemcpyAsync(&left, start[sb ^ 1] + N, 4, cudaMemcpyDeviceToHost, s));
+            EK(cudaStreamSynchronize(s));
+            if ((uint64_t)left * 4 <= live * 3) {
+                // (the first copy of each buffer is the largest it will hold)
+                if (!lsrc[ab]) {
+                    EKS(sc.get(&lsrc[ab], left));
+                    EKS(sc.get(&lidx[ab], left));
+                    EKS(sc.get(&lw[ab], left));
+                }
+                ++rbsc::launch_counter();
+                k_l64_live_arcs<<<grid_of(live), kT, 0, s>>>(live, asrc, aidx, aw, start[sb], start[sb ^ 1], alone, lsrc[ab], lidx[ab],
+                                                            lw[ab]);
+                EK(cudaGetLastError());
+                asrc = lsrc[ab];
+                aidx = lidx[ab];
+                aw = lw[ab];
+                ab ^= 1;
+                sb ^= 1;
+                live = left;
+            }
+        }
+        const uint64_t M = live;
         // one signature pass; prev = the current number of blocks
         const uint32_t cb = bits_of(prev - 1u);  // block-id bits of a key
         bool in_alt = false;
@@ -427,7 +532,7 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
             ++rbsc::launch_counter();
             k_l64_block_ids<<<grid_of(N), kT, 0, s>>>(N, col, first, bid);
             ++rbsc::launch_counter();
-            k_l64_keys<<<grid_of(M), kT, 0, s>>>(M, lb, src, g->d_idx, bid, w64, keys, vals);
+            k_l64_keys<<<grid_of(M), kT, 0, s>>>(M, lb, asrc, aidx, bid, aw, keys, vals);
             EK(cudaGetLastError());
             EK(radix_sort<unsigned long long>(keys, keys_alt, vals, vals_alt, M, (int)lb, (int)(lb + cb), tmp, s, &in_alt));
         }

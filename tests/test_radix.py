@@ -55,3 +55,23 @@ def test_long_rows_of_the_check():
         with R.Context(0, persistent=False) as ctx:
             r = ctx.refine(off, idx, wt)
         assert r.blocks == ex.blocks and np.array_equal(r.labels, ex.labels) and r.verified == 1
+
+
+@pytest.mark.parametrize("n_rows", [1, 3])
+@pytest.mark.parametrize("d", [32, 33, 127, 128, 129, 256, 257, 5000])
+def test_long_groups_of_double_weights(d, n_rows):
+    """Rows of d arcs into one block, summed in arc order (the float of the sum
+    depends on it); rows that end up alone leave the later passes."""
+    rng = np.random.default_rng(d)
+    n = 600
+    src = np.concatenate([np.repeat(np.arange(2 * n_rows), d), np.arange(50, n - 1)])
+    dst = np.concatenate([rng.integers(300, n, 2 * n_rows * d), np.arange(51, n)])
+    w = rng.choice([0.1, 1e8, -1e8, 3e-5, 0.7], size=n_rows * d)
+    wt = np.concatenate([w, w, np.full(n - 51, 0.3)])  # the second half repeats the first: equal rows
+    dst[n_rows * d: 2 * n_rows * d] = dst[: n_rows * d]
+    off, idx, order = G.csr_from_arcs(n, src, dst, np.arange(len(src)), sort=False)
+    wt = wt[order.astype(np.int64)]
+    ex = oracle.refine_f64(off, idx, wt)
+    with R.Context(0) as ctx:
+        r = ctx.refine_f64(off, idx, wt)
+    assert r.blocks == ex.blocks and np.array_equal(r.labels, ex.labels) and r.rounds == ex.rounds
