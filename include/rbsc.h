@@ -466,8 +466,8 @@ typedef struct {
     uint32_t queue_cap;       /* jobs waiting to start, 0 = 65536; submit beyond
                                  returns RBSC_ERR_BUSY                                */
     rbsc_opts opts;           /* refinement options of every job (no_persist is forced
-                                 on: a cooperative grid must not share the GPU with
-                                 the other slots' kernels)                            */
+                                 on; the cooperative launches of jobs below 2^22 arcs
+                                 wait for one another)                                */
     int32_t dry_run;          /* TEST HOOK: 1 = no GPU work at all; each job "runs" for
                                  dry_run_ns_per_arc * arcs + 20 us of host sleep and
                                  writes no labels (exercises admission and packing)   */

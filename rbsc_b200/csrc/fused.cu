@@ -23,11 +23,6 @@ namespace {
 // 70 / 71, 8,000 and 32,000 76-97 / 72-84, 16,000 and 64,000 115-135 / 80-87).
 constexpr uint32_t kClusterNodes = 8192;
 constexpr uint64_t kClusterArcs = 1u << 15;
-// Beside other contexts' work (a server's executors) only a cluster is safe to
-// launch, and it still beats the launch-per-phase path up to these sizes
-// (16,000 nodes and 128,000 arcs: 92-149 us against 325).
-constexpr uint32_t kSharedNodes = 16384;
-constexpr uint64_t kSharedArcs = 1u << 17;
 constexpr unsigned kClusterBlocks = 8;
 // A host graph of at most this many bytes goes through one pinned staging
 // buffer and one copy.
@@ -40,14 +35,11 @@ bool default_knobs(const rbsc_opts& o)
            o.persist_bps == 0 && o.persist_sig == 0;
 }
 
-bool one_cluster(const rbsc_ctx* ctx, uint32_t n, uint64_t m)
-{
-    return ctx->shared_gpu || (n <= kClusterNodes && m <= kClusterArcs);
-}
+bool one_cluster(uint32_t n, uint64_t m) { return n <= kClusterNodes && m <= kClusterArcs; }
 
 rbsc_status launch(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
 {
-    const bool cluster = one_cluster(ctx, a.n, a.m);
+    const bool cluster = one_cluster(a.n, a.m);
     cudaLaunchConfig_t cfg{};
     cfg.blockDim = kFuThreads;
     cfg.stream = s;
@@ -174,6 +166,17 @@ rbsc_status deep_tail(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
     return RBSC_OK;
 }
 
+// One launch, waited for.
+rbsc_status launch_and_wait(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
+{
+    std::unique_lock<std::mutex> lock;
+    if (!one_cluster(a.n, a.m)) lock = coop_lock(ctx->device);
+    EKS(launch(ctx, a, s));
+    EK(cudaEventRecord(ctx->ev[1], s));
+    EK(cudaStreamSynchronize(s));
+    return RBSC_OK;
+}
+
 // The launch, and where it stops early the work-list passes and a launch that
 // confirms them; waits for the stream.  ev[0] and ev[1] enclose it.
 rbsc_status run(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
@@ -181,16 +184,12 @@ rbsc_status run(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
     FusedResult& r = *static_cast<FusedResult*>(ctx->h_fused);
     a.deep_round = deep_round(a.m);
     EK(cudaEventRecord(ctx->ev[0], s));
-    EKS(launch(ctx, a, s));
-    EK(cudaEventRecord(ctx->ev[1], s));
-    EK(cudaStreamSynchronize(s));
+    EKS(launch_and_wait(ctx, a, s));
     const uint32_t initial = r.initial_blocks;
     const uint64_t t0 = r.t[0], t1 = r.t[1];
     while (r.status == kFuDeep) {
         EKS(deep_tail(ctx, a, s));
-        EKS(launch(ctx, a, s));
-        EK(cudaEventRecord(ctx->ev[1], s));
-        EK(cudaStreamSynchronize(s));
+        EKS(launch_and_wait(ctx, a, s));
         r.initial_blocks = initial;
         r.t[0] = t0;
         r.t[1] = t1;
@@ -240,13 +239,19 @@ rbsc_status outcome(rbsc_ctx* ctx, rbsc_stats* stats, float ms, bool* handled)
 // R-MAT-22 with 65 M 1933 / 1852.
 constexpr uint64_t kSmallArcs = 1ull << 22, kLargeArcs = 3ull << 23, kLargeWeighted = 1ull << 25;
 
+std::unique_lock<std::mutex> coop_lock(int device)
+{
+    static std::mutex mu[64];
+    return std::unique_lock<std::mutex>(mu[(unsigned)device % 64u]);
+}
+
 bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m, bool weighted, bool rival)
 {
     if (!default_knobs(ctx->opts) || n == 0 || n > kIncMaxNodes) return false;
     if (m >= kSmallArcs && (rival || m >= (weighted ? kLargeWeighted : kLargeArcs))) return false;
-    // a cooperative grid needs the chip to itself; a cluster does not
-    if (ctx->shared_gpu) return n <= kSharedNodes && m <= kSharedArcs;
-    return !ctx->opts.no_persist;
+    // a server's contexts (whose no_persist keeps k_refine_persistent out) take
+    // it too: cooperative launches wait for one another (coop_lock)
+    return ctx->shared_gpu || !ctx->opts.no_persist;
 }
 
 rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled)

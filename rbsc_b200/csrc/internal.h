@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 #include <map>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -43,8 +44,7 @@ struct rbsc_ctx {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     int sm_count = 148;
-    // other contexts' work runs beside this one's (a server's executors): no
-    // cooperative launches
+    // other contexts' work runs beside this one's (a server's executors)
     bool shared_gpu = false;
     // the one-launch refinement (fused.cu): its page-locked result and the
     // staging buffer of small one-shot calls
@@ -195,9 +195,11 @@ rbsc_status host_alloc(rbsc_ctx* ctx, void** p, size_t bytes);
 void host_free(rbsc_ctx* ctx, void*& p);
 rbsc_status ensure_temp(rbsc_ctx* ctx, rbsc_graph* g, size_t bytes);
 rbsc_status graph_prepare(rbsc_ctx* ctx, rbsc_graph* g);
-// Copies a host CSR to the device without checking or tiling it, for a graph
-// that fused_wanted takes (refine_resident prepares it if it has to).
-rbsc_status graph_upload_unprepared(rbsc_ctx* ctx, const rbsc_csr* host_graph, rbsc_graph** out, double* h2d_ms, uint64_t* h2d_bytes);
+// The graph of a one-shot call: not checked or tiled where fused_wanted takes
+// it (refine_resident prepares it if it has to); a large unweighted one's heads
+// arrive during the first pass.
+rbsc_status graph_upload_oneshot(rbsc_ctx* ctx, const rbsc_csr* host_graph, const uint32_t* init_colors, rbsc_graph** out, double* h2d_ms,
+                                 uint64_t* h2d_bytes);
 rbsc_status graph_alloc_csr(rbsc_ctx* ctx, rbsc_graph* g, bool weighted);
 rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats,
                             rbsc_kernel_times* kt);
@@ -247,6 +249,12 @@ struct Scratch {
         rbsc_status s_ = (call);       \
         if (s_ != RBSC_OK) return s_;  \
     } while (0)
+
+// Held from a cooperative launch until its stream is done: the blocks of such a
+// grid wait for one another, so two grids of different contexts, each partly
+// on the chip, would wait for good (their waits are bounded, and end in an
+// error).  Any other kernel ends by itself and makes room.
+std::unique_lock<std::mutex> coop_lock(int device);
 
 // The one-launch refinement (fused.cu).  fused_wanted: the context's options
 // and the sizes allow it; rival: a large graph would get hot heads or an

@@ -641,9 +641,15 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
     return RBSC_OK;
 }
 
-rbsc_status graph_upload_unprepared(rbsc_ctx* ctx, const rbsc_csr* host_graph, rbsc_graph** out, double* h2d_ms, uint64_t* h2d_bytes)
+rbsc_status graph_upload_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init_colors, rbsc_graph** out, double* h2d_ms,
+                                 uint64_t* h2d_bytes)
 {
-    return graph_load(ctx, host_graph, false, out, h2d_ms, h2d_bytes, false, nullptr, true);
+    CKS(check_csr_args(ctx, c));
+    // large unweighted graphs: the heads' copy overlaps the refinement
+    const bool defer = !c->weights && c->m >= (1ull << 22);
+    CKS(graph_load(ctx, c, false, out, h2d_ms, h2d_bytes, defer, init_colors, fused_wanted(ctx, c->n, c->m, c->weights != nullptr, defer)));
+    (*out)->oneshot = true;
+    return RBSC_OK;
 }
 
 extern "C" rbsc_status rbsc_graph_upload(rbsc_ctx* ctx, const rbsc_csr* host_graph, rbsc_graph** out)
@@ -1400,6 +1406,7 @@ static rbsc_status run_persistent(rbsc_ctx* ctx, rbsc_graph* g, rbsc_kernel_time
     void* args[] = {&a};
     const uint32_t r0 = g->h_st->round;
     if (kt) CK(cudaEventRecord(ctx->ev[2], s));
+    const std::unique_lock<std::mutex> lock = coop_lock(ctx->device);
     ++rbsc::launch_counter();
     CK(cudaLaunchCooperativeKernel(kern, dim3(grid), dim3(kNodeThreads), args, 0, s));
     if (kt) CK(cudaEventRecord(ctx->ev[3], s));
@@ -1952,11 +1959,7 @@ extern "C" rbsc_status rbsc_refine(rbsc_ctx* ctx, const rbsc_csr* host_graph, co
     bool handled = false;
     CKS(fused_oneshot(ctx, host_graph, init_colors, out_labels, stats, &handled));
     if (handled) return RBSC_OK;
-    // large unweighted graphs: the heads' copy overlaps the refinement
-    const bool defer = !host_graph->weights && host_graph->m >= (1ull << 22);
-    CKS(graph_load(ctx, host_graph, false, &g, &up_ms, &up_bytes, defer, init_colors,
-                   fused_wanted(ctx, host_graph->n, host_graph->m, host_graph->weights != nullptr, defer)));
-    g->oneshot = true;
+    CKS(graph_upload_oneshot(ctx, host_graph, init_colors, &g, &up_ms, &up_bytes));
     rbsc_status st = rbsc_graph_refine(ctx, g, init_colors, out_labels, stats);
     up_ms += g->up_ms;
     rbsc_graph_free(g);

@@ -156,3 +156,32 @@ def test_batch_rejects_bad_graph_nodes():
         bad[3] = bad[2]
         with pytest.raises(R.RbscError):
             ctx.batch_refine(off, idx, bad, lab)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [[1], [2, 1, 3], [31, 32, 33, 64], [255, 256, 257, 511, 513, 5], [2047, 2048, 1, 700],
+                                   [2049, 3, 40]], ids=lambda s: "-".join(map(str, s)))
+@pytest.mark.parametrize("labels", [1, 5])
+def test_per_graph_results_by_size(sizes, labels):
+    """One block per graph up to 2,048 nodes, the global sort with a larger one:
+    both against results taken from the oracle's colouring of the union."""
+    rng = np.random.default_rng(sum(sizes))
+    parts = [G.er_undirected(n, 3.0, seed=7 + n) for n in sizes] * 2  # every graph twice: shared colours
+    off, idx, nb = G.disjoint_union(parts)
+    init = np.concatenate([rng.integers(0, labels, n) for n in sizes] * 2).astype(np.uint32)
+    ex = oracle.refine_exact(off, idx, None, init)
+    with R.Context(0) as ctx:
+        g = ctx.upload(off, idx)
+        res = [ctx.batch_refine(off, idx, nb, init=init), g.batch_refine(nb, init=init)]
+        g.free()
+    for b in res:
+        assert np.array_equal(b.colors, ex.labels)
+        for i in range(len(parts)):
+            lo, hi = int(nb[i]), int(nb[i + 1])
+            c, first, inv, cnt = np.unique(ex.labels[lo:hi], return_index=True, return_inverse=True, return_counts=True)
+            hc, hn = b.histogram(i)
+            assert np.array_equal(hc, c) and np.array_equal(hn, cnt) and b.blocks[i] == len(c)
+            assert np.array_equal(b.local[lo:hi], first[inv])
+        half = len(parts) // 2
+        same = [all(map(np.array_equal, b.histogram(i), b.histogram(i + half))) for i in range(half)]
+        assert [bool(x) for x in b.fingerprint[:half] == b.fingerprint[half:]] == same
