@@ -18,8 +18,8 @@ using namespace rbsc;
 
 namespace {
 
-// Graphs up to these sizes run on one cluster of 8 blocks, larger ones on the
-// whole chip (us a refinement, cluster / chip: 3,000 nodes and 12,000 arcs
+// Graphs that fit one block's shared memory (fused_fits_block) run there, the
+// next larger ones on one cluster of 8 blocks, larger ones on the whole chip (us a refinement, cluster / chip: 3,000 nodes and 12,000 arcs
 // 70 / 71, 8,000 and 32,000 76-97 / 72-84, 16,000 and 64,000 115-135 / 80-87).
 constexpr uint32_t kClusterNodes = 8192;
 constexpr uint64_t kClusterArcs = 1u << 15;
@@ -37,13 +37,22 @@ bool default_knobs(const rbsc_opts& o)
 
 bool one_cluster(uint32_t n, uint64_t m) { return n <= kClusterNodes && m <= kClusterArcs; }
 
-rbsc_status launch(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
+rbsc_status launch(rbsc_ctx* ctx, FusedArgs& a, const FusedLayout& l, bool block, cudaStream_t s)
 {
     const bool cluster = one_cluster(a.n, a.m);
     cudaLaunchConfig_t cfg{};
     cfg.blockDim = kFuThreads;
     cfg.stream = s;
     cudaLaunchAttribute at{};
+    if (block) {
+        const void* k = a.wt ? (const void*)k_refine_block<true> : (const void*)k_refine_block<false>;
+        EK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFuBlockSmem));
+        cfg.gridDim = 1;
+        cfg.dynamicSmemBytes = fused_block_smem(a, l);
+        ++rbsc::launch_counter();
+        EK(a.wt ? cudaLaunchKernelEx(&cfg, k_refine_block<true>, a, l) : cudaLaunchKernelEx(&cfg, k_refine_block<false>, a, l));
+        return RBSC_OK;
+    }
     if (cluster) {
         cfg.gridDim = kClusterBlocks;
         at.id = cudaLaunchAttributeClusterDimension;
@@ -59,10 +68,13 @@ rbsc_status launch(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     ++rbsc::launch_counter();
-    if (cluster) EK(a.wt ? cudaLaunchKernelEx(&cfg, k_refine_fused<true, true>, a) : cudaLaunchKernelEx(&cfg, k_refine_fused<true, false>, a));
-    else EK(a.wt ? cudaLaunchKernelEx(&cfg, k_refine_fused<false, true>, a) : cudaLaunchKernelEx(&cfg, k_refine_fused<false, false>, a));
+    if (cluster) EK(a.wt ? cudaLaunchKernelEx(&cfg, k_refine_fused<kFuCluster, true>, a) : cudaLaunchKernelEx(&cfg, k_refine_fused<kFuCluster, false>, a));
+    else EK(a.wt ? cudaLaunchKernelEx(&cfg, k_refine_fused<kFuGrid, true>, a) : cudaLaunchKernelEx(&cfg, k_refine_fused<kFuGrid, false>, a));
     return RBSC_OK;
 }
+
+// The rows are a CSR's.
+bool rows_side_by_side(const FusedArgs& a) { return a.off_end == static_cast<const char*>(a.off) + (a.off64 ? 8 : 4); }
 
 rbsc_status ensure_pinned(rbsc_ctx* ctx)
 {
@@ -167,11 +179,11 @@ rbsc_status deep_tail(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
 }
 
 // One launch, waited for.
-rbsc_status launch_and_wait(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
+rbsc_status launch_and_wait(rbsc_ctx* ctx, FusedArgs& a, const FusedLayout& l, bool block, cudaStream_t s)
 {
     std::unique_lock<std::mutex> lock;
-    if (!one_cluster(a.n, a.m)) lock = coop_lock(ctx->device);
-    EKS(launch(ctx, a, s));
+    if (!block && !one_cluster(a.n, a.m)) lock = coop_lock(ctx->device);
+    EKS(launch(ctx, a, l, block, s));
     EK(cudaEventRecord(ctx->ev[1], s));
     EK(cudaStreamSynchronize(s));
     return RBSC_OK;
@@ -179,17 +191,20 @@ rbsc_status launch_and_wait(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
 
 // The launch, and where it stops early the work-list passes and a launch that
 // confirms them; waits for the stream.  ev[0] and ev[1] enclose it.
-rbsc_status run(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
+rbsc_status run(rbsc_ctx* ctx, FusedArgs& a, const FusedLayout& l, cudaStream_t s)
 {
     FusedResult& r = *static_cast<FusedResult*>(ctx->h_fused);
-    a.deep_round = deep_round(a.m);
+    // one block keeps its classes in shared memory: nothing to continue from
+    // (and a pass there costs less than one on the work list)
+    const bool block = rows_side_by_side(a) && fused_fits_block(a, l);
+    a.deep_round = block ? 0u : deep_round(a.m);
     EK(cudaEventRecord(ctx->ev[0], s));
-    EKS(launch_and_wait(ctx, a, s));
+    EKS(launch_and_wait(ctx, a, l, block, s));
     const uint32_t initial = r.initial_blocks;
     const uint64_t t0 = r.t[0], t1 = r.t[1];
     while (r.status == kFuDeep) {
         EKS(deep_tail(ctx, a, s));
-        EKS(launch_and_wait(ctx, a, s));
+        EKS(launch_and_wait(ctx, a, l, false, s));
         r.initial_blocks = initial;
         r.t[0] = t0;
         r.t[1] = t1;
@@ -277,7 +292,7 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
     a.out = d_out;
     a.validate = g->prepared ? 0 : 1;
     common_args(ctx, a);
-    EKS(run(ctx, a, s));
+    EKS(run(ctx, a, l, s));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (!g->prepared) cudaEventElapsedTime(&g->up_ms, ctx->ev[2], ctx->ev[3]);
@@ -306,7 +321,7 @@ rbsc_status fused_refine_rows(rbsc_ctx* ctx, const FusedRows& r, const uint32_t*
     a.init = d_init;
     a.out = d_out;
     common_args(ctx, a);
-    EKS(run(ctx, a, s));
+    EKS(run(ctx, a, l, s));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (stats) std::memset(stats, 0, sizeof *stats);
@@ -340,25 +355,31 @@ rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init
     if (b_wt) std::memcpy(h + o_wt, c->weights, b_wt);
     if (b_init) std::memcpy(h + o_init, init, b_init);
     const FusedLayout l = fused_layout(n, c->m);
-    Scratch sc(ctx);
-    unsigned char* d = nullptr;
-    EKS(sc.get(&d, l.bytes + in));
-    unsigned char* din = d + l.bytes;
     FusedArgs a{};
-    fused_bind(a, l, d);
     a.n = n;
     a.m = c->m;
-    fused_csr(a, din, c->offset_bytes == 8);
-    a.idx = reinterpret_cast<const uint32_t*>(din + o_idx);
-    a.wt = b_wt ? reinterpret_cast<const uint64_t*>(din + o_wt) : nullptr;
-    a.init = b_init ? reinterpret_cast<const uint32_t*>(din + o_init) : nullptr;
+    auto bind_input = [&](unsigned char* p) {
+        fused_csr(a, p, c->offset_bytes == 8);
+        a.idx = reinterpret_cast<const uint32_t*>(p + o_idx);
+        a.wt = b_wt ? reinterpret_cast<const uint64_t*>(p + o_wt) : nullptr;
+        a.init = b_init ? reinterpret_cast<const uint32_t*>(p + o_init) : nullptr;
+    };
+    bind_input(h);
+    const bool block = fused_fits_block(a, l);
+    Scratch sc(ctx);
+    EK(cudaEventRecord(ctx->ev[2], s));
+    if (!block) {  // one block brings the arrays in itself, straight from the pinned buffer
+        unsigned char* d = nullptr;
+        EKS(sc.get(&d, l.bytes + in));
+        fused_bind(a, l, d);
+        bind_input(d + l.bytes);
+        EK(cudaMemcpyAsync(d + l.bytes, h, in, cudaMemcpyHostToDevice, s));
+    }
+    EK(cudaEventRecord(ctx->ev[3], s));
     a.out = h_out;
     a.validate = 1;
     common_args(ctx, a);
-    EK(cudaEventRecord(ctx->ev[2], s));
-    EK(cudaMemcpyAsync(din, h, in, cudaMemcpyHostToDevice, s));
-    EK(cudaEventRecord(ctx->ev[3], s));
-    EKS(run(ctx, a, s));
+    EKS(run(ctx, a, l, s));
     float ms = 0.f, up = 0.f;
     cudaEventElapsedTime(&up, ctx->ev[2], ctx->ev[3]);
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);

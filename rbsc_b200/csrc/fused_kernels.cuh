@@ -37,9 +37,12 @@
 // R-MAT-14 (228,000 arcs), first pass with only rows above 512 arcs shared:
 // 90 us, one warp holding most of the arcs.
 //
-// CLUSTER: the grid is one cluster (blocks are resident together by
-// construction, hardware barrier); otherwise a cooperative launch with a
-// counter barrier whose waits are bounded.
+// MODE: a cooperative grid with a counter barrier whose waits are bounded
+// (kFuGrid); one cluster, whose blocks are resident together by construction
+// (kFuCluster: hardware barrier, block totals exchanged through the blocks'
+// shared memory); or one block with the graph and all working arrays in shared
+// memory (kFuBlock): a pass of a 1,000-arc graph is then a microsecond of work
+// instead of nine dependent trips to L2.
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -124,12 +127,27 @@ struct FusedArgs {
 
 constexpr uint32_t kFuDeepNew = 256;  // "few": at most this many
 
-__device__ __forceinline__ uint64_t fu_ld(const void* p, bool wide, uint32_t u)
+constexpr int kFuGrid = 0, kFuCluster = 1, kFuBlock = 2;
+
+// Loads of arrays that the launch itself writes (at L2) and of its inputs; in
+// kFuBlock both lie in shared memory.
+template <int MODE, typename T> __device__ __forceinline__ T fu_cg(const T* p)
 {
-    return wide ? __ldg(reinterpret_cast<const unsigned long long*>(p) + u) : (uint64_t)__ldg(reinterpret_cast<const uint32_t*>(p) + u);
+    if constexpr (MODE == kFuBlock) return *(const volatile T*)p;
+    else return __ldcg(p);
 }
-__device__ __forceinline__ uint64_t fu_off(const FusedArgs& a, uint32_t u) { return fu_ld(a.off, a.off64, u); }
-__device__ __forceinline__ uint64_t fu_end(const FusedArgs& a, uint32_t u) { return fu_ld(a.off_end, a.off64, u); }
+template <int MODE, typename T> __device__ __forceinline__ T fu_ro(const T* p)
+{
+    if constexpr (MODE == kFuBlock) return *p;
+    else return __ldg(p);
+}
+template <int MODE> __device__ __forceinline__ uint64_t fu_ld(const void* p, bool wide, uint32_t u)
+{
+    return wide ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(p) + u)
+                : (uint64_t)fu_ro<MODE>(reinterpret_cast<const uint32_t*>(p) + u);
+}
+template <int MODE = kFuGrid> __device__ __forceinline__ uint64_t fu_off(const FusedArgs& a, uint32_t u) { return fu_ld<MODE>(a.off, a.off64, u); }
+template <int MODE = kFuGrid> __device__ __forceinline__ uint64_t fu_end(const FusedArgs& a, uint32_t u) { return fu_ld<MODE>(a.off_end, a.off64, u); }
 
 // Whether a row of d arcs in a group of `group` arcs goes in chunks.
 __device__ __forceinline__ bool fu_shared_row(uint32_t d, uint32_t group)
@@ -178,12 +196,13 @@ __device__ __forceinline__ void fu_cache_clear(FuCache& c)
 // shared memory: the few big classes of an early pass would otherwise be one
 // L2 address for the whole grid.  A cache word is written once per pass, by
 // the thread whose compare-and-swap took it.
+template <int MODE>
 __device__ __forceinline__ uint32_t fu_insert(unsigned long long* __restrict__ tab, uint32_t log2tab, uint64_t fp, bool multi, FuCache& cache,
                                               bool& claimed)
 {
     const uint64_t h = fp * kGolden;
     const uint32_t ci = (uint32_t)(h >> 20) & (kFuCache - 1u);
-    const uint64_t ck = *(volatile unsigned long long*)&cache.key[ci];
+    const uint64_t ck = MODE == kFuBlock ? 1ull : *(volatile unsigned long long*)&cache.key[ci];
     claimed = false;
     if (ck == fp) {
         const uint32_t s = *(volatile uint32_t*)&cache.slot[ci];
@@ -194,7 +213,7 @@ __device__ __forceinline__ uint32_t fu_insert(unsigned long long* __restrict__ t
     // at most half of the entries are taken, so an empty one ends the probe;
     // the bound only keeps a broken table from looping
     for (uint32_t probe = 0; probe <= mask; ++probe, s = (s + 1u) & mask) {
-        unsigned long long e = __ldcg(tab + s);
+        unsigned long long e = fu_cg<MODE>(tab + s);
         if (e == 0ull) {
             e = atomicCAS(tab + s, 0ull, (unsigned long long)fp | (multi ? 1ull : 0ull));
             if (e == 0ull) {
@@ -215,6 +234,7 @@ __device__ __forceinline__ uint32_t fu_insert(unsigned long long* __restrict__ t
 // The lanes with `need` insert their keys; `few`: the classes are few beside
 // the nodes, so lanes with equal keys send one of them (32 compare-and-swaps
 // of a warp on one address would be served one after another).
+template <int MODE>
 __device__ __forceinline__ uint32_t fu_insert_warp(bool need, bool few, unsigned long long* __restrict__ tab, uint32_t log2tab,
                                                    uint64_t fp, FuCache& cache, uint32_t& made)
 {
@@ -225,10 +245,10 @@ __device__ __forceinline__ uint32_t fu_insert_warp(bool need, bool few, unsigned
         if (few) {
             const unsigned peers = __match_any_sync(m, (unsigned long long)fp);
             const int leader = __ffs(peers) - 1;
-            if ((int)(threadIdx.x & 31) == leader) s = fu_insert(tab, log2tab, fp, (peers & (peers - 1u)) != 0u, cache, claimed);
+            if ((int)(threadIdx.x & 31) == leader) s = fu_insert<MODE>(tab, log2tab, fp, (peers & (peers - 1u)) != 0u, cache, claimed);
             s = __shfl_sync(peers, s, leader);
         } else {
-            s = fu_insert(tab, log2tab, fp, false, cache, claimed);
+            s = fu_insert<MODE>(tab, log2tab, fp, false, cache, claimed);
         }
         made += claimed ? 1u : 0u;
     }
@@ -246,41 +266,56 @@ struct FuSync {
     uint32_t seen0 = 0, seen1 = 0;  // the words' high halves after their last barriers
 };
 
-template <bool CLUSTER>
+template <int MODE>
 __device__ __forceinline__ bool fu_barrier(FusedWords* w, FuSync& y, uint32_t val, uint32_t* total, uint32_t* s_word)
 {
     const uint32_t par = y.epoch & 1u;
     const unsigned target = ((y.epoch >> 1) + 1u) * gridDim.x;  // arrivals at this word
     ++y.epoch;
+    if constexpr (MODE == kFuBlock) {
+        __syncthreads();
+        if (total) *total = val;  // every thread of the block has its total
+        return true;
+    }
+    if constexpr (MODE == kFuCluster) {
+        // thread i hands the block's value to block i: the sums need no trip to L2
+        uint32_t* const part = s_word + 2 + 8 * par;
+        if (threadIdx.x < gridDim.x) {
+            uint32_t mine = (uint32_t)__cvta_generic_to_shared(part + blockIdx.x), there;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(mine), "r"(threadIdx.x));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(there), "r"(val) : "memory");
+        }
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (total) {
+            uint32_t all = 0;
+            for (uint32_t i = 0; i < gridDim.x; ++i) all += *(volatile uint32_t*)(part + i);
+            *total = all;
+        }
+        return true;
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
         unsigned long long* const word = &w->bar[par];
         const unsigned long long add = ((unsigned long long)val << 32) | 1ull;
         __threadfence();
         unsigned long long v = atomicAdd(word, add) + add;
-        if (!CLUSTER) {
-            uint32_t it = 0;
-            while ((uint32_t)v < target) {
-                if (++it > (1u << 22)) {  // about two seconds
-                    s_word[1] = 1u;
-                    break;
-                }
-                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
+        uint32_t it = 0;
+        while ((uint32_t)v < target) {
+            if (++it > (1u << 22)) {  // about two seconds
+                s_word[1] = 1u;
+                break;
             }
-            s_word[0] = (uint32_t)(v >> 32);
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
         }
+        s_word[0] = (uint32_t)(v >> 32);
         __threadfence();
-    }
-    if (CLUSTER) {
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        if (threadIdx.x == 0) s_word[0] = (uint32_t)(__ldcg(&w->bar[par]) >> 32);
     }
     __syncthreads();
     const uint32_t all = *(volatile uint32_t*)&s_word[0];
     if (total) *total = all - (par ? y.seen1 : y.seen0);
     if (par) y.seen1 = all;
     else y.seen0 = all;
-    return CLUSTER || *(volatile uint32_t*)&s_word[1] == 0u;
+    return *(volatile uint32_t*)&s_word[1] == 0u;
 }
 
 // Group g (of 32 / G) of a warp takes the g-th set bit of `m` as its source
@@ -322,7 +357,7 @@ __device__ __forceinline__ bool fu_lane_differs(uint32_t a, uint32_t b, uint64_t
 
 // The rows (bu, du) and (br, dr) of the lanes in `m`, G lanes each; sets the
 // owner lane's `bad`.
-template <bool WEIGHTED, int G>
+template <int MODE, bool WEIGHTED, int G>
 __device__ __forceinline__ void fu_check_rows(unsigned m, int lane, const uint32_t* __restrict__ idx, const uint64_t* __restrict__ wt,
                                               const uint32_t* __restrict__ col, uint64_t bu, uint32_t du, uint64_t br, uint32_t dr,
                                               bool& bad)
@@ -338,12 +373,12 @@ __device__ __forceinline__ void fu_check_rows(unsigned m, int lane, const uint32
         uint64_t wa = 0, wb = 0;
         if (src >= 0) {
             if ((uint32_t)gl < xdu) {
-                a = __ldcg(col + __ldg(idx + xbu + gl));
-                if (WEIGHTED) wa = __ldg(reinterpret_cast<const unsigned long long*>(wt) + xbu + gl);
+                a = fu_cg<MODE>(col + fu_ro<MODE>(idx + xbu + gl));
+                if (WEIGHTED) wa = fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + xbu + gl);
             }
             if ((uint32_t)gl < xdr) {
-                b = __ldcg(col + __ldg(idx + xbr + gl));
-                if (WEIGHTED) wb = __ldg(reinterpret_cast<const unsigned long long*>(wt) + xbr + gl);
+                b = fu_cg<MODE>(col + fu_ro<MODE>(idx + xbr + gl));
+                if (WEIGHTED) wb = fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + xbr + gl);
             }
         }
         const unsigned diff = __ballot_sync(0xffffffffu, fu_lane_differs<WEIGHTED, G>(a, b, wa, wb));
@@ -391,7 +426,7 @@ template <int K> __device__ __forceinline__ void fu_sort(uint32_t (&v)[K])
 
 // The rows of the lanes in `m` (unit weights, equal lengths of at most 32 * K
 // arcs), one after another by the whole warp.
-template <int K>
+template <int MODE, int K>
 __device__ __forceinline__ void fu_check_long(unsigned m, int lane, const uint32_t* __restrict__ idx, const uint32_t* __restrict__ col,
                                               uint64_t bu, uint64_t br, uint32_t d, bool& bad)
 {
@@ -404,8 +439,8 @@ __device__ __forceinline__ void fu_check_long(unsigned m, int lane, const uint32
 #pragma unroll
         for (int q = 0; q < K; ++q) {
             const uint32_t i = 32u * q + lane;
-            a[q] = i < xd ? __ldcg(col + __ldg(idx + xbu + i)) : 0xffffffffu;
-            b[q] = i < xd ? __ldcg(col + __ldg(idx + xbr + i)) : 0xffffffffu;
+            a[q] = i < xd ? fu_cg<MODE>(col + fu_ro<MODE>(idx + xbu + i)) : 0xffffffffu;
+            b[q] = i < xd ? fu_cg<MODE>(col + fu_ro<MODE>(idx + xbr + i)) : 0xffffffffu;
         }
         fu_sort<K>(a);
         fu_sort<K>(b);
@@ -430,13 +465,13 @@ __device__ __forceinline__ bool fu_count(uint32_t* key, unsigned long long* val,
     return false;
 }
 
-template <bool CLUSTER, bool WEIGHTED>
-static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __grid_constant__ FusedArgs a)
+template <int MODE, bool WEIGHTED>
+__device__ __forceinline__ void fused_body(const FusedArgs& a)
 {
     __shared__ FuCache s_cache;
     __shared__ unsigned long long s_val[kFuCheckSlots];
     __shared__ uint32_t s_key[kFuCheckSlots];
-    __shared__ uint32_t s_sum, s_flag, s_word[2];
+    __shared__ uint32_t s_sum, s_flag, s_word[2 + 16];
     __shared__ uint32_t s_delta[kFuThreads];  // per warp: its rows' (first arc - position) by rank
     const uint32_t n = a.n;
     const int lane = threadIdx.x & 31;
@@ -457,14 +492,14 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         s_word[0] = s_word[1] = 0u;
     }
     fu_cache_clear(s_cache);
-    if (CLUSTER) {
+    if constexpr (MODE != kFuGrid) {
         if (first) {
-            w->bar[0] = w->bar[1] = 0ull;
             w->bad = w->overflow = 0u;
             w->nlong = w->nchunk = 0u;
             w->nlist[0] = w->nlist[1] = 0u;
         }
-        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if constexpr (MODE == kFuBlock) __syncthreads();
+        else asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
 
     auto finish = [&](int status, uint32_t rounds, uint32_t blocks, uint32_t initial, uint32_t repairs) {
@@ -516,8 +551,8 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         uint64_t b = 0, e = 0;
         bool bad = false;
         if (u < n) {
-            b = fu_off(a, u);
-            e = fu_end(a, u);
+            b = fu_off<MODE>(a, u);
+            e = fu_end<MODE>(a, u);
             bad = a.validate && (b > e || e > a.m || (u == 0 && b != 0) || (u == n - 1 && e != a.m));
             if (!ini) a.col[0][u] = 0u;
         }
@@ -538,20 +573,20 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
     }
     if (a.validate)
         for (uint64_t k = gt; k < a.m; k += nt)
-            if (__ldg(idx + k) >= n) bad_in |= 2u;
+            if (fu_ro<MODE>(idx + k) >= n) bad_in |= 2u;
     if (bad_in) atomicOr(&w->bad, bad_in);
-    if (!fu_barrier<CLUSTER>(w, sync, 0u, nullptr, s_word)) {
+    if (!fu_barrier<MODE>(w, sync, 0u, nullptr, s_word)) {
         finish(kFuBarrier, 0u, 0u, 0u, 0u);
         return;
     }
     {
-        const uint32_t bad = __ldcg(&w->bad);
+        const uint32_t bad = fu_cg<MODE>(&w->bad);
         if (bad) {  // nothing is written, nothing read through the graph
             finish((bad & 1u) ? kFuBadOffsets : kFuBadHead, 0u, 0u, 0u, 0u);
             return;
         }
     }
-    const uint32_t nchunk = min(__ldcg(&w->nchunk), a.chunk_cap);
+    const uint32_t nchunk = min(fu_cg<MODE>(&w->nchunk), a.chunk_cap);
 
     uint32_t p = 0;  // current colours: col[p & 1], classes: tab[p % 3]
     uint32_t made = 0;
@@ -567,12 +602,12 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
             const uint32_t u = base + lane;
             const bool valid = u < n;
-            const uint64_t fp = valid ? ((uint64_t)__ldcg(ini + u) + 1ull) << 1 : 0ull;
-            const uint32_t s = fu_insert_warp(valid, true, a.tab[0], a.log2tab, fp, s_cache, made);
+            const uint64_t fp = valid ? ((uint64_t)fu_cg<MODE>(ini + u) + 1ull) << 1 : 0ull;
+            const uint32_t s = fu_insert_warp<MODE>(valid, true, a.tab[0], a.log2tab, fp, s_cache, made);
             if (valid) a.col[0][u] = s;
         }
         const uint32_t tot = block_total(made);
-        if (!fu_barrier<CLUSTER>(w, sync, tot, &prev, s_word)) {
+        if (!fu_barrier<MODE>(w, sync, tot, &prev, s_word)) {
             finish(kFuBarrier, 0u, 0u, 0u, 0u);
             return;
         }
@@ -609,17 +644,17 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
             const uint32_t u = base + lane;
             const bool valid = u < n;
-            uint32_t c = valid ? __ldcg(co + u) : kSingleton;
+            uint32_t c = valid ? fu_cg<MODE>(co + u) : kSingleton;
             bool act = !(c & kSingleton);
             unsigned long long e = 1ull;
             uint64_t b = 0;
             uint32_t d = 0;
             if (valid && !repair) {
-                b = fu_off(a, u);
-                d = (uint32_t)(fu_end(a, u) - b);
+                b = fu_off<MODE>(a, u);
+                d = (uint32_t)(fu_end<MODE>(a, u) - b);
             }
             if (act) {
-                if (has_classes) e = __ldcg(tp + c);
+                if (has_classes) e = fu_cg<MODE>(tp + c);
                 else e = n > 1u ? 1ull : 0ull;
                 if (!(e & 1ull)) {  // nobody joined: alone for good
                     act = false;
@@ -667,14 +702,14 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
                             pos[q] = j + lane < total ? delta[rank - 1u] + j + lane : 0xffffffffu;
                         }
 #pragma unroll
-                        for (int q = 0; q < U; ++q) cc[q] = pos[q] != 0xffffffffu ? __ldg(idx + pos[q]) : 0u;
+                        for (int q = 0; q < U; ++q) cc[q] = pos[q] != 0xffffffffu ? fu_ro<MODE>(idx + pos[q]) : 0u;
                         if (WEIGHTED) {
 #pragma unroll
                             for (int q = 0; q < U; ++q)
-                                x[q] = pos[q] != 0xffffffffu ? __ldg(reinterpret_cast<const unsigned long long*>(wt) + pos[q]) : 0ull;
+                                x[q] = pos[q] != 0xffffffffu ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + pos[q]) : 0ull;
                         }
 #pragma unroll
-                        for (int q = 0; q < U; ++q) cc[q] = pos[q] != 0xffffffffu ? __ldcg(co + cc[q]) : 0u;
+                        for (int q = 0; q < U; ++q) cc[q] = pos[q] != 0xffffffffu ? fu_cg<MODE>(co + cc[q]) : 0u;
 #pragma unroll
                         for (int q = 0; q < U; ++q) {
                             uint64_t t = pos[q] != 0xffffffffu ? fu_term(cc[q], salt) : 0ull;
@@ -700,21 +735,21 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
                 }
                 if (act) fp = fingerprint(c, s1);
             }
-            const uint32_t s = fu_insert_warp(act, few, tc, a.log2tab, fp, s_cache, made);
+            const uint32_t s = fu_insert_warp<MODE>(act, few, tc, a.log2tab, fp, s_cache, made);
             if (act) cn[u] = s;
         }
         if (!repair && !uniform)
             for (uint32_t ch = nw - 1u - gw; ch < nchunk; ch += nw) {
                 const uint32_t j = a.lchunk[ch], u = a.lrow[j], f = a.lfirst[j];
-                const uint32_t c = __ldcg(co + u);
-                if ((c & kSingleton) || (has_classes && !(__ldcg(tp + c) & 1ull)) || n == 1u) continue;
-                const uint64_t b = fu_off(a, u), e = fu_end(a, u);
+                const uint32_t c = fu_cg<MODE>(co + u);
+                if ((c & kSingleton) || (has_classes && !(fu_cg<MODE>(tp + c) & 1ull)) || n == 1u) continue;
+                const uint64_t b = fu_off<MODE>(a, u), e = fu_end<MODE>(a, u);
                 const uint64_t s = b + (uint64_t)(ch - f) * kFuChunk, t = min(e, s + kFuChunk);
                 uint64_t sum = 0;
 #pragma unroll 8
                 for (uint64_t i = s + lane; i < t; i += 32) {
-                    const uint64_t x = fu_term(__ldcg(co + __ldg(idx + i)), salt);
-                    sum += WEIGHTED ? x * __ldg(reinterpret_cast<const unsigned long long*>(wt) + i) : x;
+                    const uint64_t x = fu_term(fu_cg<MODE>(co + fu_ro<MODE>(idx + i)), salt);
+                    sum += WEIGHTED ? x * fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + i) : x;
                 }
                 sum = fu_warp_sum(sum, 32);
                 if (lane == 0) {
@@ -732,13 +767,13 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
                     }
                     if (last) {
                         bool claimed;
-                        cn[u] = fu_insert(tc, a.log2tab, fingerprint(c, sum), false, s_cache, claimed);
+                        cn[u] = fu_insert<MODE>(tc, a.log2tab, fingerprint(c, sum), false, s_cache, claimed);
                         made += claimed ? 1u : 0u;
                     }
                 }
             }
         const uint32_t tot = block_total(made);
-        if (!fu_barrier<CLUSTER>(w, sync, tot, &count, s_word)) return false;
+        if (!fu_barrier<MODE>(w, sync, tot, &count, s_word)) return false;
         ++p;
         has_classes = true;
         return true;
@@ -774,10 +809,10 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         const uint32_t par = repairs & 1u;
         if (first) w->nlist[par ^ 1u] = 0u;
         for (uint32_t u = gt; u < n; u += nt) {
-            const uint32_t c = __ldcg(col + u);
-            if (!(c & kSingleton) && __ldcg(a.minm + c) > u) atomicMin(a.minm + c, u);
+            const uint32_t c = fu_cg<MODE>(col + u);
+            if (!(c & kSingleton) && fu_cg<MODE>(a.minm + c) > u) atomicMin(a.minm + c, u);
         }
-        if (!fu_barrier<CLUSTER>(w, sync, 0u, nullptr, s_word)) {
+        if (!fu_barrier<MODE>(w, sync, 0u, nullptr, s_word)) {
             finish(kFuBarrier, round, prev, initial, repairs);
             return;
         }
@@ -787,32 +822,32 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
             const uint32_t u = base + lane;
             const bool valid = u < n;
-            const uint32_t c = valid ? __ldcg(col + u) : kSingleton;
-            const uint32_t r = (c & kSingleton) ? u : __ldcg(a.minm + c);
+            const uint32_t c = valid ? fu_cg<MODE>(col + u) : kSingleton;
+            const uint32_t r = (c & kSingleton) ? u : fu_cg<MODE>(a.minm + c);
             if (valid) a.out[u] = r;
             if (!check) continue;
             const bool chk = valid && r != u;
             uint64_t bu = 0, br = 0;
             uint32_t du = 0, dr = 0, iu = 0, ir = 0;
             if (chk) {
-                bu = fu_off(a, u);
-                br = fu_off(a, r);
-                du = (uint32_t)(fu_end(a, u) - bu);
-                dr = (uint32_t)(fu_end(a, r) - br);
+                bu = fu_off<MODE>(a, u);
+                br = fu_off<MODE>(a, r);
+                du = (uint32_t)(fu_end<MODE>(a, u) - bu);
+                dr = (uint32_t)(fu_end<MODE>(a, r) - br);
                 if (a.init) {
-                    iu = __ldg(a.init + u);
-                    ir = __ldg(a.init + r);
+                    iu = fu_ro<MODE>(a.init + u);
+                    ir = fu_ro<MODE>(a.init + r);
                 }
             }
             bool bad = chk && (iu != ir || (!WEIGHTED && du != dr));
             const uint32_t mx = chk && !bad ? max(du, dr) : 0u;
-            fu_check_rows<WEIGHTED, 8>(__ballot_sync(0xffffffffu, mx > 0 && mx <= 8), lane, idx, wt, col, bu, du, br, dr, bad);
-            fu_check_rows<WEIGHTED, 16>(__ballot_sync(0xffffffffu, mx > 8 && mx <= 16), lane, idx, wt, col, bu, du, br, dr, bad);
-            fu_check_rows<WEIGHTED, 32>(__ballot_sync(0xffffffffu, mx > 16 && mx <= 32), lane, idx, wt, col, bu, du, br, dr, bad);
+            fu_check_rows<MODE, WEIGHTED, 8>(__ballot_sync(0xffffffffu, mx > 0 && mx <= 8), lane, idx, wt, col, bu, du, br, dr, bad);
+            fu_check_rows<MODE, WEIGHTED, 16>(__ballot_sync(0xffffffffu, mx > 8 && mx <= 16), lane, idx, wt, col, bu, du, br, dr, bad);
+            fu_check_rows<MODE, WEIGHTED, 32>(__ballot_sync(0xffffffffu, mx > 16 && mx <= 32), lane, idx, wt, col, bu, du, br, dr, bad);
             uint32_t reg = 32;  // longest row compared in registers
             if (!WEIGHTED) {
-                fu_check_long<2>(__ballot_sync(0xffffffffu, mx > 32 && mx <= 64), lane, idx, col, bu, br, du, bad);
-                fu_check_long<4>(__ballot_sync(0xffffffffu, mx > 64 && mx <= 128), lane, idx, col, bu, br, du, bad);
+                fu_check_long<MODE, 2>(__ballot_sync(0xffffffffu, mx > 32 && mx <= 64), lane, idx, col, bu, br, du, bad);
+                fu_check_long<MODE, 4>(__ballot_sync(0xffffffffu, mx > 64 && mx <= 128), lane, idx, col, bu, br, du, bad);
                 reg = 128;
             }
             const unsigned ml = __ballot_sync(0xffffffffu, mx > reg);
@@ -832,11 +867,11 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
         if (threadIdx.x == 0) s_sum = 0u;
         __syncthreads();
         uint32_t tot = block_total(nbad), nfail = 0, more = 0;
-        if (!fu_barrier<CLUSTER>(w, sync, tot, &nfail, s_word)) {
+        if (!fu_barrier<MODE>(w, sync, tot, &nfail, s_word)) {
             finish(kFuBarrier, round, prev, initial, repairs);
             return;
         }
-        const uint32_t nlist = __ldcg(&w->nlist[par]);
+        const uint32_t nlist = fu_cg<MODE>(&w->nlist[par]);
         if (nlist) {
             // longer rows: colours counted in a table, + for the member's row
             // and - for the node's; all must end at 0.  A warp tries the short
@@ -846,22 +881,22 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
             auto add_row = [&](uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t x, bool minus, uint32_t at,
                                uint32_t step) -> bool {
                 bool ok = true;
-                const uint64_t b = fu_off(a, x), e = fu_end(a, x);
+                const uint64_t b = fu_off<MODE>(a, x), e = fu_end<MODE>(a, x);
                 for (uint64_t i = b + at; i < e; i += step) {
-                    const uint64_t v = WEIGHTED ? __ldg(reinterpret_cast<const unsigned long long*>(wt) + i) : 1ull;
-                    ok &= fu_count(key, val, mask, __ldcg(col + __ldg(idx + i)), minus ? 0ull - v : v);
+                    const uint64_t v = WEIGHTED ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + i) : 1ull;
+                    ok &= fu_count(key, val, mask, fu_cg<MODE>(col + fu_ro<MODE>(idx + i)), minus ? 0ull - v : v);
                 }
                 return ok;
             };
             auto longest = [&](uint32_t u, uint32_t r) {
-                return max((uint32_t)(fu_end(a, u) - fu_off(a, u)), (uint32_t)(fu_end(a, r) - fu_off(a, r)));
+                return max((uint32_t)(fu_end<MODE>(a, u) - fu_off<MODE>(a, u)), (uint32_t)(fu_end<MODE>(a, r) - fu_off<MODE>(a, r)));
             };
             if (WEIGHTED) {
                 const uint32_t wi = threadIdx.x >> 5;
                 uint32_t* key = s_key + wi * kFuWarpSlots;
                 unsigned long long* val = s_val + wi * kFuWarpSlots;
                 for (uint32_t i = gw; i < nlist; i += nw) {
-                    const uint32_t u = a.list[i], r = __ldcg(a.minm + __ldcg(col + u));
+                    const uint32_t u = a.list[i], r = fu_cg<MODE>(a.minm + fu_cg<MODE>(col + u));
                     if (longest(u, r) > kFuWarpRow) continue;
                     for (uint32_t k = lane; k < kFuWarpSlots; k += 32) {
                         key[k] = 0xffffffffu;
@@ -885,14 +920,14 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
                     __syncwarp();
                 }
                 // the undecided marks are read by other blocks
-                if (!fu_barrier<CLUSTER>(w, sync, 0u, nullptr, s_word)) {
+                if (!fu_barrier<MODE>(w, sync, 0u, nullptr, s_word)) {
                     finish(kFuBarrier, round, prev, initial, repairs);
                     return;
                 }
             }
             for (uint32_t i = blockIdx.x; i < nlist; i += gridDim.x) {
-                const uint32_t u = a.list[i], r = __ldcg(a.minm + __ldcg(col + u));
-                if (WEIGHTED && longest(u, r) <= kFuWarpRow && __ldcg(a.fail + u) != 2) continue;
+                const uint32_t u = a.list[i], r = fu_cg<MODE>(a.minm + fu_cg<MODE>(col + u));
+                if (WEIGHTED && longest(u, r) <= kFuWarpRow && fu_cg<MODE>(a.fail + u) != 2) continue;
                 uint32_t* key = s_key;
                 unsigned long long* val = s_val;
                 uint32_t slots = kFuCheckSlots;
@@ -931,11 +966,11 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
             if (threadIdx.x == 0) s_sum = 0u;
             __syncthreads();
             tot = block_total(nbad);
-            if (!fu_barrier<CLUSTER>(w, sync, tot, &more, s_word)) {
+            if (!fu_barrier<MODE>(w, sync, tot, &more, s_word)) {
                 finish(kFuBarrier, round, prev, initial, repairs);
                 return;
             }
-            if (__ldcg(&w->overflow)) {
+            if (fu_cg<MODE>(&w->overflow)) {
                 finish(kFuRowTooWide, round, prev, initial, repairs);
                 return;
             }
@@ -956,22 +991,32 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __g
             status = kFuNotConverged;
             const uint32_t* __restrict__ cc = a.col[p & 1u];
             for (uint32_t u = gt; u < n; u += nt) {
-                const uint32_t c = __ldcg(cc + u);
-                if (!(c & kSingleton) && __ldcg(a.minm + c) > u) atomicMin(a.minm + c, u);
+                const uint32_t c = fu_cg<MODE>(cc + u);
+                if (!(c & kSingleton) && fu_cg<MODE>(a.minm + c) > u) atomicMin(a.minm + c, u);
             }
-            if (!fu_barrier<CLUSTER>(w, sync, 0u, nullptr, s_word)) {
+            if (!fu_barrier<MODE>(w, sync, 0u, nullptr, s_word)) {
                 finish(kFuBarrier, round, prev, initial, repairs);
                 return;
             }
             for (uint32_t u = gt; u < n; u += nt) {
-                const uint32_t c = __ldcg(cc + u);
-                a.out[u] = (c & kSingleton) ? u : __ldcg(a.minm + c);
+                const uint32_t c = fu_cg<MODE>(cc + u);
+                a.out[u] = (c & kSingleton) ? u : fu_cg<MODE>(a.minm + c);
             }
             finish(status, round, prev, initial, repairs);
             return;
         }
     }
 }
+
+template <int MODE, bool WEIGHTED>
+static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_fused(const __grid_constant__ FusedArgs a)
+{
+    static_assert(MODE != kFuBlock, "k_refine_block");
+    fused_body<MODE, WEIGHTED>(a);
+}
+
+struct FusedLayout;
+inline __host__ __device__ size_t fused_al(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // Working memory of a fused refinement: offsets of its arrays in one block.
 struct FusedLayout {
@@ -985,7 +1030,7 @@ inline FusedLayout fused_layout(uint32_t n, uint64_t m)
     size_t at = 0;
     auto take = [&](size_t bytes) {
         const size_t r = at;
-        at += (bytes + 255) & ~(size_t)255;
+        at += fused_al(bytes);
         return r;
     };
     l.log2tab = 10;
@@ -1015,7 +1060,7 @@ inline void fused_csr(FusedArgs& a, const void* off, bool off64)
     a.off64 = off64 ? 1 : 0;
 }
 
-inline void fused_bind(FusedArgs& a, const FusedLayout& l, unsigned char* base)
+__host__ __device__ inline void fused_bind(FusedArgs& a, const FusedLayout& l, unsigned char* base)
 {
     a.w = reinterpret_cast<FusedWords*>(base + l.words);
     for (int i = 0; i < 2; ++i) a.col[i] = reinterpret_cast<uint32_t*>(base + l.col[i]);
@@ -1031,6 +1076,55 @@ inline void fused_bind(FusedArgs& a, const FusedLayout& l, unsigned char* base)
     a.lchunk = reinterpret_cast<uint32_t*>(base + l.lchunk);
     a.long_cap = l.long_cap;
     a.chunk_cap = l.chunk_cap;
+}
+
+// kFuBlock: the graph's arrays are copied to shared memory (from device or
+// page-locked host memory), behind the working arrays.
+constexpr uint32_t kFuBlockNodes = 1024;
+constexpr uint64_t kFuBlockArcs = 8192;
+constexpr size_t kFuBlockSmem = 184u << 10;  // beside 43 KB of static shared memory
+
+inline size_t fused_block_smem(const FusedArgs& a, const FusedLayout& l)
+{
+    return l.bytes + fused_al((size_t)(a.off64 ? 8 : 4) * ((size_t)a.n + 1)) + fused_al(4 * (size_t)a.m) +
+           (a.wt ? fused_al(8 * (size_t)a.m) : 0) + (a.init ? fused_al(4 * (size_t)a.n) : 0);
+}
+
+// A CSR small enough for one block (offsets side by side, as fused_csr sets them).
+inline bool fused_fits_block(const FusedArgs& a, const FusedLayout& l)
+{
+    return a.n <= kFuBlockNodes && a.m <= kFuBlockArcs && fused_block_smem(a, l) <= kFuBlockSmem;
+}
+
+template <bool WEIGHTED>
+static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_block(const __grid_constant__ FusedArgs in, const __grid_constant__ FusedLayout l)
+{
+    extern __shared__ __align__(256) unsigned char s_work[];
+    __shared__ FusedArgs s_args;
+    const size_t ob = in.off64 ? 8 : 4;
+    unsigned char* const off = s_work + l.bytes;
+    unsigned char* const idx = off + fused_al(ob * ((size_t)in.n + 1));
+    unsigned char* const wt = idx + fused_al(4 * (size_t)in.m);
+    unsigned char* const init = wt + (WEIGHTED ? fused_al(8 * (size_t)in.m) : 0);
+    auto bring = [&](unsigned char* dst, const void* src, size_t bytes) {
+        for (size_t i = threadIdx.x; i < bytes / 4; i += kFuThreads)
+            reinterpret_cast<uint32_t*>(dst)[i] = reinterpret_cast<const uint32_t*>(src)[i];
+    };
+    bring(off, in.off, ob * ((size_t)in.n + 1));
+    bring(idx, in.idx, 4 * (size_t)in.m);
+    if (WEIGHTED) bring(wt, in.wt, 8 * (size_t)in.m);
+    if (in.init) bring(init, in.init, 4 * (size_t)in.n);
+    if (threadIdx.x == 0) {
+        s_args = in;
+        fused_bind(s_args, l, s_work);
+        s_args.off = off;
+        s_args.off_end = off + ob;
+        s_args.idx = reinterpret_cast<const uint32_t*>(idx);
+        s_args.wt = reinterpret_cast<const uint64_t*>(wt);
+        if (in.init) s_args.init = reinterpret_cast<const uint32_t*>(init);
+    }
+    __syncthreads();
+    fused_body<kFuBlock, WEIGHTED>(s_args);
 }
 
 }  // namespace rbsc

@@ -10,8 +10,8 @@
 // __device__ array (g_noalloc_scratch, about 5 MB), which every GPU that loads
 // this library holds until the process exits.
 //
-// The kernel is k_refine_fused (fused_kernels.cuh) as one cluster of eight
-// thread blocks: the same hashed passes, exact check and repair as the
+// The kernel is the one-launch refinement (fused_kernels.cuh), in one thread
+// block for the smallest graphs and one cluster of eight otherwise: the same hashed passes, exact check and repair as the
 // multi-kernel path, so its labels and counts equal those of rbsc_refine on
 // the same graph.
 //
@@ -81,6 +81,11 @@ extern "C" rbsc_status rbsc_refine_noalloc(const rbsc_csr* g, const uint32_t* d_
             e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
             if (e != cudaSuccess)
                 return rbsc_fail(nullptr, RBSC_ERR_CUDA, "cudaGetSymbolAddress(scratch) failed: %s", cudaGetErrorString(e));
+            for (const void* k : {(const void*)k_refine_block<false>, (const void*)k_refine_block<true>}) {
+                e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFuBlockSmem);
+                if (e != cudaSuccess)
+                    return rbsc_fail(nullptr, RBSC_ERR_CUDA, "cudaFuncSetAttribute failed: %s", cudaGetErrorString(e));
+            }
             g_na_ptr[dev] = static_cast<unsigned char*>(p);
         }
         scratch = g_na_ptr[dev];
@@ -108,6 +113,18 @@ extern "C" rbsc_status rbsc_refine_noalloc(const rbsc_csr* g, const uint32_t* d_
     a.hash_bits = o.test_hash_bits < 0 ? 64u : (uint32_t)o.test_hash_bits;
     ++launch_counter();
     cudaLaunchConfig_t cfg{};
+    if (fused_fits_block(a, l)) {
+        cfg.gridDim = 1;
+        cfg.blockDim = kFuThreads;
+        cfg.dynamicSmemBytes = fused_block_smem(a, l);
+        cfg.stream = static_cast<cudaStream_t>(stream);
+        e = a.wt ? cudaLaunchKernelEx(&cfg, k_refine_block<true>, a, l) : cudaLaunchKernelEx(&cfg, k_refine_block<false>, a, l);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return rbsc_fail(nullptr, RBSC_ERR_CUDA, "k_refine_block launch failed: %s", cudaGetErrorString(e));
+        }
+        return RBSC_OK;
+    }
     cfg.gridDim = kNaBlocks;
     cfg.blockDim = kFuThreads;
     cfg.stream = static_cast<cudaStream_t>(stream);
@@ -117,7 +134,7 @@ extern "C" rbsc_status rbsc_refine_noalloc(const rbsc_csr* g, const uint32_t* d_
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    e = a.wt ? cudaLaunchKernelEx(&cfg, k_refine_fused<true, true>, a) : cudaLaunchKernelEx(&cfg, k_refine_fused<true, false>, a);
+    e = a.wt ? cudaLaunchKernelEx(&cfg, k_refine_fused<kFuCluster, true>, a) : cudaLaunchKernelEx(&cfg, k_refine_fused<kFuCluster, false>, a);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return rbsc_fail(nullptr, RBSC_ERR_CUDA, "k_refine_fused launch failed: %s", cudaGetErrorString(e));

@@ -64,10 +64,12 @@ def test_node_counts(n):
     _both(off, idx, None, R.degree_bucket_colors(off))
 
 
-@pytest.mark.parametrize("m", [(1 << 17) - 1, 1 << 17, (1 << 17) + 1])
-def test_arc_counts_around_one_cluster(m):
-    off, idx = G.er_directed(9000, m, seed=m & 7)
+@pytest.mark.parametrize("n,m", [(900, 8191), (900, 8192), (900, 8193), (1024, 3000), (1025, 3000), (8192, (1 << 15) - 1),
+                                 (8192, 1 << 15), (8193, 1 << 15), (8192, (1 << 15) + 1)])
+def test_sizes_around_one_block_and_one_cluster(n, m):
+    off, idx = G.er_directed(n, m, seed=m & 7)
     _both(off, idx, _rng_weights(m), None)
+    _both(off, idx, None, (np.arange(n) % 9).astype(np.uint32))
 
 
 def _rng_weights(m):
