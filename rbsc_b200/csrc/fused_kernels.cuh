@@ -26,11 +26,13 @@
 // fingerprint would merge two classes; the exact check finds that.
 //
 // Rows: nodes are dealt to warps 32 at a time, interleaved over the SMs.  The
-// warp lays the arcs of its unfinished rows end to end and takes 32 of them
-// per step, one per lane (the heads of neighbouring rows lie side by side in
-// memory, so a step's loads coalesce, and no lane waits for a longer row);
+// warp lays the arcs of its unfinished rows end to end and takes 128 of them
+// per step, four per lane (the heads of neighbouring rows lie side by side in
+// memory, so a step touches few lines, and no lane waits for a longer row);
 // a running prefix sum is read off at the row starts, and a row's sum is the
-// difference of two of them.  Rows of more than kFuChunk arcs, and
+// difference of two of them.  (One arc per lane and step took four times the
+// shuffles: the 131,072-node lift 101 us against 96, weighted R-MAT-20 699
+// against 650.)  Rows of more than kFuChunk arcs, and
 // rows of more than kFuGroupRow arcs in a group of more than kFuGroupArcs (the
 // low node ids of an R-MAT graph are all hubs), are cut into chunks that all
 // warps share (the warp that completes a row's last chunk inserts it).
@@ -57,7 +59,7 @@ constexpr int kFuThreads = 1024;
 constexpr uint32_t kFuChunk = 256;
 constexpr uint32_t kFuGroupArcs = 1024;  // a warp's 32 rows together: beyond this its rows of more than
 constexpr uint32_t kFuGroupRow = 64;     // kFuGroupRow arcs are shared out too
-constexpr uint32_t kFuCache = 1024;         // per block: slots of classes it met that have two members
+constexpr uint32_t kFuCache = 512;         // per block: slots of classes it met that have two members
 // Shared memory is kept small on purpose: what it leaves is L1, whose lines
 // hold the gathers in flight (with 200 KB of check tables a pass of the
 // 131,072-node lift took 16.5 us, with 48 KB 13 us).
@@ -469,8 +471,11 @@ template <int MODE, bool WEIGHTED>
 __device__ __forceinline__ void fused_body(const FusedArgs& a)
 {
     __shared__ FuCache s_cache;
-    __shared__ unsigned long long s_val[kFuCheckSlots];
-    __shared__ uint32_t s_key[kFuCheckSlots];
+    // the passes' prefix sums (128 per warp); the check's table of one long row
+    __shared__ __align__(16) unsigned long long s_buf[kFuThreads / 32 * 128];
+    static_assert(sizeof s_buf >= kFuCheckSlots * 12, "values, then keys");
+    unsigned long long* const s_val = s_buf;
+    uint32_t* const s_key = reinterpret_cast<uint32_t*>(s_buf + kFuCheckSlots);
     __shared__ uint32_t s_sum, s_flag, s_word[2 + 16];
     __shared__ uint32_t s_delta[kFuThreads];  // per warp: its rows' (first arc - position) by rank
     const uint32_t n = a.n;
@@ -686,46 +691,63 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                     uint32_t* const delta = s_delta + (threadIdx.x & ~31u);
                     if (dd) delta[__popc(rows & ((1u << lane) - 1u))] = (uint32_t)b - start;
                     __syncwarp();
+                    ulonglong2* const pre = reinterpret_cast<ulonglong2*>(s_buf + (threadIdx.x >> 5) * 128);
                     uint64_t run = 0, at_start = 0;
                     uint32_t before = 0;  // rows that start before the step
-                    constexpr int U = 4;  // steps whose loads are in flight together
-                    for (uint32_t j0 = 0; j0 < total; j0 += 32u * U) {
-                        uint32_t cc[U], pos[U];
-                        uint64_t x[U];
+                    // a step: 128 arcs, four consecutive ones per lane
+                    for (uint32_t j0 = 0; j0 < total; j0 += 128) {
+                        // bit i of heads[w]: a row starts at position j0 + 32 w + i
+                        uint32_t heads[4], rank = before;
+                        const uint32_t rel = start - j0;
 #pragma unroll
-                        for (int q = 0; q < U; ++q) {
-                            const uint32_t j = j0 + 32u * q;
-                            // bit i: a row starts at position j + i
-                            const unsigned heads = __reduce_or_sync(0xffffffffu, dd && start - j < 32u ? 1u << (start - j) : 0u);
-                            const uint32_t rank = before + __popc(heads & (0xffffffffu >> (31 - lane)));
-                            before += __popc(heads);
-                            pos[q] = j + lane < total ? delta[rank - 1u] + j + lane : 0xffffffffu;
+                        for (int w = 0; w < 4; ++w)
+                            heads[w] = __reduce_or_sync(0xffffffffu, dd && rel - 32u * w < 32u ? 1u << (rel & 31u) : 0u);
+                        uint32_t mine = heads[0];
+#pragma unroll
+                        for (int w = 0; w < 4; ++w) {
+                            if (w < lane >> 3) {
+                                rank += __popc(heads[w]);
+                                mine = heads[w + 1 < 4 ? w + 1 : 3];
+                            }
+                            before += __popc(heads[w]);
+                        }
+                        uint32_t cc[4], pos[4];
+                        uint64_t x[4], t[4];
+#pragma unroll
+                        for (int q = 0; q < 4; ++q) {
+                            const uint32_t j = j0 + 4u * lane + q;
+                            const uint32_t r = rank + __popc(mine & (0xffffffffu >> (31 - ((lane & 7) * 4 + q))));
+                            pos[q] = j < total ? delta[r - 1u] + j : 0xffffffffu;
                         }
 #pragma unroll
-                        for (int q = 0; q < U; ++q) cc[q] = pos[q] != 0xffffffffu ? fu_ro<MODE>(idx + pos[q]) : 0u;
+                        for (int q = 0; q < 4; ++q) cc[q] = pos[q] != 0xffffffffu ? fu_ro<MODE>(idx + pos[q]) : 0u;
                         if (WEIGHTED) {
 #pragma unroll
-                            for (int q = 0; q < U; ++q)
+                            for (int q = 0; q < 4; ++q)
                                 x[q] = pos[q] != 0xffffffffu ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + pos[q]) : 0ull;
                         }
 #pragma unroll
-                        for (int q = 0; q < U; ++q) cc[q] = pos[q] != 0xffffffffu ? fu_cg<MODE>(co + cc[q]) : 0u;
+                        for (int q = 0; q < 4; ++q) cc[q] = pos[q] != 0xffffffffu ? fu_cg<MODE>(co + cc[q]) : 0u;
 #pragma unroll
-                        for (int q = 0; q < U; ++q) {
-                            uint64_t t = pos[q] != 0xffffffffu ? fu_term(cc[q], salt) : 0ull;
-                            if (WEIGHTED) t *= x[q];
-                            uint64_t in = t;
-#pragma unroll
-                            for (int o = 1; o < 32; o <<= 1) {
-                                const uint64_t y = __shfl_up_sync(0xffffffffu, in, o);
-                                if (lane >= o) in += y;
-                            }
-                            const uint64_t ex = run + in - t;
-                            const uint32_t rel = start - (j0 + 32u * q);
-                            const uint64_t v = __shfl_sync(0xffffffffu, ex, rel & 31u);
-                            if (dd && rel < 32u) at_start = v;
-                            run += __shfl_sync(0xffffffffu, in, 31);
+                        for (int q = 0; q < 4; ++q) {
+                            t[q] = pos[q] != 0xffffffffu ? fu_term(cc[q], salt) : 0ull;
+                            if (WEIGHTED) t[q] *= x[q];
                         }
+                        const uint64_t sum = t[0] + t[1] + t[2] + t[3];
+                        uint64_t in = sum;
+#pragma unroll
+                        for (int o = 1; o < 32; o <<= 1) {
+                            const uint64_t y = __shfl_up_sync(0xffffffffu, in, o);
+                            if (lane >= o) in += y;
+                        }
+                        // the sums before each position, for the rows that start there
+                        const uint64_t ex = run + in - sum;
+                        pre[2 * lane] = make_ulonglong2(ex, ex + t[0]);
+                        pre[2 * lane + 1] = make_ulonglong2(ex + t[0] + t[1], ex + t[0] + t[1] + t[2]);
+                        run += __shfl_sync(0xffffffffu, in, 31);
+                        __syncwarp();
+                        if (dd && rel < 128u) at_start = reinterpret_cast<const unsigned long long*>(pre)[rel];
+                        __syncwarp();
                     }
                     // a row ends where the next one starts
                     const unsigned above = lane == 31 ? 0u : rows & (0xffffffffu << (lane + 1));
