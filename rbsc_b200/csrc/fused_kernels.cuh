@@ -31,8 +31,8 @@
 // memory, so a step touches few lines, and no lane waits for a longer row);
 // a running prefix sum is read off at the row starts, and a row's sum is the
 // difference of two of them.  (One arc per lane and step took four times the
-// shuffles: the 131,072-node lift 101 us against 96, weighted R-MAT-20 699
-// against 650.)  Rows of more than kFuChunk arcs, and
+// shuffles: the 131,072-node lift 101 us against 96, a lift of 170 rounds 1102
+// against 1045.)  Rows of more than kFuChunk arcs, and
 // rows of more than kFuGroupRow arcs in a group of more than kFuGroupArcs (the
 // low node ids of an R-MAT graph are all hubs), are cut into chunks that all
 // warps share (the warp that completes a row's last chunk inserts it).
@@ -172,6 +172,13 @@ __device__ __forceinline__ uint64_t fu_term(uint32_t c, uint64_t salt)
     y *= 0xd6e8feb86659fd93ull;
     y ^= y >> 32;
     return y + (salt >> 32);
+}
+
+// The table fingerprint of (colour, signature): bit 0 clear, never 0.
+__device__ __forceinline__ uint64_t fu_fingerprint(uint32_t c, uint64_t s1, uint64_t seed)
+{
+    const uint64_t f = fmix64(s1 ^ (((uint64_t)c + 1ull) * kGolden ^ seed)) & ~1ull;
+    return f ? f : 2ull;
 }
 
 __device__ __forceinline__ uint64_t fu_warp_sum(uint64_t v, int width)
@@ -333,6 +340,90 @@ __device__ __forceinline__ int fu_take(unsigned& m, int lane)
         if (lane / G == q) src = b;
     }
     return src;
+}
+
+// The arc sums of a warp's 32 rows (lane: row [b, b + d) where act; see the top
+// of the file).  delta: 32 words, pre: 128 sums of shared memory of the warp.
+template <int MODE, bool WEIGHTED>
+__device__ __forceinline__ uint64_t fu_row_sums(bool act, uint64_t b, uint32_t d, const uint32_t* __restrict__ idx,
+                                                const uint64_t* __restrict__ wt, const uint32_t* __restrict__ co, uint64_t salt,
+                                                uint32_t* delta, ulonglong2* pre)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned rows = __ballot_sync(0xffffffffu, act && d > 0);
+    const uint32_t dd = act ? d : 0u;
+    uint32_t end = dd;  // inclusive prefix: where the row ends in the warp's sequence
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += x;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, end, 31), start = end - dd;
+    if (dd) delta[__popc(rows & ((1u << lane) - 1u))] = (uint32_t)b - start;
+    __syncwarp();
+    uint64_t run = 0, at_start = 0;
+    uint32_t before = 0;  // rows that start before the step
+    // a step: 128 arcs, four consecutive ones per lane
+    for (uint32_t j0 = 0; j0 < total; j0 += 128) {
+        // bit i of heads[w]: a row starts at position j0 + 32 w + i
+        uint32_t heads[4], rank = before;
+        const uint32_t rel = start - j0;
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+            heads[w] = __reduce_or_sync(0xffffffffu, dd && rel - 32u * w < 32u ? 1u << (rel & 31u) : 0u);
+        uint32_t mine = heads[0];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            if (w < lane >> 3) {
+                rank += __popc(heads[w]);
+                mine = heads[w + 1 < 4 ? w + 1 : 3];
+            }
+            before += __popc(heads[w]);
+        }
+        // (a lane's positions past the end read nothing and add nothing)
+        const uint32_t left = total - min(total, j0 + 4u * lane);
+        uint32_t cc[4];
+        uint64_t t[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t r = rank + __popc(mine & (0xffffffffu >> (31 - ((lane & 7) * 4 + q))));
+            cc[q] = q < left ? delta[r - 1u] + j0 + 4u * lane + q : 0u;
+        }
+        if (WEIGHTED) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                t[q] = q < left ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + cc[q]) : 0ull;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cc[q] = q < left ? fu_ro<MODE>(idx + cc[q]) : 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cc[q] = q < left ? fu_cg<MODE>(co + cc[q]) : 0u;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (WEIGHTED) t[q] *= fu_term(cc[q], salt);
+            else t[q] = q < left ? fu_term(cc[q], salt) : 0ull;
+        }
+        const uint64_t sum = t[0] + t[1] + t[2] + t[3];
+        uint64_t in = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint64_t y = __shfl_up_sync(0xffffffffu, in, o);
+            if (lane >= o) in += y;
+        }
+        // the sums before each position, for the rows that start there
+        const uint64_t ex = run + in - sum;
+        pre[2 * lane] = make_ulonglong2(ex, ex + t[0]);
+        pre[2 * lane + 1] = make_ulonglong2(ex + t[0] + t[1], ex + t[0] + t[1] + t[2]);
+        run += __shfl_sync(0xffffffffu, in, 31);
+        __syncwarp();
+        if (dd && rel < 128u) at_start = reinterpret_cast<const unsigned long long*>(pre)[rel];
+        __syncwarp();
+    }
+    // a row ends where the next one starts
+    const unsigned above = lane == 31 ? 0u : rows & (0xffffffffu << (lane + 1));
+    const uint64_t next = __shfl_sync(0xffffffffu, at_start, above ? __ffs(above) - 1 : 0);
+    __syncwarp();
+    return dd ? (above ? next : run) - at_start : 0ull;
 }
 
 // Exact comparison of two rows of at most G arcs by groups of G lanes: lane gl
@@ -642,10 +733,7 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
         const uint64_t t_one = fu_term(0u, salt);
         const uint64_t hmask = a.hash_bits == 0 ? ~0ull : a.hash_bits >= 64 ? 0ull : (1ull << a.hash_bits) - 1ull;
         made = 0;
-        auto fingerprint = [&](uint32_t c, uint64_t s1) -> uint64_t {
-            const uint64_t f = fmix64((s1 & hmask) ^ (((uint64_t)c + 1ull) * kGolden ^ a.seed)) & ~1ull;
-            return f ? f : 2ull;
-        };
+        auto fingerprint = [&](uint32_t c, uint64_t s1) { return fu_fingerprint(c, s1 & hmask, a.seed); };
         for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
             const uint32_t u = base + lane;
             const bool valid = u < n;
@@ -679,81 +767,8 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                     s1 = t_one * d;
                 } else {
                     if (fu_shared_row(d, __reduce_add_sync(0xffffffffu, d))) act = false;  // in chunks, below
-                    const unsigned rows = __ballot_sync(0xffffffffu, act && d > 0);
-                    const uint32_t dd = act ? d : 0u;
-                    uint32_t end = dd;  // inclusive prefix: where the row ends in the warp's sequence
-#pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
-                        if (lane >= o) end += x;
-                    }
-                    const uint32_t total = __shfl_sync(0xffffffffu, end, 31), start = end - dd;
-                    uint32_t* const delta = s_delta + (threadIdx.x & ~31u);
-                    if (dd) delta[__popc(rows & ((1u << lane) - 1u))] = (uint32_t)b - start;
-                    __syncwarp();
-                    ulonglong2* const pre = reinterpret_cast<ulonglong2*>(s_buf + (threadIdx.x >> 5) * 128);
-                    uint64_t run = 0, at_start = 0;
-                    uint32_t before = 0;  // rows that start before the step
-                    // a step: 128 arcs, four consecutive ones per lane
-                    for (uint32_t j0 = 0; j0 < total; j0 += 128) {
-                        // bit i of heads[w]: a row starts at position j0 + 32 w + i
-                        uint32_t heads[4], rank = before;
-                        const uint32_t rel = start - j0;
-#pragma unroll
-                        for (int w = 0; w < 4; ++w)
-                            heads[w] = __reduce_or_sync(0xffffffffu, dd && rel - 32u * w < 32u ? 1u << (rel & 31u) : 0u);
-                        uint32_t mine = heads[0];
-#pragma unroll
-                        for (int w = 0; w < 4; ++w) {
-                            if (w < lane >> 3) {
-                                rank += __popc(heads[w]);
-                                mine = heads[w + 1 < 4 ? w + 1 : 3];
-                            }
-                            before += __popc(heads[w]);
-                        }
-                        uint32_t cc[4], pos[4];
-                        uint64_t x[4], t[4];
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            const uint32_t j = j0 + 4u * lane + q;
-                            const uint32_t r = rank + __popc(mine & (0xffffffffu >> (31 - ((lane & 7) * 4 + q))));
-                            pos[q] = j < total ? delta[r - 1u] + j : 0xffffffffu;
-                        }
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) cc[q] = pos[q] != 0xffffffffu ? fu_ro<MODE>(idx + pos[q]) : 0u;
-                        if (WEIGHTED) {
-#pragma unroll
-                            for (int q = 0; q < 4; ++q)
-                                x[q] = pos[q] != 0xffffffffu ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + pos[q]) : 0ull;
-                        }
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) cc[q] = pos[q] != 0xffffffffu ? fu_cg<MODE>(co + cc[q]) : 0u;
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) {
-                            t[q] = pos[q] != 0xffffffffu ? fu_term(cc[q], salt) : 0ull;
-                            if (WEIGHTED) t[q] *= x[q];
-                        }
-                        const uint64_t sum = t[0] + t[1] + t[2] + t[3];
-                        uint64_t in = sum;
-#pragma unroll
-                        for (int o = 1; o < 32; o <<= 1) {
-                            const uint64_t y = __shfl_up_sync(0xffffffffu, in, o);
-                            if (lane >= o) in += y;
-                        }
-                        // the sums before each position, for the rows that start there
-                        const uint64_t ex = run + in - sum;
-                        pre[2 * lane] = make_ulonglong2(ex, ex + t[0]);
-                        pre[2 * lane + 1] = make_ulonglong2(ex + t[0] + t[1], ex + t[0] + t[1] + t[2]);
-                        run += __shfl_sync(0xffffffffu, in, 31);
-                        __syncwarp();
-                        if (dd && rel < 128u) at_start = reinterpret_cast<const unsigned long long*>(pre)[rel];
-                        __syncwarp();
-                    }
-                    // a row ends where the next one starts
-                    const unsigned above = lane == 31 ? 0u : rows & (0xffffffffu << (lane + 1));
-                    const uint64_t next = __shfl_sync(0xffffffffu, at_start, above ? __ffs(above) - 1 : 0);
-                    if (dd) s1 = (above ? next : run) - at_start;
-                    __syncwarp();
+                    s1 = fu_row_sums<MODE, WEIGHTED>(act, b, d, idx, wt, co, salt, s_delta + (threadIdx.x & ~31u),
+                                                     reinterpret_cast<ulonglong2*>(s_buf + (threadIdx.x >> 5) * 128));
                 }
                 if (act) fp = fingerprint(c, s1);
             }
