@@ -11,6 +11,7 @@
 #include "common.cuh"
 #include "fused_kernels.cuh"
 #include "deep_kernels.cuh"
+#include "list_kernels.cuh"
 #include "scan.cuh"
 #include "internal.h"
 
@@ -249,7 +250,9 @@ rbsc_status outcome(rbsc_ctx* ctx, rbsc_stats* stats, float ms, bool* handled)
 // launch-per-phase path catches up, first where it has more to offer (rival:
 // hot heads, or heads whose copy overlaps the first pass).  us a refinement,
 // one launch / launch per phase, uniform start: R-MAT-20 with 16 M arcs 487 /
-// 626, R-MAT-21 with 32 M 918 / 810; weighted (whose rows the launch-per-phase
+// 626, R-MAT-21 with 32 M 918 / 810 (with list_kernels.cuh after the first pass:
+// R-MAT-20 410, R-MAT-21 625, Erdos-Renyi with 16 M arcs 501 against 447, a lift
+// with 8.4 M 456 against 378); weighted (whose rows the launch-per-phase
 // check sorts) R-MAT-20 511 / 938 and R-MAT-21 947 / 1220 from degree colours,
 // R-MAT-22 with 65 M 1933 / 1852.
 constexpr uint64_t kSmallArcs = 1ull << 22, kLargeArcs = 3ull << 23, kLargeWeighted = 1ull << 25;
@@ -269,13 +272,141 @@ bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m, bool weighted, bo
     return ctx->shared_gpu || !ctx->opts.no_persist;
 }
 
+static rbsc_status ensure_work(rbsc_ctx* ctx, rbsc_graph* g, size_t bytes)
+{
+    if (g->fused_bytes >= bytes) return RBSC_OK;
+    dev_free(ctx, g->d_fused);
+    g->fused_bytes = 0;
+    EKS(dev_alloc(ctx, &g->d_fused, bytes));
+    g->fused_bytes = bytes;
+    return RBSC_OK;
+}
+
+// The working arrays of k_refine_rows behind its counters; K rows, n nodes.
+static FusedLayout list_layout(const rbsc_ctx* ctx, const rbsc_graph* g, size_t* seg = nullptr, uint32_t* seg_len = nullptr)
+{
+    FusedLayout l{};
+    size_t at = fused_al(sizeof(ListWords));
+    auto take = [&](size_t bytes) {
+        const size_t r = at;
+        at += fused_al(bytes);
+        return r;
+    };
+    l.log2tab = 10;
+    while ((1ull << l.log2tab) < 2ull * g->K) ++l.log2tab;
+    l.long_cap = (uint32_t)std::min<uint64_t>(g->K, g->m / (kFuGroupRow + 1)) + 1u;
+    l.chunk_cap = (uint32_t)(g->m / kFuChunk) + l.long_cap;
+    for (int i = 0; i < 3; ++i) l.tab[i] = take(8ull << l.log2tab);
+    l.minm = take(4ull << l.log2tab);
+    l.list = take(4ull * g->K);
+    l.lrow = take(4ull * l.long_cap);
+    l.lfirst = take(4ull * l.long_cap);
+    l.lsum = take(8ull * l.long_cap);
+    l.ldone = take(4ull * l.long_cap);
+    l.lchunk = take(4ull * l.chunk_cap);
+    const uint64_t warps = (uint64_t)ctx->sm_count * (kFuThreads / 32), len = (g->K + 32 * warps - 1) / (32 * warps) * 32;
+    const size_t sg = take(12ull * warps * len);
+    if (seg) *seg = sg;
+    if (seg_len) *seg_len = (uint32_t)len;
+    l.bytes = at;
+    return l;
+}
+
+// Graphs that fused_wanted leaves over, from 2^22 arcs: see the figures in
+// list_kernels.cuh.  Below, the launch-per-phase path is only taken with options
+// that this one does not know.
+bool list_wanted(const rbsc_ctx* ctx, const rbsc_graph* g)
+{
+    return default_knobs(ctx->opts) && (ctx->shared_gpu || !ctx->opts.no_persist) && ctx->opts.test_hash_bits == 0 && !g->weighted &&
+           !g->host_arcs && !g->list_off && g->K > 0 && g->m >= kSmallArcs && g->m < (1ull << 32) && g->n < kListMaxNodes &&
+           g->K <= (1u << 28);
+}
+
+bool list_reserve(rbsc_ctx* ctx, rbsc_graph* g) { return ensure_work(ctx, g, list_layout(ctx, g).bytes) == RBSC_OK; }
+
+rbsc_status list_clear(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s)
+{
+    const FusedLayout l = list_layout(ctx, g);
+    unsigned char* b = static_cast<unsigned char*>(g->d_fused);
+    EK(cudaMemsetAsync(b, 0, sizeof(ListWords), s));
+    for (int i = 1; i < 3; ++i) EK(cudaMemsetAsync(b + l.tab[i], 0, 8ull << l.log2tab, s));
+    return RBSC_OK;
+}
+
+rbsc_status list_arcless(rbsc_ctx* ctx, rbsc_graph* g, uint32_t* d_out)
+{
+    ++rbsc::launch_counter();
+    k_list_arcless<<<(unsigned)ctx->sm_count * 8, 256, 0, ctx->stream>>>(g->n, g->d_off, g->d_initlab, g->d_grep, d_out,
+                                                                        &static_cast<ListWords*>(g->d_fused)->arcless);
+    EK(cudaGetLastError());
+    return RBSC_OK;
+}
+
+rbsc_status list_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, uint32_t initial_blocks, rbsc_stats* stats,
+                        bool* handled)
+{
+    *handled = false;
+    cudaStream_t s = ctx->stream;
+    ListArgs x{};
+    size_t seg = 0;
+    const FusedLayout l = list_layout(ctx, g, &seg, &x.seg_len);
+    EKS(ensure_pinned(ctx));
+    fused_bind(x.f, l, static_cast<unsigned char*>(g->d_fused));
+    x.f.n = g->n;
+    x.f.m = g->m;
+    fused_csr(x.f, g->d_off, true);
+    x.f.idx = g->d_idx;
+    x.f.init = d_init;
+    x.f.out = d_out;
+    common_args(ctx, x.f);
+    x.K = g->K;
+    x.rows = g->d_rows;
+    x.seg = reinterpret_cast<uint2*>(static_cast<unsigned char*>(g->d_fused) + seg);
+    x.alone = reinterpret_cast<uint32_t*>(x.seg + (size_t)ctx->sm_count * (kFuThreads / 32) * x.seg_len);
+    x.sig = g->d_sig;
+    // a node without arcs keeps the words that the initial pass left in both
+    x.f.col[0] = g->d_initlab;
+    x.f.col[1] = g->d_col[0];
+    x.w = reinterpret_cast<ListWords*>(g->d_fused);
+    x.err = &g->d_st->error;
+    x.initial = initial_blocks;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = (unsigned)ctx->sm_count;
+    cfg.blockDim = kFuThreads;
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const FusedResult& r = *static_cast<const FusedResult*>(ctx->h_fused);
+    // other contexts' cooperative launches need not wait for this graph's copies
+    if (ctx->shared_gpu || g->oneshot) EK(cudaEventSynchronize(ctx->ev_sig[1]));
+    {
+        const std::unique_lock<std::mutex> lock = coop_lock(ctx->device);
+        ++rbsc::launch_counter();
+        EK(cudaLaunchKernelEx(&cfg, k_refine_rows, x));
+        EK(cudaEventRecord(ctx->ev[1], s));
+        EK(cudaStreamSynchronize(s));
+    }
+    if (r.status == kFuBadHead) {
+        // what the first pass found wrong: the caller reports the state's error bits
+        return RBSC_OK;
+    }
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+    EKS(outcome(ctx, stats, ms, handled));
+    if (!*handled) g->list_off = true;
+    return RBSC_OK;
+}
+
 rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled)
 {
     *handled = false;
     cudaStream_t s = ctx->stream;
     const uint64_t lc0 = rbsc::launch_counter();
     const FusedLayout l = fused_layout(g->n, g->m);
-    if (!g->d_fused) EKS(dev_alloc(ctx, &g->d_fused, l.bytes));
+    EKS(ensure_work(ctx, g, l.bytes));
     if (!d_out) {
         if (!g->d_out) EKS(dev_alloc(ctx, (void**)&g->d_out, 4 * (size_t)g->n));
         d_out = g->d_out;

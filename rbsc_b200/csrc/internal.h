@@ -76,9 +76,12 @@ struct rbsc_graph {
     float up_ms = 0.f;           // its host-to-device copies, timed by fused_refine
 
     void* d_fused = nullptr;     // working memory of the one-launch refinement
+    size_t fused_bytes = 0;
+    bool list_off = false;       // list_refine met a collision or a row too wide: launch per phase
 
     // refinement state (allocated on first refine, reused)
     bool bufs = false;
+    bool compact_bufs = false;  // and its node lists and arc sets
     uint32_t* d_col[1] = {nullptr};  // colours, updated in place
     uint32_t* d_initlab = nullptr;
     rbsc::Sig* d_sig = nullptr;  // per-node signature (16 B)
@@ -104,6 +107,7 @@ struct rbsc_graph {
     unsigned long long* d_tab8 = nullptr;    // 8-byte entries: the list passes (same entry count)
     uint32_t log2tab = 0;
     uint32_t next_stamp = 1;
+    bool stamp_wrapped = false;    // the table still holds entries of the stamp's last turn
     rbsc::RoundState* d_st = nullptr;
     rbsc::RoundState* h_st = nullptr;  // pinned mirror
     void* d_small = nullptr;           // 256 B of counters
@@ -262,6 +266,18 @@ std::unique_lock<std::mutex> coop_lock(int device);
 // does not apply after all, and the caller takes the launch-per-phase path.
 bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m, bool weighted, bool rival);
 rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled);
+// Whether the passes after a large refinement's first signatures run in one
+// launch (list_kernels.cuh); its working memory (false: there is none to be
+// had) and its clearing; the labels of the nodes without arcs, after their
+// groups; the launch after the first pass's signatures, which reports as
+// fused_refine does and leaves neither the initial labels nor col[0].
+bool list_wanted(const rbsc_ctx* ctx, const rbsc_graph* g);
+bool list_reserve(rbsc_ctx* ctx, rbsc_graph* g);
+rbsc_status list_clear(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s);
+rbsc_status list_arcless(rbsc_ctx* ctx, rbsc_graph* g, uint32_t* d_out);
+rbsc_status list_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, uint32_t initial_blocks, rbsc_stats* stats,
+                        bool* handled);
+
 // The same on rows that lie anywhere in the arc arrays (device memory, checked
 // by the caller): row u = arcs [begin[u], end[u]), m arcs in all.
 struct FusedRows {

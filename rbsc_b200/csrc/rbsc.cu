@@ -327,11 +327,12 @@ static void graph_release_refine(rbsc_graph* g)
     dev_free(g->ctx, (void*&)g->d_small);
     dev_free(g->ctx, g->d_tmp);
     dev_free(g->ctx, g->d_fused);
+    g->fused_bytes = 0;
     g->tmp_bytes = 0;
     g->key_cap = 0;
     host_free(g->ctx, (void*&)g->h_st);
     host_free(g->ctx, (void*&)g->h_as);
-    g->bufs = false;
+    g->bufs = g->compact_bufs = false;
     sortrelabel_release(g);
 }
 
@@ -790,6 +791,19 @@ static rbsc_status ensure_refine_bufs(rbsc_ctx* ctx, rbsc_graph* g)
     CKS(dev_alloc(ctx, (void**)&g->d_grep, 4 * n));
     CKS(dev_alloc(ctx, (void**)&g->d_gcnt, 4 * n));
     g->compact_arcs = g->m > 0;
+    CK(cudaMemsetAsync(g->d_sig, 0, sizeof(Sig) * n, ctx->stream));
+    CK(cudaMemsetAsync(g->d_tab, 0, sizeof(Entry) << g->log2tab, ctx->stream));
+    g->next_stamp = 1;
+    g->stamp_wrapped = false;
+    g->bufs = true;
+    return RBSC_OK;
+}
+
+// The node lists and compacted arc sets of the launch-per-phase passes.
+static rbsc_status ensure_compact_bufs(rbsc_ctx* ctx, rbsc_graph* g)
+{
+    if (g->compact_bufs) return RBSC_OK;
+    const size_t n = std::max<uint32_t>(g->n, 1);
     const size_t K = std::max<uint32_t>(g->K, 1);
     // compacted arc sets: as large as the graph's own (in device memory), or
     // the resident capacity of a streamed graph; k_compact_decide copies only
@@ -811,10 +825,7 @@ static rbsc_status ensure_refine_bufs(rbsc_ctx* ctx, rbsc_graph* g)
         CKS(dev_alloc(ctx, (void**)&g->cb.split[d], 4 * (ctiles + 1)));
         CKS(dev_alloc(ctx, (void**)&g->cb.chunk_row[d], 4 * (cpad / 16 + 1)));
     }
-    CK(cudaMemsetAsync(g->d_sig, 0, sizeof(Sig) * n, ctx->stream));
-    CK(cudaMemsetAsync(g->d_tab, 0, sizeof(Entry) << g->log2tab, ctx->stream));
-    g->next_stamp = 1;
-    g->bufs = true;
+    g->compact_bufs = true;
     return RBSC_OK;
 }
 
@@ -1112,29 +1123,9 @@ static rbsc_status finish_upload(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s)
     return RBSC_OK;
 }
 
-static rbsc_status launch_pass(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s, cudaGraphConditionalHandle h, int use_handle,
-                               PassTimer* t = nullptr, int first = kPassFull, uint32_t c0 = 0)
+// The signatures of one pass.
+static rbsc_status launch_signature(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s, int first, uint32_t c0)
 {
-    const uint32_t n = g->n;
-    const unsigned clear_grid = (unsigned)std::min<uint64_t>(ctx->sm_count * 8ull, grid_for(1ull << g->log2tab, 256));
-    const unsigned ngrid = persistent_grid(ctx, n, kNodeThreads);
-    const bool hash = ctx->opts.relabel != RBSC_RELABEL_SORT;
-    if (t) CK(cudaEventRecord(t->ev[0], s));
-    ++rbsc::launch_counter();
-    k_clear_table<<<clear_grid, 256, 0, s>>>(g->d_st, g->d_tab, 1ull << g->log2tab);
-    if (hash) {
-        // the list table's window, zeroed on the side stream beside the
-        // signature kernel (which neither reads nor writes the table); the
-        // inserts wait for it below
-        CK(cudaEventRecord(ctx->ev_fork, s));
-        CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-        ++rbsc::launch_counter();
-        k_clear_window8<<<clear_grid, 256, 0, ctx->side>>>(g->d_as, g->d_tab8, g->log2tab);
-        CK(cudaEventRecord(ctx->ev_join, ctx->side));
-    }
-    if (t) CK(cudaEventRecord(t->ev[1], s));
-    // the host-launched first pass is never captured: time its signature kernel
-    if (first != kPassFull) CK(cudaEventRecord(ctx->ev_sig[0], s));
     const bool streamed = (g->arcs_on_host || g->stream_upload) && g->m > 0 && first != kPassUniform;
     if (g->stream_upload && !streamed) CKS(finish_upload(ctx, g, s));
     if (streamed) {
@@ -1197,6 +1188,34 @@ static rbsc_status launch_pass(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s, cud
             k_signature_auto<false><<<blocks, kTileThreads, 0, s>>>(g->d_as, g->d_st, g->d_col[0], g->d_sig);
         }
     }
+    CK(cudaGetLastError());
+    return RBSC_OK;
+}
+
+static rbsc_status launch_pass(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s, cudaGraphConditionalHandle h, int use_handle,
+                               PassTimer* t = nullptr, int first = kPassFull, uint32_t c0 = 0)
+{
+    const uint32_t n = g->n;
+    const unsigned clear_grid = (unsigned)std::min<uint64_t>(ctx->sm_count * 8ull, grid_for(1ull << g->log2tab, 256));
+    const unsigned ngrid = persistent_grid(ctx, n, kNodeThreads);
+    const bool hash = ctx->opts.relabel != RBSC_RELABEL_SORT;
+    if (t) CK(cudaEventRecord(t->ev[0], s));
+    ++rbsc::launch_counter();
+    k_clear_table<<<clear_grid, 256, 0, s>>>(g->d_st, g->d_tab, 1ull << g->log2tab);
+    if (hash) {
+        // the list table's window, zeroed on the side stream beside the
+        // signature kernel (which neither reads nor writes the table); the
+        // inserts wait for it below
+        CK(cudaEventRecord(ctx->ev_fork, s));
+        CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
+        ++rbsc::launch_counter();
+        k_clear_window8<<<clear_grid, 256, 0, ctx->side>>>(g->d_as, g->d_tab8, g->log2tab);
+        CK(cudaEventRecord(ctx->ev_join, ctx->side));
+    }
+    if (t) CK(cudaEventRecord(t->ev[1], s));
+    // the host-launched first pass is never captured: time its signature kernel
+    if (first != kPassFull) CK(cudaEventRecord(ctx->ev_sig[0], s));
+    CKS(launch_signature(ctx, g, s, first, c0));
     if (t) CK(cudaEventRecord(t->ev[2], s));
     if (first != kPassFull) CK(cudaEventRecord(ctx->ev_sig[1], s));
     if (!hash) {
@@ -1503,7 +1522,8 @@ static rbsc_status clear_setup_words(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t 
 // follower pairs from the current colouring (after the initial or a repair
 // pass).  side_cleared: clear_setup_words ran on the side stream, which
 // recorded ev_join after it.
-static rbsc_status init_active_set(rbsc_ctx* ctx, rbsc_graph* g, bool side_cleared = false)
+// rows_only: no lists, k_refine_rows follows.
+static rbsc_status init_active_set(rbsc_ctx* ctx, rbsc_graph* g, bool side_cleared = false, bool rows_only = false)
 {
     cudaStream_t s = ctx->stream;
     const uint32_t n = g->n;
@@ -1533,6 +1553,10 @@ static rbsc_status init_active_set(rbsc_ctx* ctx, rbsc_graph* g, bool side_clear
     const unsigned lgrid = (unsigned)std::min<uint64_t>((uint64_t)ctx->sm_count * 8, ceil_div<uint64_t>(n, 256));
     ++rbsc::launch_counter();
     k_group_reps<<<lgrid, 256, 0, s>>>(n, g->d_off, g->d_initlab, g->d_grep, g->d_gcnt);
+    if (rows_only) {
+        CK(cudaGetLastError());
+        return RBSC_OK;
+    }
     ++rbsc::launch_counter();
     k_build_lists<<<lgrid, kNodeThreads, 0, s>>>(n, g->d_off, g->d_initlab, g->d_col[0], g->d_grep, g->d_gcnt, g->d_as,
                                                  g->cb.nodes[0], g->d_pairs);
@@ -1707,6 +1731,8 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
     }
     if (!g->prepared) CKS(graph_prepare(ctx, g));
     CKS(ensure_refine_bufs(ctx, g));
+    const bool rows_only = !kt && list_wanted(ctx, g) && list_reserve(ctx, g);
+    if (!rows_only) CKS(ensure_compact_bufs(ctx, g));
     g->first_sig_ms = 0.f;
     g->first_sig_arcs = 0;
     g->streamed_bytes = 0;
@@ -1716,7 +1742,8 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
     // (k_insert_init is bound by issue, not by HBM); the set-up waits for them
     CK(cudaEventRecord(ctx->ev_fork, s));
     CK(cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0));
-    CK(cudaMemsetAsync(g->d_joined, 0, 4 * (size_t)n, ctx->side));
+    if (rows_only) CKS(list_clear(ctx, g, ctx->side));
+    else CK(cudaMemsetAsync(g->d_joined, 0, 4 * (size_t)n, ctx->side));
     CKS(clear_setup_words(ctx, g, ctx->side));
     CK(cudaEventRecord(ctx->ev_join, ctx->side));
     RoundState& hs = *g->h_st;
@@ -1724,6 +1751,10 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
     hs.max_rounds = ctx->opts.max_rounds ? ctx->opts.max_rounds : (n + 1u);
     hs.seed = ctx->opts.seed;
     hs.hash_bits = ctx->opts.test_hash_bits < 0 ? 64u : (uint32_t)ctx->opts.test_hash_bits;
+    // a stamp that wrapped with the last refinement's last pass: no pass has
+    // cleared the table since
+    if (g->stamp_wrapped) CK(cudaMemsetAsync(g->d_tab, 0, sizeof(Entry) << g->log2tab, s));
+    g->stamp_wrapped = false;
     hs.stamp = g->next_stamp;
     hs.clear_pending = 0;
     CK(cudaEventRecord(ctx->ev[0], s));
@@ -1765,7 +1796,9 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         CK(cudaMemcpyAsync(g->h_st, g->d_st, sizeof(RoundState), cudaMemcpyDeviceToHost, s));
         CK(cudaEventRecord(ctx->ev[7], s));
     }
-    CKS(init_active_set(ctx, g, true));
+    uint32_t* const labels = d_out ? d_out : g->d_out;
+    CKS(init_active_set(ctx, g, true, rows_only));
+    if (rows_only) CKS(list_arcless(ctx, g, labels));
     if (kt) {
         CK(cudaEventRecord(ctx->ev[5], s));
         CK(cudaEventSynchronize(ctx->ev[5]));
@@ -1821,6 +1854,37 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         }
     }
 
+    if (rows_only && !hs.error) {
+        g->next_stamp = hs.stamp;
+        g->stamp_wrapped = hs.clear_pending != 0;
+        CK(cudaEventRecord(ctx->ev_sig[0], s));
+        CKS(launch_signature(ctx, g, s, first, c0));
+        CK(cudaEventRecord(ctx->ev_sig[1], s));
+        bool handled = false;
+        CKS(list_refine(ctx, g, d_init, labels, initial_blocks, stats, &handled));
+        if (handled) {
+            if (stats) {
+                float ms = 0.f, init_ms = 0.f;
+                cudaEventElapsedTime(&ms, ctx->ev_sig[0], ctx->ev_sig[1]);
+                cudaEventElapsedTime(&init_ms, ctx->ev[0], ctx->ev[6]);
+                stats->init_ms = init_ms;
+                stats->loop_ms += ms;
+                stats->first_signature_ms = first == kPassFull ? 0.0 : ms;
+                stats->first_signature_arcs = first == kPassUniform || first == kPassFull ? 0 : g->m;
+                stats->first_signature_hot = g->hot_active ? g->hot_n : 0u;
+                stats->streamed_bytes = g->streamed_bytes;
+                stats->streamed_passes = g->streamed_passes;
+                stats->kernel_launches = rbsc::launch_counter() - lc0;
+            }
+            return RBSC_OK;
+        }
+        CKS(read_state(ctx, g));
+        if (hs.error & kErrStage) return rbsc_fail(ctx, RBSC_ERR_DEVICE, "signature: a staged tile copy did not complete");
+        if (hs.error & kErrInput) return rbsc_fail(ctx, RBSC_ERR_INVALID, "an arc head is >= N");
+        // a collision or a row too wide: once more, launch by launch
+        return refine_resident(ctx, g, d_init, d_out, stats, kt);
+    }
+
     float verify_ms = 0.f, loop_ms = 0.f;
     uint32_t repairs = 0;
     uint32_t* out = d_out ? d_out : g->d_out;
@@ -1854,6 +1918,7 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         CKS(read_state(ctx, g));
     }
     g->next_stamp = hs.stamp;
+    g->stamp_wrapped = hs.clear_pending != 0;
     if (hs.error & kErrProbe) return rbsc_fail(ctx, RBSC_ERR_DEVICE, "relabel table overflow");
     if (hs.error & kErrStage) return rbsc_fail(ctx, RBSC_ERR_DEVICE, "signature: a staged tile copy did not complete");
     if (hs.error & kErrInput) return rbsc_fail(ctx, RBSC_ERR_INVALID, "an arc head is >= N");
