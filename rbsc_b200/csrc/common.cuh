@@ -237,4 +237,11 @@ inline uint64_t& launch_counter()
     return c;
 }
 
+// Whether a call's labels would overwrite initial colours that are still read.
+inline bool labels_over_init(const uint32_t* d_init, const uint32_t* d_out, size_t n)
+{
+    const uintptr_t i = reinterpret_cast<uintptr_t>(d_init), o = reinterpret_cast<uintptr_t>(d_out);
+    return i && o && i < o + 4 * n && o < i + 4 * n;
+}
+
 }  // namespace rbsc

@@ -407,7 +407,9 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
     const uint64_t lc0 = rbsc::launch_counter();
     const FusedLayout l = fused_layout(g->n, g->m);
     EKS(ensure_work(ctx, g, l.bytes));
-    if (!d_out) {
+    // labels may be asked for over the initial colours, which the check reads
+    uint32_t* const asked = d_out;
+    if (!d_out || labels_over_init(d_init, d_out, g->n)) {
         if (!g->d_out) EKS(dev_alloc(ctx, (void**)&g->d_out, 4 * (size_t)g->n));
         d_out = g->d_out;
     }
@@ -428,6 +430,10 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (!g->prepared) cudaEventElapsedTime(&g->up_ms, ctx->ev[2], ctx->ev[3]);
     EKS(outcome(ctx, stats, ms, handled));
+    if (*handled && asked && asked != d_out) {
+        EK(cudaMemcpyAsync(asked, d_out, 4 * (size_t)g->n, cudaMemcpyDeviceToDevice, s));
+        EK(cudaStreamSynchronize(s));
+    }
     if (stats && *handled) stats->kernel_launches = rbsc::launch_counter() - lc0;
     return RBSC_OK;
 }

@@ -45,7 +45,8 @@ constexpr uint32_t kNaMaxNodes = RBSC_NOALLOC_MAX_NODES;
 // and its barrier is a hardware one.  Eight blocks is the portable size.
 constexpr unsigned kNaBlocks = 8;
 constexpr size_t kNaWork = 2u << 20;  // fused_layout of the largest graph: 2,048,000 bytes
-constexpr size_t kNaBytes = kNaWork + (size_t)kNaBlocks * kFuWideSlots * 12;
+constexpr size_t kNaInit = kNaWork + (size_t)kNaBlocks * kFuWideSlots * 12;  // initial colours that the labels overwrite
+constexpr size_t kNaBytes = kNaInit + 4 * (size_t)kNaMaxNodes;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNaBytes];
 
@@ -124,6 +125,15 @@ extern "C" rbsc_status rbsc_refine_noalloc(const rbsc_csr* g, const uint32_t* d_
             return rbsc_fail(nullptr, RBSC_ERR_CUDA, "k_refine_block launch failed: %s", cudaGetErrorString(e));
         }
         return RBSC_OK;
+    }
+    if (labels_over_init(d_init_colors, d_out_labels, g->n)) {
+        // (one block has them in its shared memory)
+        e = cudaMemcpyAsync(scratch + kNaInit, d_init_colors, 4 * (size_t)g->n, cudaMemcpyDeviceToDevice, static_cast<cudaStream_t>(stream));
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            return rbsc_fail(nullptr, RBSC_ERR_CUDA, "copy of the initial colours failed: %s", cudaGetErrorString(e));
+        }
+        a.init = reinterpret_cast<const uint32_t*>(scratch + kNaInit);
     }
     cfg.gridDim = kNaBlocks;
     cfg.blockDim = kFuThreads;

@@ -1731,7 +1731,7 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
     }
     if (!g->prepared) CKS(graph_prepare(ctx, g));
     CKS(ensure_refine_bufs(ctx, g));
-    const bool rows_only = !kt && list_wanted(ctx, g) && list_reserve(ctx, g);
+    const bool rows_only = !kt && !labels_over_init(d_init, d_out, n) && list_wanted(ctx, g) && list_reserve(ctx, g);
     if (!rows_only) CKS(ensure_compact_bufs(ctx, g));
     g->first_sig_ms = 0.f;
     g->first_sig_arcs = 0;

@@ -259,3 +259,47 @@ def test_large_resident_graphs(m, weighted):
             assert np.array_equal(a.labels, b.labels) and a.verified == b.verified == 1
             if init is None:
                 assert (a.kernel_launches <= 2) == (len(idx) < (1 << 25 if weighted else 3 << 23))
+
+
+def _wide(k):
+    heads = np.arange(2, k + 2)
+    off, idx, _ = G.csr_from_arcs(k + 2, np.repeat([0, 1], k), np.tile(heads, 2))
+    return off, idx, np.concatenate([[0, 0], heads]).astype(np.uint32)
+
+
+@pytest.mark.parametrize("kind", ["block", "cluster", "grid", "deep", "wide", "large"])
+def test_labels_over_the_initial_colours(kind):
+    """The label array may be the array of the initial colours."""
+    import ctypes
+    import torch
+    from rbsc_b200 import _lib
+    if kind == "wide":
+        off, idx, init = _wide(20000)  # starts again launch by launch
+    else:
+        if kind == "deep":
+            off, idx = G.random_lift(300, 600, 6, seed=1)
+            s, d = G.arcs_of(off, idx)
+            n, k = len(off) - 1, np.arange(300)
+            off, idx, _ = G.csr_from_arcs(n + 301, np.concatenate([s, n + k]), np.concatenate([d, n + k + 1]))
+        else:
+            nodes, lift = dict(block=(40, 8), cluster=(600, 12), grid=(4000, 16), large=(20000, 32))[kind]
+            off, idx = G.random_lift(nodes, nodes * 7, lift, seed=1)
+        init = (np.arange(len(off) - 1) % 3).astype(np.uint32)
+        init[: len(init) // 2] = 5  # rows of one colour that stay together, of several that do not
+    n = len(off) - 1
+    ex = oracle.refine_exact(off, idx, None, init)
+    with R.Context(0) as ctx:
+        g = ctx.upload(off, idx)
+        buf = torch.from_numpy(init.view(np.int32)).cuda()
+        r = g.refine_device(buf.data_ptr(), buf.data_ptr())
+        assert r.blocks == ex.blocks and np.array_equal(buf.cpu().numpy().view(np.uint32), ex.labels)
+        g.free()
+    if n <= 16384 and len(idx) <= 1 << 16:
+        d = [torch.from_numpy(x).cuda() for x in (off.astype(np.int64), idx.view(np.int32), init.view(np.int32))]
+        res = torch.zeros(4, dtype=torch.int32, device="cuda")
+        c = _lib.Csr()
+        c.n, c.m, c.offsets, c.offset_bytes, c.indices, c.weights = n, len(idx), d[0].data_ptr(), 8, d[1].data_ptr(), None
+        torch.cuda.synchronize()
+        assert _lib.load().rbsc_refine_noalloc(ctypes.byref(c), d[2].data_ptr(), d[2].data_ptr(), res.data_ptr(), None, None) == 0
+        torch.cuda.synchronize()
+        assert res[3] == 0 and np.array_equal(d[2].cpu().numpy().view(np.uint32), ex.labels)
