@@ -336,7 +336,7 @@ rbsc_status list_clear(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s)
 rbsc_status list_arcless(rbsc_ctx* ctx, rbsc_graph* g, uint32_t* d_out)
 {
     ++rbsc::launch_counter();
-    k_list_arcless<<<(unsigned)ctx->sm_count * 8, 256, 0, ctx->stream>>>(g->n, g->d_off, g->d_initlab, g->d_grep, d_out,
+    k_list_arcless<<<(unsigned)ctx->sm_count * 8, 256, 0, ctx->stream>>>(g->n, g->d_bare, g->d_initlab, g->d_grep, d_out,
                                                                         &static_cast<ListWords*>(g->d_fused)->arcless);
     EK(cudaGetLastError());
     return RBSC_OK;

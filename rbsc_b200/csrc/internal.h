@@ -65,6 +65,7 @@ struct rbsc_graph {
     uint64_t* d_wt = nullptr;   // weights (padded) or null
     uint32_t K = 0;             // non-empty rows
     uint32_t* d_rows = nullptr;
+    uint32_t* d_bare = nullptr;  // a bit per node without arcs
     void* d_roff = nullptr;
     uint32_t ntiles = 0;
     uint32_t* d_tile_row = nullptr;

@@ -27,7 +27,7 @@
 // Bound by the random 32-byte sectors of the gathers and inserts: the passes
 // move about 3.5 TB/s of them.  R-MAT-24 from degree colours (263 M arcs), B200:
 // the kernel takes 1.37 ms (passes 190 / 440 / 265 / 147 / 120 us, labels and
-// check 195), a refinement 2.45 ms; launch by launch 3.15.  From degree colours,
+// check 195), a refinement 2.43 ms; launch by launch 3.15.  From degree colours,
 // one launch after the signatures / launch per phase, us: a lift of 4.2 M arcs
 // 340 / 519, of 8.4 M 501 / 743, Erdos-Renyi of 5 M 237 / 477, of 16 M 537 / 875;
 // R-MAT-21 from one class 625 / 820.  Walking all rows in every pass, without the
@@ -69,7 +69,9 @@ struct ListArgs {
 };
 
 // Labels of the nodes without arcs (final) and the number of their classes.
-static __global__ void __launch_bounds__(256) k_list_arcless(uint32_t n, const uint64_t* __restrict__ off,
+// `bare` has a bit per such node: with the offsets read here and in
+// k_group_reps instead, 16 bytes a node, R-MAT-24 took 2446 us against 2426.
+static __global__ void __launch_bounds__(256) k_list_arcless(uint32_t n, const uint32_t* __restrict__ bare,
                                                              const uint32_t* __restrict__ initlab, const uint32_t* __restrict__ grep,
                                                              uint32_t* __restrict__ out, uint32_t* __restrict__ count)
 {
@@ -83,7 +85,7 @@ static __global__ void __launch_bounds__(256) k_list_arcless(uint32_t n, const u
 #pragma unroll
         for (int j = 0; j < U; ++j) {
             const uint64_t u = (uint64_t)base + (uint64_t)j * stride;
-            none[j] = u < n && off[u + 1] == off[u];
+            none[j] = u < n && (bare[u >> 5] >> (u & 31u) & 1u);
         }
 #pragma unroll
         for (int j = 0; j < U; ++j) r[j] = none[j] ? initlab[base + j * stride] : 0u;

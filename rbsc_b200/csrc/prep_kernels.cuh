@@ -36,10 +36,15 @@ static __global__ void k_widen_offsets(uint64_t count, const OffIn* __restrict__
     if (i < count) out[i] = (uint64_t)in[i];
 }
 
-static __global__ void k_nonempty_flags(uint32_t n, const uint64_t* __restrict__ off, uint32_t* __restrict__ flag)
+// bare: a bit per node without arcs (whole warps).
+static __global__ void k_nonempty_flags(uint32_t n, const uint64_t* __restrict__ off, uint32_t* __restrict__ flag,
+                                        uint32_t* __restrict__ bare)
 {
     const uint32_t u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u < n) flag[u] = off[u + 1] > off[u] ? 1u : 0u;
+    const bool arcs = u < n && off[u + 1] > off[u];
+    if (u < n) flag[u] = arcs ? 1u : 0u;
+    const unsigned none = __ballot_sync(0xffffffffu, u < n && !arcs);
+    if ((threadIdx.x & 31) == 0 && u < n) bare[u >> 5] = none;
 }
 
 template <typename OffT>

@@ -365,6 +365,7 @@ extern "C" void rbsc_graph_free(rbsc_graph* g)
     dev_free(g->ctx, (void*&)g->d_idx);
     dev_free(g->ctx, (void*&)g->d_wt);
     dev_free(g->ctx, (void*&)g->d_rows);
+    dev_free(g->ctx, (void*&)g->d_bare);
     dev_free(g->ctx, g->d_roff);
     dev_free(g->ctx, (void*&)g->d_tile_row);
     dev_free(g->ctx, (void*&)g->d_split);
@@ -415,8 +416,9 @@ rbsc_status graph_prepare(rbsc_ctx* ctx, rbsc_graph* g)
     uint32_t* d_pos = nullptr;
     CKS(dev_alloc(ctx, (void**)&d_pos, sizeof(uint32_t) * ((size_t)n + 1)));
     struct Guard2 { rbsc_ctx* c; uint32_t*& p; ~Guard2() { dev_free(c, (void*&)p); } } guard2{ctx, d_pos};
+    CKS(dev_alloc(ctx, (void**)&g->d_bare, sizeof(uint32_t) * ((size_t)n / 32 + 1)));
     ++rbsc::launch_counter();
-    k_nonempty_flags<<<grid_for(n, 256), 256, 0, s>>>(n, g->d_off, d_pos);
+    k_nonempty_flags<<<grid_for(n, 256), 256, 0, s>>>(n, g->d_off, d_pos, g->d_bare);
     CK(cudaGetLastError());
     CK((exclusive_scan<uint32_t, uint32_t>(d_pos, d_pos, n, d_err + 1, g->d_tmp, s)));
     uint32_t K = 0;
@@ -1552,7 +1554,7 @@ static rbsc_status init_active_set(rbsc_ctx* ctx, rbsc_graph* g, bool side_clear
     else CKS(clear_setup_words(ctx, g, s));
     const unsigned lgrid = (unsigned)std::min<uint64_t>((uint64_t)ctx->sm_count * 8, ceil_div<uint64_t>(n, 256));
     ++rbsc::launch_counter();
-    k_group_reps<<<lgrid, 256, 0, s>>>(n, g->d_off, g->d_initlab, g->d_grep, g->d_gcnt);
+    k_group_reps<<<lgrid, 256, 0, s>>>(n, g->d_bare, g->d_initlab, g->d_grep, g->d_gcnt);
     if (rows_only) {
         CK(cudaGetLastError());
         return RBSC_OK;

@@ -1654,7 +1654,7 @@ static __global__ void k_compact_finalize(ActiveSet* as, RoundState* st, Compact
 // Node list and followers, built once per refinement after the initial pass.
 // ---------------------------------------------------------------------------
 
-// For every group of arc-less nodes with the same initial label: its smallest
+// For every group of arc-less nodes (bits of `bare`) with the same initial label: its smallest
 // node (grep) and whether it has more than one member (gcnt, saturating at 2).
 // Most such nodes share a handful of labels, so they are combined per warp
 // (__match_any_sync), then per block in a small shared-memory table, and
@@ -1662,7 +1662,7 @@ static __global__ void k_compact_finalize(ActiveSet* as, RoundState* st, Compact
 // once a label's minimum and count are settled, later blocks only read.
 constexpr int kRepSlots = 256;
 constexpr int kRepProbes = 32;
-static __global__ void __launch_bounds__(256) k_group_reps(uint32_t n, const uint64_t* __restrict__ off,
+static __global__ void __launch_bounds__(256) k_group_reps(uint32_t n, const uint32_t* __restrict__ bare,
                                                            const uint32_t* __restrict__ initlab,
                                                            uint32_t* __restrict__ grep, uint32_t* __restrict__ gcnt)
 {
@@ -1684,7 +1684,7 @@ static __global__ void __launch_bounds__(256) k_group_reps(uint32_t n, const uin
 #pragma unroll
         for (int j = 0; j < U; ++j) {
             const uint32_t u = base + j * blockDim.x + threadIdx.x;
-            dang[j] = u < n && off[u + 1] == off[u];
+            dang[j] = u < n && (bare[u >> 5] >> (u & 31u) & 1u);
         }
 #pragma unroll
         for (int j = 0; j < U; ++j) lab[j] = dang[j] ? initlab[base + j * blockDim.x + threadIdx.x] : 0u;
