@@ -250,9 +250,9 @@ rbsc_status outcome(rbsc_ctx* ctx, rbsc_stats* stats, float ms, bool* handled)
 // launch-per-phase path catches up, first where it has more to offer (rival:
 // hot heads, or heads whose copy overlaps the first pass).  us a refinement,
 // one launch / launch per phase, uniform start: R-MAT-20 with 16 M arcs 487 /
-// 626, R-MAT-21 with 32 M 918 / 810 (with list_kernels.cuh after the first pass:
-// R-MAT-20 410, R-MAT-21 625, Erdos-Renyi with 16 M arcs 501 against 447, a lift
-// with 8.4 M 456 against 378); weighted (whose rows the launch-per-phase
+// 626, R-MAT-21 with 32 M 918 / 810 (with list_kernels.cuh after the first pass,
+// before either dealt its groups out: R-MAT-20 410, R-MAT-21 625, Erdos-Renyi with
+// 16 M arcs 501 against 447, a lift with 8.4 M 456 against 378); weighted (whose rows the launch-per-phase
 // check sorts) R-MAT-20 511 / 938 and R-MAT-21 947 / 1220 from degree colours,
 // R-MAT-22 with 65 M 1933 / 1852.
 constexpr uint64_t kSmallArcs = 1ull << 22, kLargeArcs = 3ull << 23, kLargeWeighted = 1ull << 25;

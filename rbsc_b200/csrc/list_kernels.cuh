@@ -20,18 +20,21 @@
 // of its own: no atomics, and a late pass walks 1.7 M rows instead of 7.4 M.  A
 // pass first drops the rows that nobody joined, four loads in flight per lane
 // (their words are written to both arrays, the second time a pass later, when
-// nobody reads it), then folds and inserts the rest.  The tables' windows follow
+// nobody reads it); the rest is folded and inserted in groups of 32 that a
+// block's warps take as they become free.  The tables' windows follow
 // the rows in play (twice their number).  Rows too long for a warp are queued as
 // a pass meets them and shared out after a barrier.
 //
 // Bound by the random 32-byte sectors of the gathers and inserts: the passes
 // move about 3.5 TB/s of them.  R-MAT-24 from degree colours (263 M arcs), B200:
-// the kernel takes 1.37 ms (passes 190 / 440 / 265 / 147 / 120 us, labels and
-// check 195), a refinement 2.43 ms; launch by launch 3.15.  From degree colours,
+// the kernel takes 1.28 ms (passes 190 / 425 / 250 / 135 / 107 us, labels and
+// check 166), a refinement 2.33 ms; launch by launch 3.15.  From degree colours,
 // one launch after the signatures / launch per phase, us: a lift of 4.2 M arcs
-// 340 / 519, of 8.4 M 501 / 743, Erdos-Renyi of 5 M 237 / 477, of 16 M 537 / 875;
-// R-MAT-21 from one class 625 / 820.  Walking all rows in every pass, without the
-// warps' lists: 2.84 ms on R-MAT-24; lists that kept a row one pass longer: 2.62.
+// 338 / 519, of 8.4 M 472 / 743, Erdos-Renyi of 5 M 236 / 477, of 16 M 528 / 875;
+// R-MAT-21 from one class 589 / 820.  Walking all rows in every pass, without the
+// warps' lists: 2.84 ms on R-MAT-24; lists that kept a row one pass longer: 2.62;
+// each warp folding its own list only, without dealing a block's groups out (35 %
+// of the warps' time went into waiting at barriers): 2.43.
 //
 // Unit weights.  A check that fails (a hash collision) or meets a row with more
 // colours than its table holds ends the launch (kFuRowTooWide), and the
@@ -108,6 +111,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
     __shared__ __align__(16) unsigned long long s_buf[kFuThreads / 32 * 128];
     __shared__ uint32_t s_sum, s_act, s_flag, s_word[2];
     __shared__ uint32_t s_delta[kFuThreads];
+    __shared__ uint32_t s_cnt[kFuThreads / 32], s_next;
     const FusedArgs& a = x.f;
     const int lane = threadIdx.x & 31;
     const uint32_t gw = (threadIdx.x >> 5) * gridDim.x + blockIdx.x, nw = gridDim.x * (kFuThreads / 32);
@@ -151,6 +155,22 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
         ulonglong2* q = reinterpret_cast<ulonglong2*>(t);
         for (uint32_t i = gt; i < 1u << (lg - 1); i += nt) q[i] = make_ulonglong2(0ull, 0ull);
     };
+    // The block's lists as one sequence of groups of 32 rows, dealt out as warps
+    // become free: group t is group t / 32 of warp t % 32's list.
+    constexpr uint32_t kWarps = kFuThreads / 32;
+    auto share = [&]() -> uint32_t {
+        if (lane == 0) s_cnt[threadIdx.x >> 5] = cnt;
+        if (threadIdx.x == 0) s_next = 0u;
+        __syncthreads();
+        return (__reduce_max_sync(0xffffffffu, s_cnt[lane]) + 31u) / 32u * kWarps;
+    };
+    auto take = [&]() -> uint32_t {
+        uint32_t t = 0;
+        if (lane == 0) t = atomicAdd(&s_next, 1u);
+        return __shfl_sync(0xffffffffu, t, 0);
+    };
+    uint2* const segs = x.seg + (size_t)blockIdx.x * x.seg_len;
+    const size_t seg_warp = (size_t)gridDim.x * x.seg_len;  // from one warp's list to the block's next
     auto totals = [&](uint32_t made, uint32_t act) {
         made = __reduce_add_sync(0xffffffffu, made);
         act = __reduce_add_sync(0xffffffffu, act);
@@ -250,10 +270,13 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
             }
             cnt = kept;
             nalone = mk;
-            __syncwarp();
-            for (uint32_t i = 0; i < cnt; i += 32u) {
-                bool act = i + lane < cnt;
-                const uint2 q = act ? seg[i + lane] : make_uint2(0u, 0u);
+            const uint32_t groups = share();
+            for (uint32_t t = take(); t < groups; t = take()) {
+                const uint32_t i = t / kWarps * 32u, rest = s_cnt[t % kWarps];
+                if (i >= rest) continue;
+                uint2* const row = segs + (t % kWarps) * seg_warp + i + lane;
+                bool act = i + lane < rest;
+                const uint2 q = act ? *row : make_uint2(0u, 0u);
                 const uint32_t u = q.x, c = q.y;
                 uint64_t b = 0;
                 uint32_t d = 0;
@@ -281,7 +304,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
                     const uint32_t f = __shfl_sync(0xffffffffu, f0, 31) + end - nc;
                     if (queue) {
                         act = false;
-                        seg[i + lane].y = kQueued;
+                        row->y = kQueued;
                         if (j < a.long_cap) {
                             a.lrow[j] = u;
                             a.lfirst[j] = f;
@@ -297,7 +320,7 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
                 const uint32_t s = fu_insert_warp<MODE>(act, few, tc, lg, fp, s_cache, made);
                 if (act) {
                     cn[u] = kSlotBit | s;
-                    seg[i + lane].y = s;
+                    row->y = s;
                 }
             }
         }
@@ -399,9 +422,12 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
         return;
     }
     uint32_t nbad = 0;
-    for (uint32_t i = 0; i < cnt; i += 32u) {
-        const bool valid = i + lane < cnt;
-        const uint2 q = valid ? seg[i + lane] : make_uint2(0u, 0u);
+    const uint32_t groups = share();
+    for (uint32_t t = take(); t < groups; t = take()) {
+        const uint32_t i = t / kWarps * 32u, rest = s_cnt[t % kWarps];
+        if (i >= rest) continue;
+        const bool valid = i + lane < rest;
+        const uint2 q = valid ? segs[(t % kWarps) * seg_warp + i + lane] : make_uint2(0u, 0u);
         const uint32_t u = q.x;
         const uint32_t r = valid ? fu_cg<MODE>(a.minm + (q.y != kQueued ? q.y : fu_cg<MODE>(col + u) & ~kSlotBit)) : 0u;
         if (valid) a.out[u] = r;
