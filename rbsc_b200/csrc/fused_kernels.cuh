@@ -567,7 +567,7 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
     static_assert(sizeof s_buf >= kFuCheckSlots * 12, "values, then keys");
     unsigned long long* const s_val = s_buf;
     uint32_t* const s_key = reinterpret_cast<uint32_t*>(s_buf + kFuCheckSlots);
-    __shared__ uint32_t s_sum, s_flag, s_word[2 + 16];
+    __shared__ uint32_t s_sum, s_flag, s_next, s_word[2 + 16];
     __shared__ uint32_t s_delta[kFuThreads];  // per warp: its rows' (first arc - position) by rank
     const uint32_t n = a.n;
     const int lane = threadIdx.x & 31;
@@ -714,6 +714,17 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
         if (a.res && !a.start) a.res->round_blocks[0] = prev;
     }
 
+    // The next group of a block's warp: groups are dealt out as warps become free
+    // (the first ones are fixed), since rows differ in length.  Every nw-th group
+    // for each warp instead: weighted R-MAT-20 695 us against 640, R-MAT-20 480
+    // against 459, a lift of 8.4 M arcs 375 against 352.
+    auto next_group = [&](uint32_t base) -> uint32_t {
+        if constexpr (MODE != kFuGrid) return base + nw * 32u;
+        uint32_t t = 0;
+        if (lane == 0) t = atomicAdd(&s_next, 1u);
+        t = __shfl_sync(0xffffffffu, t, 0) + kFuThreads / 32;
+        return (t * gridDim.x + blockIdx.x) * 32u;
+    };
     // one pass from col[p & 1] to the other array; REPAIR: the key is (colour,
     // failed) instead of (colour, signature).  Returns false on a timeout.
     uint32_t round = a.round0, repairs = 0, count = 0;
@@ -723,7 +734,7 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
         const unsigned long long* __restrict__ tp = a.tab[p % 3u];
         unsigned long long* tc = a.tab[(p + 1u) % 3u];
         fu_cache_clear(s_cache);
-        if (threadIdx.x == 0) s_sum = 0u;
+        if (threadIdx.x == 0) s_sum = s_next = 0u;
         __syncthreads();
         clear_tab(a.tab[(p + 2u) % 3u]);
         if (repair) clear_min();
@@ -734,7 +745,7 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
         const uint64_t hmask = a.hash_bits == 0 ? ~0ull : a.hash_bits >= 64 ? 0ull : (1ull << a.hash_bits) - 1ull;
         made = 0;
         auto fingerprint = [&](uint32_t c, uint64_t s1) { return fu_fingerprint(c, s1 & hmask, a.seed); };
-        for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
+        for (uint32_t base = gw * 32u; base < n; base = next_group(base)) {
             const uint32_t u = base + lane;
             const bool valid = u < n;
             uint32_t c = valid ? fu_cg<MODE>(co + u) : kSingleton;
@@ -845,6 +856,7 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
         const uint32_t* __restrict__ col = a.col[p & 1u];
         const uint32_t par = repairs & 1u;
         if (first) w->nlist[par ^ 1u] = 0u;
+        if (threadIdx.x == 0) s_next = 0u;  // (the barrier below)
         for (uint32_t u = gt; u < n; u += nt) {
             const uint32_t c = fu_cg<MODE>(col + u);
             if (!(c & kSingleton) && fu_cg<MODE>(a.minm + c) > u) atomicMin(a.minm + c, u);
@@ -856,7 +868,7 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
         // labels, and the exact check of every node against that member
         const bool check = a.verify && status == kFuOk;
         uint32_t nbad = 0;
-        for (uint32_t base = gw * 32u; base < n; base += nw * 32u) {
+        for (uint32_t base = gw * 32u; base < n; base = next_group(base)) {
             const uint32_t u = base + lane;
             const bool valid = u < n;
             const uint32_t c = valid ? fu_cg<MODE>(col + u) : kSingleton;
