@@ -282,7 +282,10 @@ static rbsc_status ensure_work(rbsc_ctx* ctx, rbsc_graph* g, size_t bytes)
     return RBSC_OK;
 }
 
-// The working arrays of k_refine_rows behind its counters; K rows, n nodes.
+// The working arrays of k_refine_rows behind its counters.  Its second table and
+// the classes' smallest members lie in d_tab8 and d_srank, which the initial pass
+// is done with (sized by all nodes, so no smaller): the launch needs no more than
+// the arc sets and check keys of the launch-per-phase path, which a server counts.
 static FusedLayout list_layout(const rbsc_ctx* ctx, const rbsc_graph* g, size_t* seg = nullptr, uint32_t* seg_len = nullptr)
 {
     FusedLayout l{};
@@ -296,8 +299,8 @@ static FusedLayout list_layout(const rbsc_ctx* ctx, const rbsc_graph* g, size_t*
     while ((1ull << l.log2tab) < 2ull * g->K) ++l.log2tab;
     l.long_cap = (uint32_t)std::min<uint64_t>(g->K, g->m / (kFuGroupRow + 1)) + 1u;
     l.chunk_cap = (uint32_t)(g->m / kFuChunk) + l.long_cap;
-    for (int i = 0; i < 3; ++i) l.tab[i] = take(8ull << l.log2tab);
-    l.minm = take(4ull << l.log2tab);
+    l.tab[0] = take(8ull << l.log2tab);
+    l.tab[2] = take(8ull << l.log2tab);
     l.list = take(4ull * g->K);
     l.lrow = take(4ull * l.long_cap);
     l.lfirst = take(4ull * l.long_cap);
@@ -329,7 +332,8 @@ rbsc_status list_clear(rbsc_ctx* ctx, rbsc_graph* g, cudaStream_t s)
     const FusedLayout l = list_layout(ctx, g);
     unsigned char* b = static_cast<unsigned char*>(g->d_fused);
     EK(cudaMemsetAsync(b, 0, sizeof(ListWords), s));
-    for (int i = 1; i < 3; ++i) EK(cudaMemsetAsync(b + l.tab[i], 0, 8ull << l.log2tab, s));
+    EK(cudaMemsetAsync(g->d_tab8, 0, 8ull << l.log2tab, s));
+    EK(cudaMemsetAsync(b + l.tab[2], 0, 8ull << l.log2tab, s));
     return RBSC_OK;
 }
 
@@ -364,6 +368,8 @@ rbsc_status list_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, ui
     x.seg = reinterpret_cast<uint2*>(static_cast<unsigned char*>(g->d_fused) + seg);
     x.alone = reinterpret_cast<uint32_t*>(x.seg + (size_t)ctx->sm_count * (kFuThreads / 32) * x.seg_len);
     x.sig = g->d_sig;
+    x.f.tab[1] = g->d_tab8;
+    x.f.minm = g->d_srank;
     // a node without arcs keeps the words that the initial pass left in both
     x.f.col[0] = g->d_initlab;
     x.f.col[1] = g->d_col[0];
@@ -396,7 +402,11 @@ rbsc_status list_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, ui
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     EKS(outcome(ctx, stats, ms, handled));
-    if (!*handled) g->list_off = true;
+    if (!*handled) {
+        g->list_off = true;
+        dev_free(ctx, g->d_fused);  // room for the other path's arc sets
+        g->fused_bytes = 0;
+    }
     return RBSC_OK;
 }
 
