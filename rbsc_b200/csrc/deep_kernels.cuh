@@ -15,7 +15,8 @@
 // A pass groups the members of T whose sum differs from S[class] by (class,
 // sum).  A class that keeps a member outside keeps its id; of a class whose
 // members all moved, the largest group keeps it; the other groups are new
-// classes.  That is the partition a full pass gives: members outside T see
+// classes.  Ids are not used again: a class of s nodes that sheds one node a
+// pass, by a change of all others, uses s - 2 of them.  That is the partition a full pass gives: members outside T see
 // the same multiset of classes as before, and a node in T sees a class id
 // that no node outside T sees.  No new class: the fixpoint (the same pass
 // that a full pass would find unchanged).
@@ -38,7 +39,7 @@ namespace rbsc {
 constexpr uint32_t kIncCap = 2048;      // changed sums of a pass
 constexpr uint32_t kIncSlots = 4096;    // per table, at most half taken
 constexpr uint32_t kIncMark = 1u << 30; // colour word of k_inc_mark: the node changed class in the last full pass
-constexpr uint32_t kIncMaxNodes = 1u << 22;  // class ids (slots below 2^23, then new ones) stay below kIncMark
+constexpr uint32_t kIncMaxNodes = 1u << 22;  // class ids (slots below 2^23, then at most 2^22 new ones) stay below kIncMark
 constexpr uint64_t kIncNoSum = ~0ull;   // S of a class with no member outside T
 
 struct IncCounters {
@@ -144,7 +145,7 @@ static __global__ void k_inc_sums(FusedArgs a, const uint32_t* __restrict__ colm
 struct IncArgs {
     uint32_t* col;               // class ids, kSingleton | node for a class of one
     unsigned long long* sig;
-    unsigned long long* S;       // per class id
+    unsigned long long* S;       // per class id (end_id words)
     uint32_t* size;
     const uint32_t* tend;        // transpose: row ends (a row starts where the one before ends)
     const uint32_t* tsrc;
@@ -154,7 +155,7 @@ struct IncArgs {
     IncCounters* ctr;
     FusedResult* res;
     uint64_t salt;
-    uint32_t first_id;           // ids from here on are free
+    uint32_t first_id, end_id;   // ids from the one on are free, up to the other
     uint32_t round, blocks, max_rounds;
 };
 
@@ -201,6 +202,7 @@ static __global__ void __launch_bounds__(1024, 1) k_inc_passes(IncArgs a)
             over = 1;
             break;
         }
+        if (nt > a.end_id - s.nid) break;  // a pass takes at most an id per node of T
         ++stamp;
         lg = log2_slots(nt);
         const uint32_t slots = 1u << lg, mask = slots - 1u;

@@ -110,7 +110,9 @@ rbsc_status deep_tail(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
     const uint32_t n = a.n, passes = r.rounds - a.round0;
     uint32_t* col = a.col[passes & 1u];
     const uint32_t* old = a.col[(passes & 1u) ^ 1u];
-    const size_t slots = (size_t)1 << a.log2tab, ids = slots + n / 2 + 2;
+    // a new id is a new class, and there are at most n classes; room for the
+    // ids of one more pass keeps k_inc_passes' own bound from ever ending it
+    const size_t slots = (size_t)1 << a.log2tab, ids = slots + n + kIncCap;
     Scratch sc(ctx);
     // zeroed together: class sizes, in-degrees, T stamps, largest parts, counters
     const size_t z_size = 0, z_deg = z_size + 4 * ids, z_flag = z_deg + 4 * (size_t)n, z_ctr = z_flag + 4 * (size_t)n,
@@ -159,6 +161,7 @@ rbsc_status deep_tail(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
     t.res = &r;
     t.salt = salt;
     t.first_id = (uint32_t)slots;
+    t.end_id = (uint32_t)ids;
     t.round = r.rounds;
     t.blocks = r.blocks;
     t.max_rounds = a.max_rounds;
