@@ -16,8 +16,8 @@
 // published single-pass radix sort with decoupled look-back (Merrill and
 // Garland 2016, Adinets and Merrill 2022).  Tiles are taken by a ticket, so
 // every tile that a block waits for is running or done; the wait is bounded
-// all the same, and a block that gives up sets the sort's error word, which
-// ends the blocks after it.
+// all the same, and a block whose wait runs out counts the digits of the keys
+// that it did not wait for itself, so every pass ends with its output written.
 //
 // What bounds it: the latency of the ranking chain and the look-back, hidden
 // by four blocks per SM (16 M keys with 8-byte values: 182 us a digit, 2.9
@@ -42,15 +42,14 @@ constexpr int kRsIters = 16;                                  // keys per lane
 constexpr uint64_t kRsTile = (uint64_t)kRsThreads * kRsIters;  // 4096
 constexpr int kRsBins = 256;
 constexpr int kRsMaxDigits = 8;
-constexpr uint32_t kRsSpins = 1u << 22;  // polls of one predecessor: seconds
+constexpr uint32_t kRsSpins = 1u << 16;  // polls of one predecessor: tens of milliseconds
 
-// Temporary memory: digit counts, one ticket per digit and the error word,
-// then a look-back word per (tile, digit value).
+// Temporary memory: digit counts and one ticket per digit, then a look-back
+// word per (tile, digit value).
 struct RsTemp {
     uint32_t hist[kRsMaxDigits][kRsBins];
     uint32_t ticket[kRsMaxDigits];
-    uint32_t error;
-    uint32_t pad[55];
+    uint32_t pad[56];
 };
 static_assert(sizeof(RsTemp) % 256 == 0, "the look-back words follow it");
 
@@ -121,30 +120,31 @@ static __global__ void __launch_bounds__(kRsThreads, 4) k_rs_pass(const unsigned
                                                                   const V* __restrict__ vals_in,
                                                                   unsigned long long* __restrict__ keys_out, V* __restrict__ vals_out,
                                                                   uint64_t n, int digit, int shift, uint32_t mask,
-                                                                  RsTemp* __restrict__ t, unsigned long long* __restrict__ words)
+                                                                  RsTemp* __restrict__ t, unsigned long long* __restrict__ words,
+                                                                  uint32_t max_spins)
 {
     __shared__ uint32_t s_cnt[kRsWarps][kRsBins];
     __shared__ uint32_t s_start[kRsBins];  // tile-local start of each digit's run
     __shared__ uint32_t s_base[kRsBins];   // its place in the output, minus the start
+    __shared__ uint32_t s_left[kRsBins];   // tiles before this one whose counts it did not wait for
     __shared__ unsigned long long s_stage[kRsTile];
-    __shared__ uint32_t s_tile, s_fail, s_total;
+    __shared__ uint32_t s_tile, s_late, s_total;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         s_tile = atomicAdd(&t->ticket[digit], 1u);
-        s_fail = *(volatile uint32_t*)&t->error;
+        s_late = 0u;
     }
     for (int i = threadIdx.x; i < kRsWarps * kRsBins; i += kRsThreads) (&s_cnt[0][0])[i] = 0;
     __syncthreads();
-    if (s_fail) return;
     const uint32_t tile = s_tile;
     const uint64_t tbase = (uint64_t)tile * kRsTile;
     const uint32_t cnt = (uint32_t)(n - tbase < kRsTile ? n - tbase : kRsTile);
-    const uint64_t wbase = tbase + (uint64_t)warp * (kRsIters * 32);
+    const uint32_t at0 = (uint32_t)warp * (kRsIters * 32) + lane;  // the thread's first key in the tile
     unsigned long long key[kRsIters];
 #pragma unroll
     for (int it = 0; it < kRsIters; ++it) {
-        const uint64_t i = wbase + (uint64_t)it * 32 + lane;
-        key[it] = i < n ? __ldcs(keys_in + i) : 0ull;
+        const uint32_t i = at0 + it * 32;
+        key[it] = i < cnt ? __ldcs(keys_in + tbase + i) : 0ull;
     }
     // rank among the warp's equal digits, then tile-local position; two 16-bit
     // values per register
@@ -152,8 +152,7 @@ static __global__ void __launch_bounds__(kRsThreads, 4) k_rs_pass(const unsigned
     const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
     for (int it = 0; it < kRsIters; ++it) {
-        const uint64_t i = wbase + (uint64_t)it * 32 + lane;
-        const bool valid = i < n;
+        const bool valid = at0 + it * 32 < cnt;
         const uint32_t d = rs_digit(key[it], shift, mask);
         unsigned peers = __ballot_sync(0xffffffffu, valid);
 #pragma unroll
@@ -190,32 +189,36 @@ static __global__ void __launch_bounds__(kRsThreads, 4) k_rs_pass(const unsigned
         s_start[d] = start;
         if (tile != 0) {
             const uint32_t own = (uint32_t)(digit + 1);
-            uint32_t spins = 0;
-            for (uint32_t p = tile; p-- > 0;) {
-                unsigned long long w;
-                for (;;) {
-                    w = *(volatile unsigned long long*)(words + (size_t)p * kRsBins + d);
-                    if ((uint32_t)(w >> 34) == own) break;  // published in this digit's pass
-                    if (++spins > kRsSpins || ((spins & 1023u) == 0u && *(volatile uint32_t*)&t->error)) break;
-                }
-                if ((uint32_t)(w >> 34) != own) {  // gave up: nothing more is published or written
-                    atomicOr(&t->error, 1u);
-                    s_fail = 1u;
+            uint32_t spins = 0, p = tile;
+            while (p > 0) {
+                const unsigned long long w = *(volatile unsigned long long*)(words + (size_t)(p - 1u) * kRsBins + d);
+                if ((uint32_t)(w >> 34) == own) {  // published in this digit's pass
+                    prev += (uint32_t)w;
+                    spins = 0;
+                    --p;
+                    if ((uint32_t)(w >> 32) & 2u) p = 0;
+                } else if (++spins > max_spins) {
+                    s_late = 1u;
                     break;
                 }
-                prev += (uint32_t)w;
-                if ((uint32_t)(w >> 32) & 2u) break;
             }
-            if (!*(volatile uint32_t*)&s_fail) *mine = rs_word(digit, 2, prev + run);
+            s_left[d] = p;
+            if (p == 0) *mine = rs_word(digit, 2, prev + run);
         }
         s_base[d] = t->hist[digit][d] + prev - start;
     }
     __syncthreads();
-    if (s_fail) return;
+    if (s_late) {  // count them here (later tiles make do with this one's own count)
+        uint32_t c = 0;
+        const unsigned long long* k = keys_in;
+#pragma unroll 1
+        for (uint32_t j = s_left[threadIdx.x] * (uint32_t)kRsTile; j > 0; --j) c += rs_digit(*k++, shift, mask) == threadIdx.x ? 1u : 0u;
+        s_base[threadIdx.x] += c;
+        __syncthreads();
+    }
 #pragma unroll
     for (int it = 0; it < kRsIters; ++it) {
-        const uint64_t i = wbase + (uint64_t)it * 32 + lane;
-        if (i < n) {
+        if (at0 + it * 32 < cnt) {
             const uint32_t d = rs_digit(key[it], shift, mask);
             const uint32_t at = (pos2[it / 2] >> (16 * (it & 1)) & 0xffffu) + s_start[d] + s_cnt[warp][d];
             pos2[it / 2] = it & 1 ? (pos2[it / 2] & 0xffffu) | at << 16 : (pos2[it / 2] & 0xffff0000u) | at;
@@ -238,8 +241,8 @@ static __global__ void __launch_bounds__(kRsThreads, 4) k_rs_pass(const unsigned
         __syncthreads();
 #pragma unroll
         for (int it = 0; it < kRsIters; ++it) {
-            const uint64_t i = wbase + (uint64_t)it * 32 + lane;
-            if (i < n) s_val[pos2[it / 2] >> (16 * (it & 1)) & 0xffffu] = __ldcs(vals_in + i);
+            const uint32_t i = at0 + it * 32;
+            if (i < cnt) s_val[pos2[it / 2] >> (16 * (it & 1)) & 0xffffu] = __ldcs(vals_in + tbase + i);
         }
         __syncthreads();
 #pragma unroll
@@ -258,10 +261,10 @@ inline size_t radix_temp_bytes(uint64_t n)
 // Sorts keys[0..n) on bits [begin_bit, end_bit) (stable), carrying vals when
 // non-null.  Ping-pongs between (keys, vals) and (keys_alt, vals_alt); returns
 // true when the sorted result ended in the *_alt buffers.  n < 2^32.  Launches
-// only (capturable); temp holds radix_temp_bytes(n).
+// only (capturable); temp holds radix_temp_bytes(n).  max_spins: see kRsSpins.
 template <typename V>
 inline cudaError_t radix_sort(unsigned long long* keys, unsigned long long* keys_alt, V* vals, V* vals_alt, uint64_t n, int begin_bit, int end_bit,
-                              void* temp, cudaStream_t s, bool* in_alt)
+                              void* temp, cudaStream_t s, bool* in_alt, uint32_t max_spins = kRsSpins)
 {
     *in_alt = false;
     if (n <= 1 || end_bit <= begin_bit) return cudaSuccess;
@@ -280,8 +283,8 @@ inline cudaError_t radix_sort(unsigned long long* keys, unsigned long long* keys
         const int shift = begin_bit + 8 * d, bits = end_bit - shift < 8 ? end_bit - shift : 8;
         const uint32_t mask = (1u << bits) - 1u;
         ++rbsc::launch_counter();
-        if (vals) k_rs_pass<V, true><<<tiles, kRsThreads, 0, s>>>(ki, vi, ko, vo, n, d, shift, mask, t, words);
-        else k_rs_pass<V, false><<<tiles, kRsThreads, 0, s>>>(ki, vi, ko, vo, n, d, shift, mask, t, words);
+        if (vals) k_rs_pass<V, true><<<tiles, kRsThreads, 0, s>>>(ki, vi, ko, vo, n, d, shift, mask, t, words, max_spins);
+        else k_rs_pass<V, false><<<tiles, kRsThreads, 0, s>>>(ki, vi, ko, vo, n, d, shift, mask, t, words, max_spins);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         unsigned long long* tk = ki; ki = ko; ko = tk;
