@@ -291,7 +291,8 @@ rbsc_status refine_batch(rbsc_ctx* ctx, const Runs& rs, uint32_t n, uint32_t k0,
     ++rbsc::launch_counter();
     k_eb_mark_sources<<<grid_of(k1 - k0), 256, 0, s>>>(k0, k1, rs.rsrc, col);
     EK(cudaGetLastError());
-    if (fused_wanted(ctx, n, a1 - a0, rs.wt != nullptr, false)) {
+    const bool one_launch = fused_wanted(ctx, n, a1 - a0, rs.wt != nullptr, false);
+    if (one_launch) {
         // refined where the runs lie: no local copy of the arcs (0.26 ms per
         // batch of R-MAT-20 in quarters), no check and no tiling
         Scratch sc(ctx);
@@ -317,6 +318,7 @@ rbsc_status refine_batch(rbsc_ctx* ctx, const Runs& rs, uint32_t n, uint32_t k0,
     g->n = n;
     g->m = a1 - a0;
     g->oneshot = true;
+    g->launch_off = one_launch;  // (it gave up)
     EKS(graph_alloc_csr(ctx, g, rs.wt != nullptr));
     EK(cudaMemsetAsync(g->d_off, 0, 8 * ((size_t)n + 1), s));
     ++rbsc::launch_counter();

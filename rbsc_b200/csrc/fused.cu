@@ -4,6 +4,8 @@
 #include <algorithm>
 #include <chrono>
 #include <cstring>
+#include <new>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -12,6 +14,7 @@
 #include "fused_kernels.cuh"
 #include "deep_kernels.cuh"
 #include "list_kernels.cuh"
+#include "check_kernels.cuh"
 #include "scan.cuh"
 #include "internal.h"
 
@@ -193,8 +196,87 @@ rbsc_status launch_and_wait(rbsc_ctx* ctx, FusedArgs& a, const FusedLayout& l, b
     return RBSC_OK;
 }
 
+// Table slots of a batch of rows in check_rows (12 bytes each).
+constexpr uint64_t kCheckSlots = 1u << 23;
+
+// The rows that a launch's check left undecided (check_kernels.cuh), in batches
+// whose tables fit kCheckSlots, or one row; col: the final colours, nlist: the
+// check's list length on the device.  *equal: all of them are as their class's
+// smallest member is.  False too when the tables cannot be had or the rows are
+// read too often (one long member beside many short rows of the same sums):
+// the launch-per-phase check, which sorts each row once, decides then.
+rbsc_status check_rows(rbsc_ctx* ctx, const FusedArgs& a, const uint32_t* col, const uint32_t* nlist, cudaStream_t s, bool* equal)
+{
+    *equal = false;
+    uint32_t n = 0, count = 0;
+    EK(cudaMemcpyAsync(&n, nlist, 4, cudaMemcpyDeviceToHost, s));
+    EK(cudaStreamSynchronize(s));
+    Scratch sc(ctx);
+    uint32_t *words = nullptr, *keys = nullptr;  // words: rows, differences
+    unsigned long long* vals = nullptr;
+    CheckRow* rows = nullptr;
+    if (sc.get(&words, 2) != RBSC_OK || sc.get(&rows, n) != RBSC_OK) return RBSC_OK;
+    EK(cudaMemsetAsync(words, 0, 8, s));
+    const unsigned grid = (unsigned)ctx->sm_count * 8;
+    ++rbsc::launch_counter();
+    k_check_rows<<<grid, 256, 0, s>>>(a, n, col, rows, words);
+    EK(cudaGetLastError());
+    EK(cudaMemcpyAsync(&count, words, 4, cudaMemcpyDeviceToHost, s));
+    EK(cudaStreamSynchronize(s));
+    std::vector<CheckRow> h;
+    try {
+        h.resize(count);
+    } catch (const std::bad_alloc&) {
+        return RBSC_OK;
+    }
+    EK(cudaMemcpyAsync(h.data(), rows, sizeof(CheckRow) * count, cudaMemcpyDeviceToHost, s));
+    EK(cudaStreamSynchronize(s));
+    uint64_t arcs = 0, most = 0;
+    for (CheckRow& x : h) {
+        arcs += (uint64_t)x.du + x.dr;
+        // equal rows of unit weights have the member's colours; others may have
+        // colours whose weights add up to 0
+        const uint64_t colours = std::min<uint64_t>(a.wt ? (uint64_t)x.du + x.dr : x.dr, a.n);
+        uint64_t slots = 1024;
+        while (slots < 2 * colours) slots <<= 1;
+        x.mask = (uint32_t)(slots - 1);
+        most = std::max(most, slots);
+    }
+    if (arcs > 8 * a.m) return RBSC_OK;
+    const uint64_t cap = std::max(most, std::min<uint64_t>(kCheckSlots, 2 * a.m));
+    if (sc.get(&keys, cap) != RBSC_OK || sc.get(&vals, cap) != RBSC_OK) return RBSC_OK;
+    for (size_t i = 0; i < h.size();) {
+        uint64_t used = 0, pieces = 0;
+        size_t e = i;
+        for (; e < h.size(); ++e) {
+            CheckRow& x = h[e];
+            if (used + x.mask + 1 > cap) break;
+            x.base = used;
+            x.first = (uint32_t)pieces;
+            used += (uint64_t)x.mask + 1;
+            pieces += ((uint64_t)x.du + kCkChunk - 1) / kCkChunk + ((uint64_t)x.dr + kCkChunk - 1) / kCkChunk;
+        }
+        EK(cudaMemcpyAsync(rows + i, h.data() + i, sizeof(CheckRow) * (e - i), cudaMemcpyHostToDevice, s));
+        EK(cudaMemsetAsync(keys, 0xff, 4 * used, s));
+        EK(cudaMemsetAsync(vals, 0, 8 * used, s));
+        rbsc::launch_counter() += 2;
+        if (a.wt) k_check_count<true><<<grid, 256, 0, s>>>(a, col, rows + i, (uint32_t)(e - i), (uint32_t)pieces, keys, vals, words + 1);
+        else k_check_count<false><<<grid, 256, 0, s>>>(a, col, rows + i, (uint32_t)(e - i), (uint32_t)pieces, keys, vals, words + 1);
+        k_check_zero<<<grid, 256, 0, s>>>(used, vals, words + 1);
+        EK(cudaGetLastError());
+        i = e;
+    }
+    uint32_t bad = 0;
+    EK(cudaMemcpyAsync(&bad, words + 1, 4, cudaMemcpyDeviceToHost, s));
+    EK(cudaEventRecord(ctx->ev[1], s));
+    EK(cudaStreamSynchronize(s));
+    *equal = bad == 0;
+    return RBSC_OK;
+}
+
 // The launch, and where it stops early the work-list passes and a launch that
-// confirms them; waits for the stream.  ev[0] and ev[1] enclose it.
+// confirms them, and the rows that its check left; waits for the stream.  ev[0]
+// and ev[1] enclose it.
 rbsc_status run(rbsc_ctx* ctx, FusedArgs& a, const FusedLayout& l, cudaStream_t s)
 {
     FusedResult& r = *static_cast<FusedResult*>(ctx->h_fused);
@@ -213,16 +295,21 @@ rbsc_status run(rbsc_ctx* ctx, FusedArgs& a, const FusedLayout& l, cudaStream_t 
         r.t[0] = t0;
         r.t[1] = t1;
     }
+    if (r.status == kFuUndecided && !r.failed) {
+        bool equal = false;
+        EKS(check_rows(ctx, a, a.col[(r.rounds - a.round0 + r.repairs) & 1u], &a.w->nlist[r.repairs & 1u], s, &equal));
+        if (equal) r.status = kFuOk;
+    }
     return RBSC_OK;
 }
 
 // Status and statistics of a finished launch.  *handled false: the exact
-// check met a row with more colours than its table holds; the caller refines
-// the graph launch by launch.
+// check is not decided, or found a difference that the launch could not split
+// off; the caller refines the graph launch by launch.
 rbsc_status outcome(rbsc_ctx* ctx, rbsc_stats* stats, float ms, bool* handled)
 {
     const FusedResult& r = *static_cast<const FusedResult*>(ctx->h_fused);
-    *handled = r.status != kFuRowTooWide;
+    *handled = r.status != kFuUndecided;
     switch (r.status) {
         case kFuBadOffsets:
             return rbsc_fail(ctx, RBSC_ERR_INVALID, "offsets are not a valid CSR (must start at 0, be non-decreasing and end at M)");
@@ -285,6 +372,14 @@ static rbsc_status ensure_work(rbsc_ctx* ctx, rbsc_graph* g, size_t bytes)
     return RBSC_OK;
 }
 
+// From here on launch by launch; makes room for that path's arc sets.
+static void launch_gave_up(rbsc_ctx* ctx, rbsc_graph* g)
+{
+    g->launch_off = true;
+    dev_free(ctx, g->d_fused);
+    g->fused_bytes = 0;
+}
+
 // The working arrays of k_refine_rows behind its counters.  Its second table and
 // the classes' smallest members lie in d_tab8 and d_srank, which the initial pass
 // is done with (sized by all nodes, so no smaller): the launch needs no more than
@@ -324,7 +419,7 @@ static FusedLayout list_layout(const rbsc_ctx* ctx, const rbsc_graph* g, size_t*
 bool list_wanted(const rbsc_ctx* ctx, const rbsc_graph* g)
 {
     return default_knobs(ctx->opts) && (ctx->shared_gpu || !ctx->opts.no_persist) && ctx->opts.test_hash_bits == 0 && !g->weighted &&
-           !g->host_arcs && !g->list_off && g->K > 0 && g->m >= kSmallArcs && g->m < (1ull << 32) && g->n < kListMaxNodes &&
+           !g->host_arcs && !g->launch_off && g->K > 0 && g->m >= kSmallArcs && g->m < (1ull << 32) && g->n < kListMaxNodes &&
            g->K <= (1u << 28);
 }
 
@@ -388,7 +483,7 @@ rbsc_status list_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, ui
     at.val.cooperative = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    const FusedResult& r = *static_cast<const FusedResult*>(ctx->h_fused);
+    FusedResult& r = *static_cast<FusedResult*>(ctx->h_fused);
     // other contexts' cooperative launches need not wait for this graph's copies
     if (ctx->shared_gpu || g->oneshot) EK(cudaEventSynchronize(ctx->ev_sig[1]));
     {
@@ -402,14 +497,15 @@ rbsc_status list_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, ui
         // what the first pass found wrong: the caller reports the state's error bits
         return RBSC_OK;
     }
+    if (r.status == kFuUndecided && !r.failed) {
+        bool equal = false;
+        EKS(check_rows(ctx, x.f, x.f.col[r.rounds & 1u], &x.w->f.nlist[0], s, &equal));
+        if (equal) r.status = kFuOk;
+    }
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     EKS(outcome(ctx, stats, ms, handled));
-    if (!*handled) {
-        g->list_off = true;
-        dev_free(ctx, g->d_fused);  // room for the other path's arc sets
-        g->fused_bytes = 0;
-    }
+    if (!*handled) launch_gave_up(ctx, g);
     return RBSC_OK;
 }
 
@@ -443,6 +539,7 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (!g->prepared) cudaEventElapsedTime(&g->up_ms, ctx->ev[2], ctx->ev[3]);
     EKS(outcome(ctx, stats, ms, handled));
+    if (!*handled) launch_gave_up(ctx, g);
     if (*handled && asked && asked != d_out) {
         EK(cudaMemcpyAsync(asked, d_out, 4 * (size_t)g->n, cudaMemcpyDeviceToDevice, s));
         EK(cudaStreamSynchronize(s));
@@ -481,9 +578,10 @@ rbsc_status fused_refine_rows(rbsc_ctx* ctx, const FusedRows& r, const uint32_t*
 // A small host graph, labels back in host memory: the arrays are gathered in a
 // pinned buffer, go to the device in one copy, and the kernel writes the
 // labels and counts into pinned memory.
-rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled)
+rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled,
+                          bool* gave_up)
 {
-    *handled = false;
+    *handled = *gave_up = false;
     const uint64_t lc0 = rbsc::launch_counter();
     if (c->m > kStageBytes / 4 || c->n > kStageNodes) return RBSC_OK;  // before the sizes below are added up
     const uint32_t n = c->n;
@@ -535,6 +633,7 @@ rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init
     cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
     if (stats) std::memset(stats, 0, sizeof *stats);
     EKS(outcome(ctx, stats, ms, handled));
+    *gave_up = !*handled;
     if (!*handled) return RBSC_OK;
     if (out) std::memcpy(out, h_out, 4 * (size_t)n);
     if (stats) {

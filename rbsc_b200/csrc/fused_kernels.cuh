@@ -68,9 +68,12 @@ constexpr uint32_t kFuWarpSlots = kFuCheckSlots / (kFuThreads / 32);
 constexpr uint32_t kFuWarpRow = kFuWarpSlots - 8;  // rows up to this length are tried by one warp
 constexpr uint32_t kFuWideSlots = 32768;    // per block, in global memory: any row of a graph of at most 16384 nodes
 
+constexpr uint32_t kFuProbes = 256;  // of the shared table: one that takes longer is as good as full
+
 // outcome of a launch (FusedResult.status)
-// kFuRowTooWide: the launcher takes the launch-per-phase path
-constexpr int kFuOk = 0, kFuBadOffsets = 1, kFuBadHead = 2, kFuNotConverged = 3, kFuRowTooWide = 4, kFuBarrier = 5,
+// kFuUndecided: labels are written, but the exact check left rows to check_kernels.cuh (marked with
+// kSingleton in the list) or, with `failed`, found a node that differs and could not split it off
+constexpr int kFuOk = 0, kFuBadOffsets = 1, kFuBadHead = 2, kFuNotConverged = 3, kFuUndecided = 4, kFuBarrier = 5,
               kFuDeep = 6;  // stopped after deep_round passes or more: the last ones changed little (deep_kernels.cuh)
 
 // Counters of one launch, zero at its start (zeroed by the launcher, or by
@@ -79,7 +82,7 @@ struct FusedWords {
     unsigned long long bar[2];  // barrier words (fu_barrier)
     uint32_t pad[28];
     uint32_t bad;          // 1 = offsets, 2 = a head
-    uint32_t overflow;     // a long row had more colours than the check's table
+    uint32_t overflow;     // a row had more colours than the check's table: marked in the list
     uint32_t nlong, nchunk;
     uint32_t nlist[2];     // long rows of the running check (by repair parity)
 };
@@ -87,7 +90,7 @@ struct FusedWords {
 struct FusedResult {
     uint32_t rounds, blocks, initial_blocks, repairs;
     int32_t status;
-    uint32_t pad;
+    uint32_t failed;       // kFuUndecided: another node failed the check
     uint64_t t[4];         // globaltimer: start, initial colours done, fixpoint, end
     uint32_t round_blocks[kRoundLog];
 };
@@ -109,7 +112,7 @@ struct FusedArgs {
     uint32_t* list;        // nodes whose check needs a shared table
     uint8_t* fail;
     unsigned char* wide;   // kFuWideSlots counters per block for rows with more colours than the
-                           // shared table holds; null: such a row ends the launch (kFuRowTooWide)
+                           // shared table holds; null: such a row is left undecided (kFuUndecided)
     uint32_t* lrow;        // long rows: node, first chunk, running sum, chunks done
     uint32_t* lfirst;
     unsigned long long* lsum;
@@ -544,11 +547,12 @@ __device__ __forceinline__ void fu_check_long(unsigned m, int lane, const uint32
     }
 }
 
-// Adds sign * weight to colour c in an open-addressed table; false when full.
-__device__ __forceinline__ bool fu_count(uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t c, uint64_t w)
+// Adds sign * weight to colour c in an open-addressed table; false when it
+// finds no place in so many probes.
+__device__ __forceinline__ bool fu_count(uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t probes, uint32_t c, uint64_t w)
 {
     uint32_t h = (c * 0x9e3779b1u) >> 7 & mask;
-    for (uint32_t p = 0; p <= mask; ++p, h = (h + 1u) & mask) {
+    for (uint32_t p = 0; p < probes; ++p, h = (h + 1u) & mask) {
         const uint32_t k = atomicCAS(&key[h], 0xffffffffu, c);
         if (k == 0xffffffffu || k == c) {
             atomicAdd(&val[h], (unsigned long long)w);
@@ -927,15 +931,15 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
             // ones (weighted) in its part of the block's table and leaves them
             // to the block when they do not fit.
             nbad = 0;
-            auto add_row = [&](uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t x, bool minus, uint32_t at,
+            // (false: the table is full, and what it holds is of no use)
+            auto add_row = [&](uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t probes, uint32_t x, bool minus, uint32_t at,
                                uint32_t step) -> bool {
-                bool ok = true;
                 const uint64_t b = fu_off<MODE>(a, x), e = fu_end<MODE>(a, x);
                 for (uint64_t i = b + at; i < e; i += step) {
                     const uint64_t v = WEIGHTED ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + i) : 1ull;
-                    ok &= fu_count(key, val, mask, fu_cg<MODE>(col + fu_ro<MODE>(idx + i)), minus ? 0ull - v : v);
+                    if (!fu_count(key, val, mask, probes, fu_cg<MODE>(col + fu_ro<MODE>(idx + i)), minus ? 0ull - v : v)) return false;
                 }
-                return ok;
+                return true;
             };
             auto longest = [&](uint32_t u, uint32_t r) {
                 return max((uint32_t)(fu_end<MODE>(a, u) - fu_off<MODE>(a, u)), (uint32_t)(fu_end<MODE>(a, r) - fu_off<MODE>(a, r)));
@@ -952,8 +956,8 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                         val[k] = 0ull;
                     }
                     __syncwarp();
-                    bool ok = add_row(key, val, kFuWarpSlots - 1u, r, false, lane, 32);
-                    ok &= add_row(key, val, kFuWarpSlots - 1u, u, true, lane, 32);
+                    bool ok = add_row(key, val, kFuWarpSlots - 1u, kFuWarpSlots, r, false, lane, 32);
+                    ok = ok && add_row(key, val, kFuWarpSlots - 1u, kFuWarpSlots, u, true, lane, 32);
                     __syncwarp();
                     bool diff = false;
                     for (uint32_t k = lane; k < kFuWarpSlots; k += 32) diff |= val[k] != 0ull;
@@ -979,7 +983,8 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                 if (WEIGHTED && longest(u, r) <= kFuWarpRow && fu_cg<MODE>(a.fail + u) != 2) continue;
                 uint32_t* key = s_key;
                 unsigned long long* val = s_val;
-                uint32_t slots = kFuCheckSlots;
+                // (a graph in shared memory has fewer nodes than the table half its slots)
+                uint32_t slots = kFuCheckSlots, probes = MODE == kFuBlock ? kFuCheckSlots : kFuProbes;
                 for (;;) {
                     for (uint32_t k = threadIdx.x; k < slots; k += kFuThreads) {
                         key[k] = 0xffffffffu;
@@ -987,8 +992,8 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                     }
                     if (threadIdx.x == 0) s_flag = 0u;
                     __syncthreads();
-                    bool ok = add_row(key, val, slots - 1u, r, false, threadIdx.x, kFuThreads);
-                    ok &= add_row(key, val, slots - 1u, u, true, threadIdx.x, kFuThreads);
+                    bool ok = add_row(key, val, slots - 1u, probes, r, false, threadIdx.x, kFuThreads);
+                    ok = ok && add_row(key, val, slots - 1u, probes, u, true, threadIdx.x, kFuThreads);
                     if (!ok) atomicOr(&s_flag, 2u);
                     __syncthreads();
                     bool diff = false;
@@ -1001,13 +1006,17 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                         // more colours than the shared table holds: once more in global memory
                         val = reinterpret_cast<unsigned long long*>(a.wide + (size_t)blockIdx.x * kFuWideSlots * 12);
                         key = reinterpret_cast<uint32_t*>(val + kFuWideSlots);
-                        slots = kFuWideSlots;
+                        slots = probes = kFuWideSlots;
                         continue;
                     }
                     if (threadIdx.x == 0) {
-                        if (f & 2u) atomicOr(&w->overflow, 1u);
-                        a.fail[u] = (f & 1u) ? 1 : 0;
-                        nbad += f & 1u;
+                        if (f & 2u) {
+                            atomicOr(&w->overflow, 1u);
+                            a.list[i] = u | kSingleton;
+                        } else {
+                            a.fail[u] = (f & 1u) ? 1 : 0;
+                            nbad += f & 1u;
+                        }
                     }
                     break;
                 }
@@ -1020,7 +1029,8 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                 return;
             }
             if (fu_cg<MODE>(&w->overflow)) {
-                finish(kFuRowTooWide, round, prev, initial, repairs);
+                if (first && a.res) a.res->failed = nfail + more;
+                finish(kFuUndecided, round, prev, initial, repairs);
                 return;
             }
         }

@@ -78,7 +78,7 @@ struct rbsc_graph {
 
     void* d_fused = nullptr;     // working memory of the one-launch refinement
     size_t fused_bytes = 0;
-    bool list_off = false;       // list_refine met a collision or a row too wide: launch per phase
+    bool launch_off = false;     // a one-launch refinement gave up on it (fused.cu): launch per phase
 
     // refinement state (allocated on first refine, reused)
     bool bufs = false;
@@ -202,9 +202,9 @@ rbsc_status ensure_temp(rbsc_ctx* ctx, rbsc_graph* g, size_t bytes);
 rbsc_status graph_prepare(rbsc_ctx* ctx, rbsc_graph* g);
 // The graph of a one-shot call: not checked or tiled where fused_wanted takes
 // it (refine_resident prepares it if it has to); a large unweighted one's heads
-// arrive during the first pass.
+// arrive during the first pass.  launch_off: as the graph's.
 rbsc_status graph_upload_oneshot(rbsc_ctx* ctx, const rbsc_csr* host_graph, const uint32_t* init_colors, rbsc_graph** out, double* h2d_ms,
-                                 uint64_t* h2d_bytes);
+                                 uint64_t* h2d_bytes, bool launch_off = false);
 rbsc_status graph_alloc_csr(rbsc_ctx* ctx, rbsc_graph* g, bool weighted);
 rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats,
                             rbsc_kernel_times* kt);
@@ -264,7 +264,8 @@ std::unique_lock<std::mutex> coop_lock(int device);
 // The one-launch refinement (fused.cu).  fused_wanted: the context's options
 // and the sizes allow it; rival: a large graph would get hot heads or an
 // overlapped upload on the launch-per-phase path.  *handled false on RBSC_OK: it
-// does not apply after all, and the caller takes the launch-per-phase path.
+// does not apply, or (gave_up, and the graph's launch_off) its exact check was
+// not decided: the caller takes the launch-per-phase path.
 bool fused_wanted(const rbsc_ctx* ctx, uint32_t n, uint64_t m, bool weighted, bool rival);
 rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled);
 // Whether the passes after a large refinement's first signatures run in one
@@ -290,7 +291,8 @@ struct FusedRows {
     const uint64_t* wt;
 };
 rbsc_status fused_refine_rows(rbsc_ctx* ctx, const FusedRows& r, const uint32_t* d_init, uint32_t* d_out, rbsc_stats* stats, bool* handled);
-rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled);
+rbsc_status fused_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init, uint32_t* out, rbsc_stats* stats, bool* handled,
+                          bool* gave_up);
 
 // sort-based relabel (sortrelabel.cu)
 rbsc_status ensure_sort_relabel_bufs(rbsc_ctx* ctx, rbsc_graph* g);

@@ -36,8 +36,8 @@
 // each warp folding its own list only, without dealing a block's groups out (35 %
 // of the warps' time went into waiting at barriers): 2.43.
 //
-// Unit weights.  A check that fails (a hash collision) or meets a row with more
-// colours than its table holds ends the launch (kFuRowTooWide), and the
+// Unit weights.  Rows with more colours than the check's table holds are left to
+// check_kernels.cuh.  When a node fails the check (a hash collision), the
 // refinement is done again launch by launch.
 #pragma once
 #include <cstdint>
@@ -484,11 +484,11 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
             if (threadIdx.x == 0) s_flag = 0u;
             __syncthreads();
             bool ok = true;
-            for (int side = 0; side < 2; ++side) {
+            for (int side = 0; side < 2 && ok; ++side) {
                 const uint32_t v = side ? u : r;
                 const uint64_t e = fu_end<MODE>(a, v);
-                for (uint64_t q = fu_off<MODE>(a, v) + threadIdx.x; q < e; q += kFuThreads)
-                    ok &= fu_count(key, val, kFuCheckSlots - 1u, fu_cg<MODE>(col + fu_ro<MODE>(idx + q)), side ? ~0ull : 1ull);
+                for (uint64_t q = fu_off<MODE>(a, v) + threadIdx.x; q < e && ok; q += kFuThreads)
+                    ok = fu_count(key, val, kFuCheckSlots - 1u, kFuProbes, fu_cg<MODE>(col + fu_ro<MODE>(idx + q)), side ? ~0ull : 1ull);
             }
             if (!ok) atomicOr(&s_flag, 2u);
             __syncthreads();
@@ -496,7 +496,14 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
             for (uint32_t k = threadIdx.x; k < kFuCheckSlots; k += kFuThreads) diff |= val[k] != 0ull;
             if (diff) atomicOr(&s_flag, 1u);
             __syncthreads();
-            if (threadIdx.x == 0 && s_flag) ++nbad;
+            if (threadIdx.x == 0) {
+                if (s_flag & 2u) {
+                    atomicOr(&w->overflow, 1u);
+                    a.list[i] = u | kSingleton;
+                } else {
+                    nbad += s_flag;
+                }
+            }
             __syncthreads();
         }
         if (threadIdx.x == 0) s_sum = 0u;
@@ -507,7 +514,8 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
             return;
         }
     }
-    finish(nfail ? kFuRowTooWide : kFuOk);
+    if (first) a.res->failed = nfail;
+    finish(nfail || fu_cg<MODE>(&w->overflow) ? kFuUndecided : kFuOk);
 }
 
 }  // namespace rbsc

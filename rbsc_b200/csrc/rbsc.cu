@@ -645,13 +645,15 @@ static rbsc_status graph_load(rbsc_ctx* ctx, const rbsc_csr* c, bool from_device
 }
 
 rbsc_status graph_upload_oneshot(rbsc_ctx* ctx, const rbsc_csr* c, const uint32_t* init_colors, rbsc_graph** out, double* h2d_ms,
-                                 uint64_t* h2d_bytes)
+                                 uint64_t* h2d_bytes, bool launch_off)
 {
     CKS(check_csr_args(ctx, c));
     // large unweighted graphs: the heads' copy overlaps the refinement
     const bool defer = !c->weights && c->m >= (1ull << 22);
-    CKS(graph_load(ctx, c, false, out, h2d_ms, h2d_bytes, defer, init_colors, fused_wanted(ctx, c->n, c->m, c->weights != nullptr, defer)));
+    const bool unprepared = !launch_off && fused_wanted(ctx, c->n, c->m, c->weights != nullptr, defer);
+    CKS(graph_load(ctx, c, false, out, h2d_ms, h2d_bytes, defer, init_colors, unprepared));
     (*out)->oneshot = true;
+    (*out)->launch_off = launch_off;
     return RBSC_OK;
 }
 
@@ -1726,7 +1728,7 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         if (stats) stats->done = stats->verified = 1;
         return RBSC_OK;
     }
-    if (!kt && !g->host_arcs && !g->stream_upload && fused_wanted(ctx, n, g->m, g->weighted, d_init && !g->oneshot)) {
+    if (!kt && !g->host_arcs && !g->stream_upload && !g->launch_off && fused_wanted(ctx, n, g->m, g->weighted, d_init && !g->oneshot)) {
         bool handled = false;
         CKS(fused_refine(ctx, g, d_init, d_out, stats, &handled));
         if (handled) return RBSC_OK;
@@ -1883,7 +1885,7 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         CKS(read_state(ctx, g));
         if (hs.error & kErrStage) return rbsc_fail(ctx, RBSC_ERR_DEVICE, "signature: a staged tile copy did not complete");
         if (hs.error & kErrInput) return rbsc_fail(ctx, RBSC_ERR_INVALID, "an arc head is >= N");
-        // a collision or a row too wide: once more, launch by launch
+        // (its launch_off is set) once more, launch by launch
         return refine_resident(ctx, g, d_init, d_out, stats, kt);
     }
 
@@ -2023,10 +2025,10 @@ extern "C" rbsc_status rbsc_refine(rbsc_ctx* ctx, const rbsc_csr* host_graph, co
     double up_ms = 0;
     uint64_t up_bytes = 0;
     CKS(check_csr_args(ctx, host_graph));
-    bool handled = false;
-    CKS(fused_oneshot(ctx, host_graph, init_colors, out_labels, stats, &handled));
+    bool handled = false, gave_up = false;
+    CKS(fused_oneshot(ctx, host_graph, init_colors, out_labels, stats, &handled, &gave_up));
     if (handled) return RBSC_OK;
-    CKS(graph_upload_oneshot(ctx, host_graph, init_colors, &g, &up_ms, &up_bytes));
+    CKS(graph_upload_oneshot(ctx, host_graph, init_colors, &g, &up_ms, &up_bytes, gave_up));
     rbsc_status st = rbsc_graph_refine(ctx, g, init_colors, out_labels, stats);
     up_ms += g->up_ms;
     rbsc_graph_free(g);
