@@ -1,6 +1,6 @@
 // check_kernels.cuh -- the rows that a one-launch refinement's exact check left
 // undecided (fused_kernels.cuh, list_kernels.cuh): those with more colours than
-// a block's table in shared memory holds.
+// a block's table in shared memory holds, or more arcs than it may count.
 //
 // They are few and long (both copies of a hub of a lifted skewed graph, pages
 // with the same list of thousands of links), so all warps share their arcs:

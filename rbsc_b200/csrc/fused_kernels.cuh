@@ -68,6 +68,12 @@ constexpr uint32_t kFuWarpSlots = kFuCheckSlots / (kFuThreads / 32);
 constexpr uint32_t kFuWarpRow = kFuWarpSlots - 8;  // rows up to this length are tried by one warp
 constexpr uint32_t kFuWideSlots = 32768;    // per block, in global memory: any row of a graph of at most 16384 nodes
 
+// Arcs that a block counts in its table of the check, beside 4 / blocks of the
+// graph's: the others wait for it at a bounded barrier, so the rows beyond are
+// left undecided.  A block counts an arc in 1.7 ns (two rows of 3 M arcs: 10 ms,
+// shared by all warps 0.6), so these take 2 ms, and the share of a graph of 2^32
+// arcs 0.2 s.
+constexpr uint64_t kFuCheckArcs = 1ull << 20;
 constexpr uint32_t kFuProbes = 256;  // of the shared table: one that takes longer is as good as full
 
 // outcome of a launch (FusedResult.status)
@@ -82,7 +88,7 @@ struct FusedWords {
     unsigned long long bar[2];  // barrier words (fu_barrier)
     uint32_t pad[28];
     uint32_t bad;          // 1 = offsets, 2 = a head
-    uint32_t overflow;     // a row had more colours than the check's table: marked in the list
+    uint32_t overflow;     // a row had more colours than the check's table, or too many arcs: marked in the list
     uint32_t nlong, nchunk;
     uint32_t nlist[2];     // long rows of the running check (by repair parity)
 };
@@ -978,9 +984,22 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                     return;
                 }
             }
+            uint64_t spent = 0;
+            const uint64_t most = kFuCheckArcs + 4 * (a.m / gridDim.x);
             for (uint32_t i = blockIdx.x; i < nlist; i += gridDim.x) {
-                const uint32_t u = a.list[i], r = fu_cg<MODE>(a.minm + fu_cg<MODE>(col + u));
+                // (thread 0 may be marking it already)
+                const uint32_t u = a.list[i] & ~kSingleton, r = fu_cg<MODE>(a.minm + fu_cg<MODE>(col + u));
                 if (WEIGHTED && longest(u, r) <= kFuWarpRow && fu_cg<MODE>(a.fail + u) != 2) continue;
+                if (MODE != kFuBlock && !a.wide) {
+                    spent += fu_end<MODE>(a, u) - fu_off<MODE>(a, u) + (fu_end<MODE>(a, r) - fu_off<MODE>(a, r));
+                    if (spent > most) {
+                        if (threadIdx.x == 0) {
+                            atomicOr(&w->overflow, 1u);
+                            a.list[i] = u | kSingleton;
+                        }
+                        continue;
+                    }
+                }
                 uint32_t* key = s_key;
                 unsigned long long* val = s_val;
                 // (a graph in shared memory has fewer nodes than the table half its slots)

@@ -36,8 +36,8 @@
 // each warp folding its own list only, without dealing a block's groups out (35 %
 // of the warps' time went into waiting at barriers): 2.43.
 //
-// Unit weights.  Rows with more colours than the check's table holds are left to
-// check_kernels.cuh.  When a node fails the check (a hash collision), the
+// Unit weights.  Rows with more colours than the check's table holds, or more
+// arcs than a block may count, are left to check_kernels.cuh.  When a node fails the check (a hash collision), the
 // refinement is done again launch by launch.
 #pragma once
 #include <cstdint>
@@ -475,8 +475,18 @@ static __global__ void __launch_bounds__(kFuThreads, 1) k_refine_rows(const __gr
         unsigned long long* const val = s_buf;
         uint32_t* const key = reinterpret_cast<uint32_t*>(s_buf + kFuCheckSlots);
         nbad = 0;
+        uint64_t spent = 0;
+        const uint64_t most = kFuCheckArcs + 4 * (a.m / gridDim.x);
         for (uint32_t i = blockIdx.x; i < nlist; i += gridDim.x) {
-            const uint32_t u = a.list[i], r = fu_cg<MODE>(a.minm + (fu_cg<MODE>(col + u) & ~kSlotBit));
+            const uint32_t u = a.list[i] & ~kSingleton, r = fu_cg<MODE>(a.minm + (fu_cg<MODE>(col + u) & ~kSlotBit));
+            spent += fu_end<MODE>(a, u) - fu_off<MODE>(a, u) + (fu_end<MODE>(a, r) - fu_off<MODE>(a, r));
+            if (spent > most) {
+                if (threadIdx.x == 0) {
+                    atomicOr(&w->overflow, 1u);
+                    a.list[i] = u | kSingleton;
+                }
+                continue;
+            }
             for (uint32_t k = threadIdx.x; k < kFuCheckSlots; k += kFuThreads) {
                 key[k] = 0xffffffffu;
                 val[k] = 0ull;

@@ -1,6 +1,6 @@
-"""Rows with more colours than a block's table of the exact check holds, whose
-node shares its class: the one-launch refinements decide them in a launch of
-their own (check_kernels.cuh) and do not start again."""
+"""Rows with more colours than a block's table of the exact check holds, or more
+arcs than it may count, whose node shares its class: the one-launch refinements
+decide them in a launch of their own (check_kernels.cuh) and do not start again."""
 import numpy as np
 import pytest
 
@@ -140,6 +140,47 @@ def test_differences_are_found(weighted, more):
         for r in (ctx.refine(off, idx, w, init), g.refine(init), g.refine(init)):
             assert r.verified == 1 and r.blocks == ex.blocks and np.array_equal(r.labels, ex.labels)
         g.free()
+
+
+def _long_hubs(d, hubs, heads=300):
+    """`hubs` nodes with d arcs each to the same few heads."""
+    dst = hubs + np.arange(d, dtype=np.int64) * 7 % heads
+    src = np.repeat(np.arange(hubs), d)
+    off, idx, _ = G.csr_from_arcs(hubs + heads, src, np.tile(dst, hubs), sort=False)
+    return off, idx, np.concatenate([np.zeros(hubs), 1 + np.arange(heads) % 40]).astype(np.uint32)
+
+
+@pytest.mark.parametrize("kind", ["unit", "weighted", "uniform"])
+@pytest.mark.parametrize("d", [540_000, 3_000_000])
+def test_rows_of_more_arcs_than_a_block_counts(d, kind):
+    """Shared by all warps: the first launch and three of the check's own (a
+    call whose only work they are would otherwise wait for one block)."""
+    off, idx, init = _long_hubs(d, 2, heads=1 if kind == "uniform" else 300)
+    wt = (idx % 3 + 1).astype(np.uint64) if kind == "weighted" else None
+    init = None if kind == "uniform" else init
+    ex = _few_launches(off, idx, wt, init, most=40)
+    assert ex.labels[1] == 0
+    with R.Context(0) as ctx:
+        r = ctx.refine(off, idx, wt, init)
+        ctx.set_opts(verify=False)
+        assert r.kernel_launches == ctx.refine(off, idx, wt, init).kernel_launches + 3
+
+
+def test_long_member_of_few_colours_beside_short_rows():
+    """60,000 arcs of the member read once for each of 5,000 rows."""
+    n_short, k, heads = 5000, 60000, 1500
+    src = np.concatenate([np.zeros(k + 1, np.int64), np.arange(1, n_short + 1)])
+    dst = np.concatenate([n_short + 1 + np.arange(k) % heads, np.full(n_short + 1, n_short + 1 + heads)])
+    n = n_short + heads + 2
+    off, idx, w = G.csr_from_arcs(n, src, dst, np.where(dst == n - 1, 5, 0), sort=False)
+    init = np.concatenate([np.zeros(n_short + 1), np.arange(1, heads + 2)]).astype(np.uint32)
+    ex = oracle.refine_exact(off, idx, w, init)
+    assert (ex.labels[: n_short + 1] == 0).all()
+    with R.Context(0) as ctx:
+        for _ in range(2):
+            r = ctx.refine(off, idx, w, init)
+            _same(r, ex)
+            assert r.kernel_launches > 30  # decided launch by launch
 
 
 def test_edge_batches_with_wide_rows():
