@@ -304,6 +304,7 @@ static __global__ void __launch_bounds__(1024, 1) k_inc_passes(IncArgs a)
         cur ^= 1u;
         __syncthreads();
     }
+    if (!done && round >= a.max_rounds) over = 1;  // (a wide last pass ends the loop before the test in it)
     if (tid == 0) {
         a.ctr->done = done;
         a.ctr->rounds = round;

@@ -120,3 +120,23 @@ def test_classes_that_shed_nodes(length, groups, weighted):
             assert r.verified == 1 and (r.blocks, r.rounds) == (ex.blocks, ex.rounds)
             assert np.array_equal(r.labels, ex.labels) and r.round_blocks == ex.round_blocks[: len(r.round_blocks)]
         g.free()
+
+
+@pytest.mark.gpu
+def test_the_last_allowed_pass_changes_many_sums():
+    """3,000 nodes point at the first two nodes of a chain, which part last: more
+    changed sums than the list holds, in the last pass but one."""
+    length, many = 100, 3000
+    c = np.arange(length - 1)
+    p = length + np.arange(many)
+    off, idx, _ = G.csr_from_arcs(length + many, np.concatenate([c, p, p]), np.concatenate([c + 1, 0 * p, 0 * p + 1]))
+    init = np.concatenate([np.zeros(length), np.ones(many)]).astype(np.uint32)
+    ex = oracle.refine_exact(off, idx, None, init)
+    assert ex.rounds == length
+    with R.Context(0, max_rounds=ex.rounds - 1) as ctx:
+        with pytest.raises(R.RbscError, match="no fixpoint"):
+            ctx.refine(off, idx, None, init)
+        ctx.set_opts(max_rounds=ex.rounds)
+        r = ctx.refine(off, idx, None, init)
+        assert r.kernel_launches > 5 and r.verified == 1
+        assert (r.blocks, r.rounds) == (ex.blocks, ex.rounds) and np.array_equal(r.labels, ex.labels)
