@@ -516,9 +516,10 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
     const uint64_t lc0 = rbsc::launch_counter();
     const FusedLayout l = fused_layout(g->n, g->m);
     EKS(ensure_work(ctx, g, l.bytes));
-    // labels may be asked for over the initial colours, which the check reads
+    // labels may be asked for over the initial colours, which the check reads;
+    // and a call that runs out of rounds leaves the caller's array alone
     uint32_t* const asked = d_out;
-    if (!d_out || labels_over_init(d_init, d_out, g->n)) {
+    if (!d_out || ctx->opts.max_rounds || labels_over_init(d_init, d_out, g->n)) {
         if (!g->d_out) EKS(dev_alloc(ctx, (void**)&g->d_out, 4 * (size_t)g->n));
         d_out = g->d_out;
     }

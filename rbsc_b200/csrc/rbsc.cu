@@ -1800,7 +1800,9 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         CK(cudaMemcpyAsync(g->h_st, g->d_st, sizeof(RoundState), cudaMemcpyDeviceToHost, s));
         CK(cudaEventRecord(ctx->ev[7], s));
     }
-    uint32_t* const labels = d_out ? d_out : g->d_out;
+    // (k_refine_rows writes labels as it goes: a call that runs out of rounds
+    // leaves the caller's array alone)
+    uint32_t* const labels = d_out && !ctx->opts.max_rounds ? d_out : g->d_out;
     CKS(init_active_set(ctx, g, true, rows_only));
     if (rows_only) CKS(list_arcless(ctx, g, labels));
     if (kt) {
@@ -1867,6 +1869,10 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         bool handled = false;
         CKS(list_refine(ctx, g, d_init, labels, initial_blocks, stats, &handled));
         if (handled) {
+            if (d_out && d_out != labels) {
+                CK(cudaMemcpyAsync(d_out, labels, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s));
+                CK(cudaStreamSynchronize(s));
+            }
             if (stats) {
                 float ms = 0.f, init_ms = 0.f;
                 cudaEventElapsedTime(&ms, ctx->ev_sig[0], ctx->ev_sig[1]);
