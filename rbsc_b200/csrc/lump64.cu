@@ -488,14 +488,15 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
     const unsigned long long* w64 = reinterpret_cast<const unsigned long long*>(g->d_wt);
     const unsigned long_grid = (unsigned)ctx->sm_count * 8;
     // the arcs in play: all of them at first; once a pass leaves less than 3/4
-    // of them, the others are dropped (a copy in order, two buffers in turn)
+    // of them, the others are dropped (a copy in order, two buffers in turn; no
+    // memory for one: the passes go on with the arcs they have)
     uint64_t live = M;
     const uint32_t *asrc = src, *aidx = g->d_idx;
     const unsigned long long* aw = w64;
     int sb = 0, ab = 0;  // start[sb]: the row starts of the arcs in play; l*[ab]: where the next copy goes
-    const uint64_t M0 = M;
+    bool drop = M > 0;
     for (;;) {
-        if (rounds > 0 && M0) {
+        if (rounds > 0 && drop) {
             ++rbsc::launch_counter();
             k_l64_live_lengths<<<grid_of(N), kT, 0, s>>>(N, start[sb], alone, start[sb ^ 1]);
             EK((exclusive_scan<uint32_t, uint32_t>(start[sb ^ 1], start[sb ^ 1], N, start[sb ^ 1] + N, tmp, s)));
@@ -504,21 +505,22 @@ extern "C" rbsc_status rbsc_refine_f64(rbsc_ctx* ctx, const rbsc_csr* host_graph
             EK(cudaStreamSynchronize(s));
             if ((uint64_t)left * 4 <= live * 3) {
                 // (the first copy of each buffer is the largest it will hold)
-                if (!lsrc[ab]) {
-                    EKS(sc.get(&lsrc[ab], left));
-                    EKS(sc.get(&lidx[ab], left));
-                    EKS(sc.get(&lw[ab], left));
+                if (!lw[ab] && (sc.get(&lsrc[ab], left) != RBSC_OK || sc.get(&lidx[ab], left) != RBSC_OK || sc.get(&lw[ab], left) != RBSC_OK)) {
+                    if (lsrc[ab]) sc.release(lsrc[ab]);
+                    if (lidx[ab]) sc.release(lidx[ab]);
+                    drop = false;
+                } else {
+                    ++rbsc::launch_counter();
+                    k_l64_live_arcs<<<grid_of(live), kT, 0, s>>>(live, asrc, aidx, aw, start[sb], start[sb ^ 1], alone, lsrc[ab], lidx[ab],
+                                                                lw[ab]);
+                    EK(cudaGetLastError());
+                    asrc = lsrc[ab];
+                    aidx = lidx[ab];
+                    aw = lw[ab];
+                    ab ^= 1;
+                    sb ^= 1;
+                    live = left;
                 }
-                ++rbsc::launch_counter();
-                k_l64_live_arcs<<<grid_of(live), kT, 0, s>>>(live, asrc, aidx, aw, start[sb], start[sb ^ 1], alone, lsrc[ab], lidx[ab],
-                                                            lw[ab]);
-                EK(cudaGetLastError());
-                asrc = lsrc[ab];
-                aidx = lidx[ab];
-                aw = lw[ab];
-                ab ^= 1;
-                sb ^= 1;
-                live = left;
             }
         }
         const uint64_t M = live;
