@@ -106,7 +106,7 @@ uint32_t deep_round(uint64_t m)
 
 // The passes after a launch that ended with kFuDeep, on a work list: the
 // classes of its last two passes are in a.col.  Leaves the launch that
-// confirms (or goes on) in `a`.
+// confirms (or goes on, as it does when there is no memory for the list) in `a`.
 rbsc_status deep_tail(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
 {
     FusedResult& r = *static_cast<FusedResult*>(ctx->h_fused);
@@ -125,15 +125,18 @@ rbsc_status deep_tail(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
     uint32_t *cursor = nullptr, *tsrc = nullptr, *colm = nullptr, *tlist = nullptr;
     uint64_t* twt = nullptr;
     unsigned char* tmp = nullptr;
-    EKS(sc.get(&z, z_bytes));
-    EKS(sc.get(&S, ids));
-    EKS(sc.get(&sig, n));
-    EKS(sc.get(&cursor, n));
-    EKS(sc.get(&colm, n));
-    EKS(sc.get(&tlist, kIncCap));
-    EKS(sc.get(&tsrc, a.m));
-    if (a.wt) EKS(sc.get(&twt, a.m));
-    EKS(sc.get(&tmp, scan_temp_bytes<uint32_t>((uint64_t)n + 1) + 1024));
+    const auto room = [&]() {
+        return sc.get(&z, z_bytes) == RBSC_OK && sc.get(&S, ids) == RBSC_OK && sc.get(&sig, n) == RBSC_OK && sc.get(&cursor, n) == RBSC_OK &&
+               sc.get(&colm, n) == RBSC_OK && sc.get(&tlist, kIncCap) == RBSC_OK && sc.get(&tsrc, a.m) == RBSC_OK &&
+               (!a.wt || sc.get(&twt, a.m) == RBSC_OK) && sc.get(&tmp, scan_temp_bytes<uint32_t>((uint64_t)n + 1) + 1024) == RBSC_OK;
+    };
+    a.start = col;
+    a.validate = 0;
+    if (!room()) {  // full passes to the end
+        a.round0 = r.rounds;
+        a.deep_round = 0;
+        return RBSC_OK;
+    }
     uint32_t* size = reinterpret_cast<uint32_t*>(z + z_size);
     uint32_t* deg = reinterpret_cast<uint32_t*>(z + z_deg);
     IncCounters* ctr = reinterpret_cast<IncCounters*>(z + z_ctr);
@@ -177,8 +180,6 @@ rbsc_status deep_tail(rbsc_ctx* ctx, FusedArgs& a, cudaStream_t s)
     EK(cudaMemcpyAsync(&h, ctr, sizeof h, cudaMemcpyDeviceToHost, s));
     EK(cudaStreamSynchronize(s));
     if (h.over) return rbsc_fail(ctx, RBSC_ERR_NOT_CONVERGED, "no fixpoint after %u passes", h.rounds);
-    a.start = col;
-    a.validate = 0;
     // the pass that found nothing to change is run again in full, to confirm it
     a.round0 = h.done ? h.rounds - 1u : h.rounds;
     a.deep_round = h.done ? 0u : 2u * h.rounds;

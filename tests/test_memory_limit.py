@@ -1,5 +1,6 @@
-"""Double weights when the device has no room for the copy of the arcs in play
-(lump64.cu), which only saves time: the call goes on without it."""
+"""Steps that only save time, on a device without the memory for them: the copy
+of the arcs in play (lump64.cu), the work list of deep refinements
+(deep_kernels.cuh).  The call goes on without them."""
 import numpy as np
 import pytest
 
@@ -21,24 +22,38 @@ def _half_twins(n, d):
     return off, heads.astype(np.uint32).ravel(), wt.ravel()
 
 
-def test_no_room_for_the_arcs_in_play():
+def _short_of(spare, call):
+    """call's result on an empty device, and on one that lacks `spare` of the
+    bytes which that took (a context keeps its blocks)."""
     import torch
-    off, idx, wt = _half_twins(1 << 17, 64)  # the copy takes 16 bytes for half of 8 M arcs
     with R.Context(0) as ctx:
-        ctx.refine_f64(off, idx, wt)
+        call(ctx)  # (the kernels are loaded)
     torch.cuda.synchronize()
     free = torch.cuda.mem_get_info()[0]
     with R.Context(0) as ctx:
-        want = ctx.refine_f64(off, idx, wt)
-        used = free - torch.cuda.mem_get_info()[0]  # the context keeps its blocks
-    copy = 16 * len(idx) // 2
-    assert used > 2 * copy
-    hog = torch.empty(torch.cuda.mem_get_info()[0] - used + copy // 2, dtype=torch.uint8, device="cuda")
+        want = call(ctx)
+        used = free - torch.cuda.mem_get_info()[0]
+    assert used > 2 * spare
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - used + spare, dtype=torch.uint8, device="cuda")
     try:
         with R.Context(0) as ctx:
-            r = ctx.refine_f64(off, idx, wt)
+            got = call(ctx)
     finally:
         del hog
         torch.cuda.empty_cache()
-    assert (r.blocks, r.rounds, r.verified) == (want.blocks, want.rounds, 1) and np.array_equal(r.labels, want.labels)
-    assert r.kernel_launches != want.kernel_launches  # (the copies' launches)
+    assert (got.blocks, got.rounds, got.verified) == (want.blocks, want.rounds, 1) and np.array_equal(got.labels, want.labels)
+    return got, want
+
+
+def test_no_room_for_the_arcs_in_play():
+    off, idx, wt = _half_twins(1 << 17, 64)  # the copy takes 16 bytes for half of 8 M arcs
+    got, want = _short_of(4 * len(idx), lambda ctx: ctx.refine_f64(off, idx, wt))
+    assert got.kernel_launches != want.kernel_launches
+
+
+def test_no_room_for_the_work_list():
+    n, k = 1 << 20, 300  # the list takes some 76 bytes per node, most of them after the launch's own
+    off = np.minimum(np.arange(n + 1), k).astype(np.uint64)
+    idx = np.arange(1, k + 1, dtype=np.uint32)
+    got, want = _short_of(30 << 20, lambda ctx: ctx.refine(off, idx))
+    assert want.rounds == k + 1 and got.kernel_launches < want.kernel_launches
