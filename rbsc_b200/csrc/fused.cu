@@ -516,7 +516,8 @@ rbsc_status fused_refine(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init, u
     cudaStream_t s = ctx->stream;
     const uint64_t lc0 = rbsc::launch_counter();
     const FusedLayout l = fused_layout(g->n, g->m);
-    EKS(ensure_work(ctx, g, l.bytes));
+    // (the launch-per-phase path may have its buffers already)
+    if (ensure_work(ctx, g, l.bytes) != RBSC_OK) return RBSC_OK;
     // labels may be asked for over the initial colours, which the check reads;
     // and a call that runs out of rounds leaves the caller's array alone
     uint32_t* const asked = d_out;

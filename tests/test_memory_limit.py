@@ -1,6 +1,7 @@
 """Steps that only save time, on a device without the memory for them: the copy
 of the arcs in play (lump64.cu), the work list of deep refinements
-(deep_kernels.cuh).  The call goes on without them."""
+(deep_kernels.cuh), the one-launch refinement itself (fused.cu) of a graph that has
+the buffers of the other path.  The call goes on without them."""
 import numpy as np
 import pytest
 
@@ -57,3 +58,26 @@ def test_no_room_for_the_work_list():
     idx = np.arange(1, k + 1, dtype=np.uint32)
     got, want = _short_of(30 << 20, lambda ctx: ctx.refine(off, idx))
     assert want.rounds == k + 1 and got.kernel_launches < want.kernel_launches
+
+
+def test_no_room_for_the_one_launch_refinement():
+    import torch
+    off, idx = G.er_directed(1 << 20, 1 << 21, seed=3)
+    with R.Context(0) as ctx:
+        one = ctx.refine(off, idx)
+        ctx.trim()
+        ctx.set_opts(persistent=False)
+        g = ctx.upload(off, idx)
+        want = g.refine()
+        ctx.set_opts(persistent=True)
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - (16 << 20), dtype=torch.uint8, device="cuda")
+        try:
+            got = g.refine()
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        again = g.refine()
+        g.free()
+    assert got.kernel_launches > again.kernel_launches == one.kernel_launches
+    for r in (one, got, again):
+        assert (r.blocks, r.rounds, r.verified) == (want.blocks, want.rounds, 1) and np.array_equal(r.labels, want.labels)
