@@ -281,6 +281,7 @@ extern "C" rbsc_status rbsc_graph_batch_refine(rbsc_ctx* ctx, rbsc_graph* g, con
     uint64_t hH = 0;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     float batch_ms = 0.f;
+    std::chrono::steady_clock::time_point c0;  // the first result copy
     // the refinement of the union
     BKS(rbsc_graph_refine(ctx, g, init_colors, nullptr, stats));
     BK(cudaEventCreate(&e0));
@@ -309,11 +310,11 @@ extern "C" rbsc_status rbsc_graph_batch_refine(rbsc_ctx* ctx, rbsc_graph* g, con
         BK(cudaEventRecord(e1, s));
         BK(cudaMemcpyAsync(&hH, hoff + G, 8, cudaMemcpyDeviceToHost, s));
         // the colours (final already) travel beside these kernels
+        c0 = std::chrono::steady_clock::now();
         if (out->colors) BKS(copy_out(ctx, out->colors, g->d_out, 4 * (size_t)n, ctx->side));
         BK(cudaStreamSynchronize(s));
         H = (uint32_t)hH;
     } else {
-        if (out->colors) BKS(copy_out(ctx, out->colors, g->d_out, 4 * (size_t)n, s));
         BKS(dev_alloc(ctx, (void**)&keys, 8 * (size_t)n));
         BKS(dev_alloc(ctx, (void**)&keys2, 8 * (size_t)n));
         BKS(dev_alloc(ctx, (void**)&vals, 4 * (size_t)n));
@@ -353,6 +354,9 @@ extern "C" rbsc_status rbsc_graph_batch_refine(rbsc_ctx* ctx, rbsc_graph* g, con
         k_batch_blocks<<<grid_of(G), 256, 0, s>>>(G, hoff, blocks);
         BK(cudaGetLastError());
         BK(cudaEventRecord(e1, s));
+        BK(cudaStreamSynchronize(s));
+        c0 = std::chrono::steady_clock::now();
+        if (out->colors) BKS(copy_out(ctx, out->colors, g->d_out, 4 * (size_t)n, s));
     }
     if (out->local) BKS(copy_out(ctx, out->local, local, 4 * (size_t)n, s));
     if (out->blocks) BK(cudaMemcpyAsync(out->blocks, blocks, 4 * (size_t)G, cudaMemcpyDeviceToHost, s));
@@ -366,6 +370,7 @@ extern "C" rbsc_status rbsc_graph_batch_refine(rbsc_ctx* ctx, rbsc_graph* g, con
     if (stats) {
         stats->device_ms += batch_ms;
         if (out->colors) stats->d2h_bytes = 4ull * n;
+        stats->d2h_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - c0).count();
         stats->time_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     }
 done:
