@@ -937,15 +937,9 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
             // ones (weighted) in its part of the block's table and leaves them
             // to the block when they do not fit.
             nbad = 0;
-            // (false: the table is full, and what it holds is of no use)
-            auto add_row = [&](uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t probes, uint32_t x, bool minus, uint32_t at,
-                               uint32_t step) -> bool {
-                const uint64_t b = fu_off<MODE>(a, x), e = fu_end<MODE>(a, x);
-                for (uint64_t i = b + at; i < e; i += step) {
-                    const uint64_t v = WEIGHTED ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + i) : 1ull;
-                    if (!fu_count(key, val, mask, probes, fu_cg<MODE>(col + fu_ro<MODE>(idx + i)), minus ? 0ull - v : v)) return false;
-                }
-                return true;
+            auto add_arc = [&](uint32_t* key, unsigned long long* val, uint32_t mask, uint32_t probes, uint64_t i, bool minus) -> bool {
+                const uint64_t v = WEIGHTED ? fu_ro<MODE>(reinterpret_cast<const unsigned long long*>(wt) + i) : 1ull;
+                return fu_count(key, val, mask, probes, fu_cg<MODE>(col + fu_ro<MODE>(idx + i)), minus ? 0ull - v : v);
             };
             auto longest = [&](uint32_t u, uint32_t r) {
                 return max((uint32_t)(fu_end<MODE>(a, u) - fu_off<MODE>(a, u)), (uint32_t)(fu_end<MODE>(a, r) - fu_off<MODE>(a, r)));
@@ -962,8 +956,11 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                         val[k] = 0ull;
                     }
                     __syncwarp();
-                    bool ok = add_row(key, val, kFuWarpSlots - 1u, kFuWarpSlots, r, false, lane, 32);
-                    ok = ok && add_row(key, val, kFuWarpSlots - 1u, kFuWarpSlots, u, true, lane, 32);
+                    bool ok = true;
+                    for (int side = 0; side < 2; ++side) {
+                        const uint64_t b = fu_off<MODE>(a, side ? u : r), e = fu_end<MODE>(a, side ? u : r);
+                        for (uint64_t k = b + lane; k < e; k += 32) ok &= add_arc(key, val, kFuWarpSlots - 1u, kFuWarpSlots, k, side);
+                    }
                     __syncwarp();
                     bool diff = false;
                     for (uint32_t k = lane; k < kFuWarpSlots; k += 32) diff |= val[k] != 0ull;
@@ -1011,8 +1008,11 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                     }
                     if (threadIdx.x == 0) s_flag = 0u;
                     __syncthreads();
-                    bool ok = add_row(key, val, slots - 1u, probes, r, false, threadIdx.x, kFuThreads);
-                    ok = ok && add_row(key, val, slots - 1u, probes, u, true, threadIdx.x, kFuThreads);
+                    bool ok = true;  // (false: the table is full, and what it holds is of no use)
+                    for (int side = 0; side < 2 && ok; ++side) {
+                        const uint64_t b = fu_off<MODE>(a, side ? u : r), e = fu_end<MODE>(a, side ? u : r);
+                        for (uint64_t k = b + threadIdx.x; k < e && ok; k += kFuThreads) ok = add_arc(key, val, slots - 1u, probes, k, side);
+                    }
                     if (!ok) atomicOr(&s_flag, 2u);
                     __syncthreads();
                     bool diff = false;
