@@ -96,11 +96,12 @@ void common_args(const rbsc_ctx* ctx, FusedArgs& a)
 }
 
 // When to look for a deep refinement: once the passes so far have cost about
-// as much as the change to the work list does (us; a pass takes about 6 + 1
-// per 100,000 arcs, the change 150 + 1 per 20,000).
-uint32_t deep_round(uint64_t m)
+// as much as the change to the work list does (us; a pass takes about 6 + 1 per
+// 100,000 arcs and per 33,000 nodes, the change 150 + 1 per 20,000 arcs and per
+// 3,000 nodes).
+uint32_t deep_round(uint32_t n, uint64_t m)
 {
-    const double pass = 6.0 + (double)m / 100e3, change = 150.0 + (double)m / 20e3;
+    const double pass = 6.0 + (double)m / 100e3 + n / 33e3, change = 150.0 + (double)m / 20e3 + n / 3e3;
     return (uint32_t)std::max(6.0, change / pass);
 }
 
@@ -284,7 +285,7 @@ rbsc_status run(rbsc_ctx* ctx, FusedArgs& a, const FusedLayout& l, cudaStream_t 
     // one block keeps its classes in shared memory: nothing to continue from
     // (and a pass there costs less than one on the work list)
     const bool block = rows_side_by_side(a) && fused_fits_block(a, l);
-    a.deep_round = block ? 0u : deep_round(a.m);
+    a.deep_round = block ? 0u : deep_round(a.n, a.m);
     EK(cudaEventRecord(ctx->ev[0], s));
     EKS(launch_and_wait(ctx, a, l, block, s));
     const uint32_t initial = r.initial_blocks;

@@ -1,0 +1,54 @@
+"""Which way a sparse graph of many nodes takes, and that it gives the oracle's
+result there."""
+import numpy as np
+import pytest
+
+import rbsc_b200 as R
+from oracle import oracle
+from rbsc_b200 import graphs as G
+
+pytestmark = pytest.mark.gpu
+
+
+def _er(n, m, seed):
+    rng = np.random.default_rng(seed)
+    src = np.sort(rng.integers(0, n, m))
+    off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.uint64)
+    return off, rng.integers(0, n, m).astype(np.uint32)
+
+
+def _same(r, ex):
+    assert r.done == 1 and r.verified == 1
+    assert (r.blocks, r.rounds) == (ex.blocks, ex.rounds)
+    assert np.array_equal(r.labels, ex.labels)
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_passes_that_soon_make_no_more_classes(seed):
+    """A random graph's last passes make fewer and fewer classes: no work list for
+    the one or two that are left."""
+    off, idx = _er(1 << 20, 734003, seed)
+    ex = oracle.refine_exact(off, idx)
+    assert ex.rounds >= 15
+    with R.Context(0) as ctx:
+        r = ctx.refine(off, idx)
+    _same(r, ex)
+    assert r.kernel_launches <= 2
+
+
+@pytest.mark.parametrize("chain,extra", [(60, 0), (400, 0), (60, 300)])
+def test_passes_that_go_on_making_classes(chain, extra):
+    """Chains keep making the same number: the work list takes over, also after
+    passes that made many at once (extra: nodes with rows of their own)."""
+    k = np.arange(chain)
+    src, dst = [k, 20000 + k], [k + 1, 20000 + k + 1]
+    n = 40000
+    for e in range(extra):
+        src.append(np.full(e % 7 + 1, 30000 + e))
+        dst.append(30000 + (e * 13 + np.arange(e % 7 + 1)) % 301)
+    off, idx, _ = G.csr_from_arcs(n, np.concatenate(src), np.concatenate(dst))
+    ex = oracle.refine_exact(off, idx)
+    with R.Context(0) as ctx:
+        r = ctx.refine(off, idx)
+    _same(r, ex)
+    assert r.rounds > chain and r.kernel_launches > 5
