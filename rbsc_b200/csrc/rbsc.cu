@@ -1728,7 +1728,15 @@ rbsc_status refine_resident(rbsc_ctx* ctx, rbsc_graph* g, const uint32_t* d_init
         if (stats) stats->done = stats->verified = 1;
         return RBSC_OK;
     }
-    if (!kt && !g->host_arcs && !g->stream_upload && !g->launch_off && fused_wanted(ctx, n, g->m, g->weighted, d_init && !g->oneshot)) {
+    // A prepared graph of many nodes and few arcs is better off with passes over
+    // its rows alone: the one launch walks all nodes and clears tables for them in
+    // every pass.  us, one launch / launch by launch, by arcs per node: 2^21 nodes
+    // 0.02: 331 / 313, 0.3: 837 / 636, 0.7: 1455 / 1120, 1.0: 1520 / 1470, 1.15: 1480
+    // / 1575; 2^22 nodes 0.02: 651 / 410, 0.3: 1702 / 1025, 0.7: 2500 / 2100-2580; at
+    // 2^20 nodes the one launch wins throughout (0.3: 424 / 517, 0.7: 798 / 815).
+    // Unprepared, or weighted (whose check sorts there), it wins at every size.
+    const bool sparse = g->prepared && !g->weighted && n > (1u << 20) && g->m < n + n / 8;
+    if (!kt && !g->host_arcs && !g->stream_upload && !g->launch_off && !sparse && fused_wanted(ctx, n, g->m, g->weighted, d_init && !g->oneshot)) {
         bool handled = false;
         CKS(fused_refine(ctx, g, d_init, d_out, stats, &handled));
         if (handled) return RBSC_OK;

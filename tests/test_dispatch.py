@@ -52,3 +52,27 @@ def test_passes_that_go_on_making_classes(chain, extra):
         r = ctx.refine(off, idx)
     _same(r, ex)
     assert r.rounds > chain and r.kernel_launches > 5
+
+
+@pytest.mark.parametrize("n,m,phases", [(1 << 20, 1 << 19, False), ((1 << 20) + 1, 1 << 19, True), ((1 << 20) + 8, (1 << 20) + 9 + (1 << 17), False),
+                                        ((1 << 20) + 8, (1 << 20) + 8 + (1 << 17), True), ((1 << 22) - 7, 90001, True)])
+def test_sparse_graphs_of_many_nodes(n, m, phases):
+    """Resident and unweighted, launch by launch; in one launch otherwise."""
+    off, idx = _er(n, m, 3)
+    ex = oracle.refine_exact(off, idx)
+    with R.Context(0) as ctx:
+        g = ctx.upload(off, idx)
+        for _ in range(2):
+            r = g.refine()
+            _same(r, ex)
+            assert (r.kernel_launches > 5) == phases
+        g.free()
+        r = ctx.refine(off, idx)
+        _same(r, ex)
+        assert r.kernel_launches <= 2
+        wt = np.full(m, 3, np.uint64)
+        g = ctx.upload(off, idx, wt)
+        r = g.refine()
+        _same(r, oracle.refine_exact(off, idx, wt))
+        assert r.kernel_launches <= 2
+        g.free()
