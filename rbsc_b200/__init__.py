@@ -19,6 +19,7 @@ Every call goes through librbsc.so; there is no CPU fallback.
 from __future__ import annotations
 
 import ctypes
+import weakref
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -128,9 +129,12 @@ class Context:
             raise RbscError(-2, self._lib.rbsc_last_error(None).decode())
         self._h = h
         self.device = device
+        self._graphs = weakref.WeakSet()  # freed with the context: they lie in its pool
 
     def close(self):
         if getattr(self, "_h", None):
+            for g in list(self._graphs):
+                g.free()
             self._lib.rbsc_ctx_destroy(self._h)
             self._h = None
 
@@ -264,6 +268,7 @@ class Graph:
     def __init__(self, ctx: Context, handle):
         self.ctx = ctx
         self._h = handle
+        ctx._graphs.add(self)
         n = ctypes.c_uint32()
         m = ctypes.c_uint64()
         ctx._lib.rbsc_graph_info(handle, ctypes.byref(n), ctypes.byref(m))
