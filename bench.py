@@ -223,7 +223,8 @@ def cpu_baseline_reference(off, idx, samples: int = 4):
                 "host_cores": os.cpu_count(), "port_all_cores": port_all_cores()}
     pa = port_all_cores()
     return {"value": pa.get("value"), "unit": UNIT, "cores": pa.get("cores"), "kind": "port",
-            "sample": "the oracle's rsc restatement, full refinement of the workload's graph", "host_cores": os.cpu_count()}
+            "sample": "the oracle's rsc restatement, full refinement of the workload's graph", "host_cores": os.cpu_count(),
+            "port_all_cores": pa}
 
 
 def reference_gpu_program(off, idx, blocks: int, timeout: float = 900.0):
