@@ -157,7 +157,7 @@ static rbsc_status run_chunks(rbsc_ctx* ctx, const std::vector<Chunk>& chunks, c
     HostCopier* c = ctx->copier;
     std::atomic<size_t> next{0};
     std::atomic<int> err{(int)cudaSuccess};
-    c->run([&](unsigned t) {
+    auto work = [&](unsigned t) {
         cudaError_t e = cudaSetDevice(ctx->device);
         Chunk pend[2] = {};  // out: what each slot holds once its copy is done
         unsigned k = 0;
@@ -184,7 +184,8 @@ static rbsc_status run_chunks(rbsc_ctx* ctx, const std::vector<Chunk>& chunks, c
                 if (e == cudaSuccess) std::memcpy(pend[slot].host, c->mem + (2 * t + slot) * kSlot, pend[slot].bytes);
             }
         if (e != cudaSuccess) err.store((int)e);
-    });
+    };
+    c->run(std::ref(work));  // (a copy of it would be allocated, which can throw)
     const cudaError_t e = (cudaError_t)err.load();
     if (e != cudaSuccess) return rbsc_cuda_fail(ctx, e, "host copy", __LINE__);
     return RBSC_OK;
