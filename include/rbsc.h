@@ -60,7 +60,11 @@ typedef struct rbsc_graph rbsc_graph;
 
 typedef struct {
     int32_t relabel;          /* RBSC_RELABEL_*                                          */
-    int32_t verify;           /* 1 (default): exact collision check at every fixpoint   */
+    int32_t verify;           /* 1 (default): exact collision check at every fixpoint;
+                                 0: the result rests on hashed keys, of 63 bits in the
+                                 one-launch kernels; launch by launch of 88 bits in the
+                                 first pass and 23 beside the table's slot (47 at 2^23
+                                 nodes in play) in later ones                          */
     uint32_t max_rounds;      /* 0 = no limit beyond N + 1                               */
     int32_t use_graph;        /* 1 (default): round loop as one CUDA graph with a
                                  device-side while node; 0 = host-driven loop           */
@@ -466,8 +470,9 @@ typedef struct {
     uint32_t queue_cap;       /* jobs waiting to start, 0 = 65536; submit beyond
                                  returns RBSC_ERR_BUSY                                */
     rbsc_opts opts;           /* refinement options of every job (no_persist is forced
-                                 on; the cooperative launches of jobs below 2^22 arcs
-                                 wait for one another)                                */
+                                 on; jobs of any size use cooperative launches, and
+                                 those of one device wait for one another: a small job
+                                 can wait for a large one's, 1.3 ms for 263 M arcs)   */
     int32_t dry_run;          /* TEST HOOK: 1 = no GPU work at all; each job "runs" for
                                  dry_run_ns_per_arc * arcs + 20 us of host sleep and
                                  writes no labels (exercises admission and packing)   */

@@ -16,10 +16,10 @@
 // sum).  A class that keeps a member outside keeps its id; of a class whose
 // members all moved, the largest group keeps it; the other groups are new
 // classes.  Ids are not used again: a class of s nodes that sheds one node a
-// pass, by a change of all others, uses s - 2 of them.  That is the partition a full pass gives: members outside T see
-// the same multiset of classes as before, and a node in T sees a class id
-// that no node outside T sees.  No new class: the fixpoint (the same pass
-// that a full pass would find unchanged).
+// pass, by a change of all others, uses s - 2 of them.  That is the partition
+// a full pass gives: members outside T see the same multiset of classes as
+// before, and a node in T sees a class id that no node outside T sees.  No new
+// class: the fixpoint (the same pass that a full pass would find unchanged).
 //
 // One block of 1024 threads runs the passes with its lists and tables in
 // shared memory: about five dependent L2 accesses a pass, 4 us, no grid barrier

@@ -338,15 +338,18 @@ rbsc_status outcome(rbsc_ctx* ctx, rbsc_stats* stats, float ms, bool* handled)
 
 }  // namespace
 
-// Below 2^22 arcs one launch always wins.  Above, the tile fold of the
-// launch-per-phase path catches up, first where it has more to offer (rival:
-// hot heads, or heads whose copy overlaps the first pass).  us a refinement,
-// one launch / launch per phase, uniform start: R-MAT-20 with 16 M arcs 487 /
-// 626, R-MAT-21 with 32 M 918 / 810 (with list_kernels.cuh after the first pass,
-// before either dealt its groups out: R-MAT-20 410, R-MAT-21 625, Erdos-Renyi with
-// 16 M arcs 501 against 447, a lift with 8.4 M 456 against 378); weighted (whose rows the launch-per-phase
-// check sorts) R-MAT-20 511 / 938 and R-MAT-21 947 / 1220 from degree colours,
-// R-MAT-22 with 65 M 1933 / 1852.
+// Below 2^22 arcs one launch always wins (sparse resident graphs apart: see
+// refine_resident).  Above, the first pass by tiles with list_kernels.cuh after
+// it catches up, first where it has more to offer (rival: hot heads, or heads
+// whose copy overlaps the first pass).  us a refinement, one launch / after the
+// first signatures / launch by launch, from one class: R-MAT-20 with 8 M arcs 385
+// / 287 / 571, with 16 M 430 / 343 / 595, R-MAT-21 with 32 M 840 / 545 / 799,
+// Erdos-Renyi with 16 M 211 / 261 / 558, a lift with 8.4 M 336 / 391 / 675: the line
+// at 24 M lies between, since a graph's skew is not known before it is prepared.
+// Weighted (whose rows the launch-per-phase check sorts), one launch / launch by
+// launch: R-MAT-20 with 16 M 627 / 1001, R-MAT-21 1114 / 1435, from degree colours
+// 467 / 789 and 863 / 1081, R-MAT-22 with 65 M 1560 / 1657: the line at 2^25, and
+// the rival that resident ones with colours have from 2^22, are older than these.
 constexpr uint64_t kSmallArcs = 1ull << 22, kLargeArcs = 3ull << 23, kLargeWeighted = 1ull << 25;
 
 std::unique_lock<std::mutex> coop_lock(int device)

@@ -1,5 +1,6 @@
 // fused_kernels.cuh -- a whole refinement in one launch, for graphs whose
-// passes are short (below about 2^22 arcs).
+// passes are short (below 2^22 arcs, and on to 24 or 32 M arcs where nothing else
+// is faster: fused_wanted).
 //
 // The launch-per-phase path spends such a graph's time on launches, host
 // synchronisations and phase boundaries, not on work: the 131,072-node lift
