@@ -140,7 +140,8 @@ struct FusedArgs {
 // "few": at most kFuDeepNew, and no sharp drop for kFuDeepSteady passes: the last
 // passes of a random graph make 200, 60, 15, 3, 1 and are soon over, a chain goes
 // on making the same number.  (With the first alone, Erdos-Renyi of 2^20 nodes and
-// 0.7 arcs per node took 1,509 us instead of 772, for the one pass saved.)
+// 0.7 arcs per node took 1,509 us instead of 772, for the one pass saved.)  After
+// twice deep_round's passes the first is enough: the numbers may go up and down.
 constexpr uint32_t kFuDeepNew = 256, kFuDeepSteady = 3;
 
 constexpr int kFuGrid = 0, kFuCluster = 1, kFuBlock = 2;
@@ -862,7 +863,8 @@ __device__ __forceinline__ void fused_body(const FusedArgs& a)
                 status = kFuNotConverged;
                 break;
             }
-            if (a.deep_round && round >= a.deep_round && trend >> 24 >= kFuDeepSteady && repairs == 0u) {
+            if (a.deep_round && round >= a.deep_round && (trend & 0xffffffu) <= kFuDeepNew && repairs == 0u &&
+                (trend >> 24 >= kFuDeepSteady || round >= 2u * a.deep_round)) {
                 if (first) t2 = fu_timer();
                 finish(kFuDeep, round, prev, initial, repairs);
                 return;

@@ -54,6 +54,25 @@ def test_passes_that_go_on_making_classes(chain, extra):
     assert r.rounds > chain and r.kernel_launches > 5
 
 
+def test_passes_that_make_more_and_fewer_classes_in_turn():
+    """A chain, and at every other node of it five nodes, each of a colour with one
+    at the first: they part when that node does, 6, 1, 6, 1 new classes."""
+    chain, each = 300, 5
+    k = np.arange(chain)
+    at = np.repeat(np.arange(0, chain, 2), each)
+    x = chain + 1 + 2 * np.arange(len(at))
+    n = chain + 1 + 2 * len(at)
+    off, idx, _ = G.csr_from_arcs(n, np.concatenate([k, x, x + 1]), np.concatenate([k + 1, at, 0 * at]))
+    init = np.concatenate([np.zeros(chain + 1), 1 + np.arange(2 * len(at)) // 2]).astype(np.uint32)
+    ex = oracle.refine_exact(off, idx, None, init)
+    new = np.diff(ex.round_blocks[20:280])
+    assert set(new) == {1, 1 + each}
+    with R.Context(0) as ctx:
+        r = ctx.refine(off, idx, None, init)
+    _same(r, ex)
+    assert r.kernel_launches > 5
+
+
 @pytest.mark.parametrize("n,m,phases", [(1 << 20, 1 << 19, False), ((1 << 20) + 1, 1 << 19, True), ((1 << 20) + 8, (1 << 20) + 9 + (1 << 17), False),
                                         ((1 << 20) + 8, (1 << 20) + 8 + (1 << 17), True), ((1 << 22) - 7, 90001, True)])
 def test_sparse_graphs_of_many_nodes(n, m, phases):
